@@ -162,16 +162,32 @@ __global__ void aos_to_rb_kernel(const double *__restrict__ aos, Fields f, Geo g
   for (int L = 0; L < 10; ++L) f.c[L][o] = aos[n * 10 + L];
 }
 
-__global__ void rb_to_aos_kernel(Fields f, double *__restrict__ aos, Geo g) {
-  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long V = 2 * g.V2;
-  if (n >= V) return;
-  const int i = (int)(n % g.N);
-  const long long r = n / g.N;
-  const int j = (int)(r % g.N), k = (int)(r / g.N);
-  const long long o = rb_off(g, i, j, k);
+// 128 sites per block, staged through shared memory so that the AoS side is
+// written in whole lines: written straight from the threads, each 8-byte store
+// of a warp touched 32 sectors (256^3: 748 us, now 396 us = 6.8 TB/s of its
+// 160 bytes per site; 160^3: 187, now 102 us).
+constexpr int kAosSites = 128;
+
+__global__ void __launch_bounds__(kAosSites) rb_to_aos_kernel(Fields f, double *__restrict__ aos, Geo g) {
+  __shared__ double s[kAosSites * 10];
+  const long long V = 2 * g.V2, n0 = (long long)blockIdx.x * kAosSites, n = n0 + threadIdx.x;
+  if (n < V) {
+    const long long r = n / g.N;
+    const int i = (int)(n - r * g.N), k = (int)(r / g.N), j = (int)(r - (long long)k * g.N);
+    const long long o = rb_off(g, i, j, k);
+    double v[10];
 #pragma unroll
-  for (int L = 0; L < 10; ++L) aos[n * 10 + L] = f.c[L][o];
+    for (int L = 0; L < 10; ++L) v[L] = f.c[L][o];
+#pragma unroll
+    for (int L = 0; L < 10; ++L) s[threadIdx.x * 10 + L] = v[L];
+  }
+  __syncthreads();
+  const int cnt = (int)min((long long)kAosSites, V - n0) * 10;
+#pragma unroll
+  for (int q = 0; q < 10; ++q) {
+    const int e = q * kAosSites + threadIdx.x;
+    if (e < cnt) aos[n0 * 10 + e] = s[e];
+  }
 }
 
 // ----------------------------------------------------------------------------
@@ -2511,7 +2527,7 @@ cudaError_t launch_aos_to_rb(const double *aos, Fields f, int N, cudaStream_t st
 }
 
 cudaError_t launch_rb_to_aos(Fields f, double *aos, const Geo &g, cudaStream_t st) {
-  rb_to_aos_kernel<<<nblocks(2 * g.V2, kThreads), kThreads, 0, st>>>(f, aos, g);
+  rb_to_aos_kernel<<<nblocks(2 * g.V2, kAosSites), kAosSites, 0, st>>>(f, aos, g);
   return cudaGetLastError();
 }
 cudaError_t launch_rb_to_aos(Fields f, double *aos, int N, cudaStream_t st) {
