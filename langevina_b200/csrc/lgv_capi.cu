@@ -87,6 +87,7 @@ struct lgv_handle {
   size_t scratch_len = 0;
   double *meas_dev = nullptr;
   double *small_dev = nullptr;  // 8 doubles
+  unsigned *meas_done = nullptr;  // counters of the measurement, zero between launches
   uint64_t key = 0, ctr = 0;
   int noise_mode = LGV_NOISE_COUNTER;
   double *inj_hb_prop = nullptr, *inj_hb_acc = nullptr, *inj_ch_q = nullptr, *inj_ch_acc = nullptr,
@@ -597,6 +598,11 @@ int create_handle(const lgv_params *params, const lgv::Geo &g, bool slab, int k0
         cudaMemset(h->waits_dev, 0, sizeof(unsigned long long)) != cudaSuccess)
       rc = fail(LGV_ERR_NOMEM, "wait counter alloc failed");
   }
+  if (rc == LGV_OK) {
+    const size_t n = lgv::kMeasCounters * sizeof(unsigned);
+    if (cudaMalloc((void **)&h->meas_done, n) != cudaSuccess || cudaMemset(h->meas_done, 0, n) != cudaSuccess)
+      rc = fail(LGV_ERR_NOMEM, "measurement counters alloc failed");
+  }
   if (rc == LGV_OK && h->hb_ordered) {
     h->hb_plan.wait_limit = h->wait_limit;
     const cudaError_t e = lgv::hb_plan_build(h->hb_plan, h->N, hb_slab, hb_spc, hb_lag);
@@ -707,6 +713,7 @@ int lgv_destroy(lgv_handle *h) {
   if (h->adj.done) cudaFree(h->adj.done);
   lgv::hb_plan_free(h->hb_plan);
   if (h->waits_dev) cudaFree(h->waits_dev);
+  if (h->meas_done) cudaFree(h->meas_done);
   for (auto &u : h->ev_used) {
     cudaEventDestroy(u.a);
     cudaEventDestroy(u.b);
@@ -870,7 +877,7 @@ int lgv_measure_device(lgv_handle *h, double *dev_out) {
   DeviceGuard g(h->device);
   LGV_TRY(ensure_scratch(h, lgv::measure_scratch_doubles(h->N)));
   KTimer tm(h, LGV_KCLASS_MEASURE);
-  LGV_CK(lgv::launch_measure(h->cur, h->N, h->scratch, dev_out, h->stream));
+  LGV_CK(lgv::launch_measure(h->cur, h->N, h->scratch, h->meas_done, dev_out, h->stream));
   return LGV_OK;
 }
 

@@ -293,10 +293,12 @@ size_t energy_scratch_doubles(int N);
 cudaError_t launch_energy(Fields f, int N, double H, double inv2chi_half, double *scratch, double *dev_out,
                           cudaStream_t st);
 // measurement: dev_out receives measure_size(N) doubles (lgv.h packing);
-// scratch >= measure_scratch_doubles(N)
+// scratch >= measure_scratch_doubles(N); done: kMeasCounters zeroed counters
+// (left zeroed), used by one stream at a time
+constexpr int kMeasCounters = 3;
 size_t measure_size(int N);
 size_t measure_scratch_doubles(int N);
-cudaError_t launch_measure(Fields f, int N, double *scratch, double *dev_out, cudaStream_t st);
+cudaError_t launch_measure(Fields f, int N, double *scratch, unsigned *done, double *dev_out, cudaStream_t st);
 // Pieces of the measurement for a lattice in host-order AoS layout (device
 // memory): the observable sums into T[25][N][N] and U[25][N][N], then walls,
 // OAverage, DFT and vev rotation into dev_out (lgv.h packing).

@@ -23,6 +23,7 @@
 //   em_adjoint_kernel, rot_phi_kernel, ideal_adj_a/b_kernel, batch_em_*
 //                       adjoints of the Euler-Maruyama and ideal steps for the
 //                       differentiable runs (no counterpart)
+#include "lgv_dft.cuh"
 #include "lgv_ideal_tma_cta.cuh"
 #include "lgv_internal.h"
 
@@ -1691,43 +1692,12 @@ __global__ void meas_walls_kernel(const double *T, const double *U, int N, MeasO
   else mo.ph[axis][(o - 11) * N + pos] = s;
 }
 
-// OAverage[l] = mean_x wallX(l, x) (measurer.cxx:292-300) and the r2c DFT of
-// every wall row, W(k) = (1/N) sum_x W(x) e^{-2 pi i k x / N}, k = 0..N/2.
-__global__ void meas_dft_kernel(int N, MeasOut mo) {
-  const int NK = N / 2 + 1;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < 11) {
-    double s = 0;
-    for (int i = 0; i < N; ++i) s += mo.wall[0][t * N + i];
-    mo.oavg[t] = s / (double)N;
-  }
-  if (t >= 3 * kNObs * NK) return;
-  const int kk = t % NK;
-  const int o = (t / NK) % kNObs;
-  const int axis = t / (NK * kNObs);
-  const double *row = (o < 11) ? mo.wall[axis] + o * N : mo.ph[axis] + (o - 11) * N;
-  double re = 0, im = 0;
-  for (int x = 0; x < N; ++x) {
-    const int m = (int)(((long long)kk * x) % N);
-    double sn, cs;
-    sincospi(2.0 * (double)m / (double)N, &sn, &cs);
-    re += row[x] * cs;
-    im -= row[x] * sn;
-  }
-  double *dst = (o < 11) ? mo.wk[axis] + (o * NK + kk) * 2 : mo.phk[axis] + ((o - 11) * NK + kk) * 2;
-  dst[0] = re / (double)N;
-  dst[1] = im / (double)N;
-}
-
 // rotate_to_vev (measurer.cxx:231-286), complex arithmetic as the reference.
-__global__ void meas_rotate_kernel(int N, MeasOut mo) {
-  const int NK = N / 2 + 1;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * NK) return;
-  const int kk = t % NK, axis = t / NK;
-  const double *w = mo.wk[axis];
-  auto re = [&](int a, int k) { return w[(a * NK + k) * 2]; };
-  auto im = [&](int a, int k) { return w[(a * NK + k) * 2 + 1]; };
+// One mode kk of one axis: w its k walls, o its rotated k walls.
+__device__ __forceinline__ void rotate_mode(const double *w, double *o, int NK, int kk) {
+  // the walls may come from other blocks of this launch (meas_finish_kernel): read at L2
+  auto re = [&](int a, int k) { return __ldcg(w + (a * NK + k) * 2); };
+  auto im = [&](int a, int k) { return __ldcg(w + (a * NK + k) * 2 + 1); };
   double nr[4], ni[4];
   double nrm = 0;
   for (int a = 0; a < 4; ++a) {
@@ -1751,7 +1721,6 @@ __global__ void meas_rotate_kernel(int N, MeasOut mo) {
     sr += nr[a] * pr[a] - ni[a] * pi[a];
     si += nr[a] * pi[a] + ni[a] * pr[a];
   }
-  double *o = mo.wkr[axis];
   auto put = [&](int a, double x, double y) { o[(a * NK + kk) * 2] = x; o[(a * NK + kk) * 2 + 1] = y; };
   put(0, sr, si);
   for (int a = 0; a < 4; ++a) {
@@ -1774,6 +1743,231 @@ __global__ void meas_rotate_kernel(int N, MeasOut mo) {
 #undef CMR
 #undef CMI
   put(13, re(10, kk), im(10, kk));
+}
+
+__global__ void meas_rotate_kernel(int N, MeasOut mo) {
+  const int NK = N / 2 + 1;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * NK) return;
+  rotate_mode(mo.wk[t / NK], mo.wkr[t / NK], NK, t % NK);
+}
+
+constexpr int kWallThreads = 256;   // block of meas_dft_kernel
+constexpr int kFinishThreads = 512;  // block of meas_finish_kernel
+
+// OAverage[l] = mean_x wallX(l, x) (measurer.cxx:292-300) and the r2c DFT of
+// one wall row (lgv_dft.cuh), W(k) = (1/N) sum_x W(x) e^{-2 pi i k x / N}, k =
+// 0..N/2, by one block: `row` is the row in shared memory, after a barrier.
+__device__ __forceinline__ void wall_modes(const double *row, const dft::Plan &p, double2 *tw, double2 *Z, int axis,
+                                           int o, const MeasOut &mo) {
+  const int N = p.N, NK = N / 2 + 1;
+  if (axis == 0 && o < 11 && threadIdx.x < 32) {
+    double s = 0;
+    for (int i = threadIdx.x; i < N; i += 32) s += row[i];
+    warp_sum(s);
+    if (threadIdx.x == 0) mo.oavg[o] = s / (double)N;
+  }
+  for (int u = threadIdx.x; u < p.K1 * p.N2; u += blockDim.x) {
+    const int k1[1] = {u / p.N2}, n2 = u - k1[0] * p.N2;
+    double2 z[1];
+    dft::inner<1>(row + n2, p, tw, n2, k1, z);
+    Z[u] = z[0];
+  }
+  __syncthreads();
+  double *dst = (o < 11) ? mo.wk[axis] + (size_t)o * NK * 2 : mo.phk[axis] + (size_t)(o - 11) * NK * 2;
+  const int n2h = p.N2 / 2 + 1;
+  for (int u = threadIdx.x; u < p.K1 * n2h; u += blockDim.x) {
+    const int k1 = u / n2h, k2[1] = {u - k1 * n2h};
+    double2 W[1], M[1];
+    dft::outer<1>(Z + k1 * p.N2, p, tw, k2, W, M);
+    dft::store(p, k1, k2[0], W[0], dst);
+    if (k2[0] > 0 && 2 * k2[0] < p.N2) dft::store(p, k1, p.N2 - k2[0], M[0], dst);
+  }
+}
+
+// dynamic shared memory of a block that transforms one row
+inline size_t wall_smem(const dft::Plan &p) {
+  return ((size_t)p.N + (size_t)p.K1 * p.N2) * sizeof(double2) + (size_t)p.N * sizeof(double);
+}
+
+// The modes of every wall row already in place; block = (row o, axis).
+__global__ void __launch_bounds__(kWallThreads) meas_dft_kernel(dft::Plan p, MeasOut mo) {
+  extern __shared__ __align__(16) double2 sm2[];
+  double2 *tw = sm2, *Z = sm2 + p.N;
+  double *row = (double *)(Z + p.K1 * p.N2);
+  const int o = blockIdx.x, axis = blockIdx.y;
+  const double *src = (o < 11) ? mo.wall[axis] + (size_t)o * p.N : mo.ph[axis] + (size_t)(o - 11) * p.N;
+  dft::fill_twiddles(tw, p.N);
+  for (int x = threadIdx.x; x < p.N; x += kWallThreads) row[x] = src[x];
+  __syncthreads();
+  wall_modes(row, p, tw, Z, axis, o, mo);
+}
+
+// ---- one-pass measurement ----------------------------------------------------
+// The 25 observables of every site are formed once and summed towards all
+// three axes: a block takes a brick of 32 sites in x (lanes) by TJ rows by 8
+// planes (warps).  A thread adds its site's observables over the rows (towards
+// x); each row of 32 sites goes through a warp's own [25][32] table in shared
+// memory, where lane l adds the row of observable l (towards y; a butterfly of
+// shuffles cost 2.3 times the instructions); and the sums over rows, added
+// over the lanes once at the end the same way, go towards z.  Each brick
+// writes its share of the walls and meas_finish_kernel adds the bricks in a
+// fixed order.  The two passes it replaces read the state twice and had N^2
+// threads, each adding N sites in a chain: a measurement took 92 us at 32^3,
+// 157 at 64^3, 295 at 120^3, 395 at 160^3 and 725 at 256^3; now 19, 25, 83,
+// 141 and 468.  It is bound by shared-memory bandwidth (73 % of the wavefronts
+// at 120^3) and the 24 % of the warps that its 128 registers leave.
+constexpr int kMtI = 32, kMtK = 8, kMtRows = 8, kMtLanes = 32;
+constexpr int kMtW = 34;  // doubles per table row: an odd number of 16-byte words, lanes on distinct banks
+constexpr size_t kMtSmem = (size_t)kMtK * (kNObs * kMtW + kMtRows * kMtLanes) * sizeof(double);
+
+struct MeasTiles {
+  int it, jt, kt, tj;
+  __host__ __device__ int npart(int axis) const { return axis == 0 ? kt * jt : axis == 1 ? kt * it : jt * it; }
+  __host__ __device__ int pitch(int axis) const { return axis == 0 ? it * kMtI : axis == 1 ? jt * tj : kt * kMtK; }
+  // doubles of the shares towards `axis`
+  __host__ __device__ size_t len(int axis) const { return (size_t)kNObs * npart(axis) * pitch(axis); }
+};
+
+// Rows per brick: as many as leave two bricks per SM, since a brick's shares
+// cost 1100 to 1900 doubles whatever its rows; at least 4.
+inline MeasTiles meas_tiles(int N) {
+  MeasTiles t;
+  t.it = (N + kMtI - 1) / kMtI;
+  t.kt = (N + kMtK - 1) / kMtK;
+  for (t.tj = 32; t.tj > 4; t.tj >>= 1)
+    if (t.it * t.kt * ((N + t.tj - 1) / t.tj) >= 2 * 148) break;
+  t.jt = (N + t.tj - 1) / t.tj;
+  return t;
+}
+
+// Sum over the warp of v[0..24] through its table: lane l < 25 returns the sum of v[l].
+__device__ __forceinline__ double warp_sum25(const double (&v)[kNObs], double *tab, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int o = 0; o < kNObs; ++o) tab[o * kMtW + lane] = v[o];
+  __syncwarp();
+  const double2 *r = (const double2 *)(tab + min(lane, kNObs - 1) * kMtW);
+  double a[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const double2 t = r[q];
+    a[q & 3] += t.x + t.y;
+  }
+  return (a[0] + a[1]) + (a[2] + a[3]);
+}
+
+__global__ void __launch_bounds__(256, 2) meas_tile_kernel(Fields f, Geo g, MeasTiles mt, double *__restrict__ xp,
+                                                        double *__restrict__ yp, double *__restrict__ zp) {
+  extern __shared__ __align__(16) double2 sm2[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double *tab = (double *)sm2 + (size_t)warp * kNObs * kMtW;       // [warp][25][kMtW]
+  double *ys = (double *)sm2 + (size_t)kMtK * kNObs * kMtW;        // [warp][row][lane]
+  const int ix = blockIdx.x, jy = blockIdx.y, kz = blockIdx.z;
+  const int N = g.N, i = ix * kMtI + 2 * (lane & 15) + (lane >> 4);  // a half warp's sites share the x parity
+  const int k = kz * kMtK + warp, j0 = jy * mt.tj, j1 = min(j0 + mt.tj, N);
+  const bool own = i < N && k < N;
+  const int V2 = (int)g.V2, base = (k * N + j0) * g.H + (i >> 1), par0 = (i + j0 + k) & 1;
+  double acc[kNObs], nx[10];
+#pragma unroll
+  for (int o = 0; o < kNObs; ++o) acc[o] = 0;
+  auto load = [&](int j) {
+    if (own && j < j1) {
+      const int off = ((par0 + j - j0) & 1) * V2 + base + (j - j0) * g.H;
+#pragma unroll
+      for (int L = 0; L < 10; ++L) nx[L] = f.c[L][off];
+    }
+  };
+  load(j0);
+  for (int jc = j0; jc < j1; jc += kMtRows) {
+    const int rows = min(min(kMtRows, mt.tj), j1 - jc);
+    for (int jj = 0; jj < rows; ++jj) {
+      double s[10], ob[kNObs];
+#pragma unroll
+      for (int L = 0; L < 10; ++L) s[L] = nx[L];
+      load(jc + jj + 1);
+      if (own) {
+        site_obs(s, ob);
+      } else {
+#pragma unroll
+        for (int o = 0; o < kNObs; ++o) ob[o] = 0;
+      }
+#pragma unroll
+      for (int o = 0; o < kNObs; ++o) acc[o] += ob[o];
+      ys[(warp * kMtRows + jj) * kMtLanes + lane] = warp_sum25(ob, tab, lane);
+    }
+    __syncthreads();
+    const size_t P = mt.npart(1), pitch = mt.pitch(1), q = (size_t)kz * mt.it + ix;
+    for (int e = threadIdx.x; e < rows * kMtLanes; e += 256) {
+      const int jj = e / kMtLanes, o = e % kMtLanes;
+      double t = 0;
+#pragma unroll
+      for (int w = 0; w < kMtK; ++w) t += ys[(w * kMtRows + jj) * kMtLanes + o];
+      if (o < kNObs) yp[((size_t)o * P + q) * pitch + jc + jj] = t;
+    }
+    __syncthreads();
+  }
+  const double zs = warp_sum25(acc, tab, lane);
+  if (lane < kNObs && k < N) zp[((size_t)lane * mt.npart(2) + (size_t)jy * mt.it + ix) * mt.pitch(2) + k] = zs;
+  // towards x: the warps' tables hold their sums over rows; thread t adds column t of the 25 x 32 over the planes
+  __syncthreads();
+  for (int e = threadIdx.x; e < kNObs * 32; e += 256) {
+    const int o = e >> 5, l = e & 31, x = ix * kMtI + 2 * (l & 15) + (l >> 4);
+    double t = 0;
+#pragma unroll
+    for (int w = 0; w < kMtK; ++w) t += ((const double *)sm2)[((size_t)w * kNObs + o) * kMtW + l];
+    if (x < N) xp[((size_t)o * mt.npart(0) + (size_t)kz * mt.jt + jy) * mt.pitch(0) + x] = t;
+  }
+}
+
+// Block (o, axis): wall row o towards `axis` from the bricks' shares, each
+// position by G groups of threads (fixed order), then its modes; the block that
+// ends last of an axis's first 11 rows then rotates that axis's modes.
+// done[3]: zero on entry, re-armed.
+__global__ void __launch_bounds__(kFinishThreads) meas_finish_kernel(const double *__restrict__ xp,
+                                                                    const double *__restrict__ yp,
+                                                                    const double *__restrict__ zp, MeasTiles mt,
+                                                                    dft::Plan p, int logP, MeasOut mo,
+                                                                    unsigned *done) {
+  extern __shared__ __align__(16) double2 sm2[];
+  __shared__ double part[kFinishThreads];
+  __shared__ bool last;
+  double2 *tw = sm2, *Z = sm2 + p.N;
+  double *row = (double *)(Z + p.K1 * p.N2);
+  const int N = p.N, o = blockIdx.x, axis = blockIdx.y;
+  const int np = mt.npart(axis), pitch = mt.pitch(axis);
+  const double *src = (axis == 0 ? xp : axis == 1 ? yp : zp) + (size_t)o * np * pitch;
+  dft::fill_twiddles(tw, N);
+  const int P = 1 << logP, G = kFinishThreads >> logP, grp = threadIdx.x >> logP;
+  double *dst = (o < 11) ? mo.wall[axis] + (size_t)o * N : mo.ph[axis] + (size_t)(o - 11) * N;
+  for (int x0 = 0; x0 < N; x0 += P) {
+    const int x = x0 + (threadIdx.x & (P - 1));
+    double s = 0;
+    if (x < N) {
+#pragma unroll 16
+      for (int q = grp; q < np; q += G) s += src[q * pitch + x];
+    }
+    part[threadIdx.x] = s;
+    __syncthreads();
+    if (grp == 0 && x < N) {
+      for (int q = 1; q < G; ++q) s += part[(q << logP) + threadIdx.x];
+      s /= (double)(N * N);
+      row[x] = s;
+      dst[x] = s;
+    }
+    __syncthreads();
+  }
+  wall_modes(row, p, tw, Z, axis, o, mo);
+  if (o >= 11) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done + axis, 1u) == 10u;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int kk = threadIdx.x; kk < N / 2 + 1; kk += kFinishThreads)
+    rotate_mode(mo.wk[axis], mo.wkr[axis], N / 2 + 1, kk);
+  if (threadIdx.x == 0) done[axis] = 0u;
 }
 
 // Sums of the 25 observables over a lattice given in the host-order AoS layout
@@ -2958,22 +3152,38 @@ size_t measure_size(int N) {
   return 11 + 75 * (size_t)N + 234 * NK;
 }
 
-size_t measure_scratch_doubles(int N) { return 2 * (size_t)kNObs * N * N; }
+// The one-pass measurement's shares grow as N^3 / 128 (they would be 1 GB at
+// N = 1024, where the tables of the two-pass sums take 0.4 GB); beyond
+// kMeasTileMaxN the two passes have N^2 threads enough to fill the chip.
+constexpr int kMeasTileMaxN = 512;
 
-cudaError_t launch_measure(Fields f, int N, double *scratch, double *dev_out, cudaStream_t st) {
-  const Geo g = make_geo(N);
-  const long long NN = (long long)N * N;
-  double *T = scratch, *U = scratch + (size_t)kNObs * NN;
-  meas_sum_j_kernel<<<nblocks(NN, 128), 128, 0, st>>>(f, g, T, 0, N, 0);
-  meas_sum_k_kernel<<<nblocks(NN, 128), 128, 0, st>>>(f, g, U, 0, N);
-  const MeasOut mo = meas_layout(dev_out, N);
-  meas_walls_kernel<<<nblocks(3LL * kNObs * N, 128), 128, 0, st>>>(T, U, N, mo);
-  const int NK = N / 2 + 1;
-  meas_dft_kernel<<<nblocks(3LL * kNObs * NK, 128), 128, 0, st>>>(N, mo);
-  meas_rotate_kernel<<<nblocks(3LL * NK, 128), 128, 0, st>>>(N, mo);
-  return cudaGetLastError();
+size_t measure_scratch_doubles(int N) {
+  if (N > kMeasTileMaxN) return 2 * (size_t)kNObs * N * N;
+  const MeasTiles t = meas_tiles(N);
+  return t.len(0) + t.len(1) + t.len(2);
 }
 
+cudaError_t launch_measure(Fields f, int N, double *scratch, unsigned *done, double *dev_out, cudaStream_t st) {
+  const Geo g = make_geo(N);
+  const long long NN = (long long)N * N;
+  if (N > kMeasTileMaxN) {
+    double *T = scratch, *U = scratch + (size_t)kNObs * NN;
+    meas_sum_j_kernel<<<nblocks(NN, 128), 128, 0, st>>>(f, g, T, 0, N, 0);
+    meas_sum_k_kernel<<<nblocks(NN, 128), 128, 0, st>>>(f, g, U, 0, N);
+    return launch_measure_finish(T, U, N, dev_out, st);
+  }
+  const MeasTiles t = meas_tiles(N);
+  double *xp = scratch, *yp = xp + t.len(0), *zp = yp + t.len(1);
+  const cudaError_t e = allow_smem(meas_tile_kernel, kMtSmem);
+  if (e != cudaSuccess) return e;
+  meas_tile_kernel<<<dim3(t.it, t.jt, t.kt), 256, kMtSmem, st>>>(f, g, t, xp, yp, zp);
+  const MeasOut mo = meas_layout(dev_out, N);
+  const dft::Plan p = dft::make_plan(N);
+  int logP = 3;
+  while (logP < 8 && (1 << logP) < N) ++logP;
+  meas_finish_kernel<<<dim3(kNObs, 3), kFinishThreads, wall_smem(p), st>>>(xp, yp, zp, t, p, logP, mo, done);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_measure_partials(Fields f, const Geo &g, int klo, int nk, int kout, double *T, double *U,
                                     cudaStream_t st) {
@@ -2993,12 +3203,16 @@ cudaError_t launch_measure_sums_aos(const double *aos, int N, double *T, double 
 cudaError_t launch_measure_finish(const double *T, const double *U, int N, double *dev_out, cudaStream_t st) {
   const MeasOut mo = meas_layout(dev_out, N);
   meas_walls_kernel<<<nblocks(3LL * kNObs * N, 128), 128, 0, st>>>(T, U, N, mo);
-  const int NK = N / 2 + 1;
-  meas_dft_kernel<<<nblocks(3LL * kNObs * NK, 128), 128, 0, st>>>(N, mo);
-  meas_rotate_kernel<<<nblocks(3LL * NK, 128), 128, 0, st>>>(N, mo);
+  const dft::Plan p = dft::make_plan(N);
+  const size_t smem = wall_smem(p);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = allow_smem(meas_dft_kernel, smem);
+    if (e != cudaSuccess) return e;
+  }
+  meas_dft_kernel<<<dim3(kNObs, 3), kWallThreads, smem, st>>>(p, mo);
+  meas_rotate_kernel<<<nblocks(3LL * (N / 2 + 1), 128), 128, 0, st>>>(N, mo);
   return cudaGetLastError();
 }
-
 
 // ---------------------------------------------------------------------------
 // Batched launchers.

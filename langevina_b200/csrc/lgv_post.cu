@@ -10,9 +10,13 @@
 // caller's stream.  Results are deterministic: every sum runs in a fixed order.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "../../include/lgv.h"
+#include "lgv_dft.cuh"
+
+namespace dft = lgv::dft;
 
 void lgv_internal_set_error(const char *msg);
 
@@ -34,84 +38,91 @@ int launched(const char *where) {
 
 // ----------------------------------------------------------------------------
 // x2k: W(k) = (1/N) sum_x W(x) e^{-2 pi i k x / N}, k = 0..N/2 (FFTW's r2c sign
-// and the 1/N of x2k.cxx:107-108).  One thread per (row, k); the block first
-// tabulates cos and sin of 2 pi m / N with the same sincospi call and argument
-// as the measurer's DFT, and the sum runs over x in order, so the transform of
-// a measured wall reproduces the measurer's k wall bit for bit.
-__global__ void __launch_bounds__(256) x2k_kernel(const double *__restrict__ w, long long rows, int N,
-                                                  double *__restrict__ out) {
-  extern __shared__ double tw[];  // tw[m] = sin, tw[N + m] = cos of 2 pi m / N
-  for (int m = threadIdx.x; m < N; m += blockDim.x) sincospi(2.0 * (double)m / (double)N, &tw[m], &tw[N + m]);
-  __syncthreads();
-  const int NK = N / 2 + 1;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= rows * NK) return;
-  const long long r = t / NK;
-  const int k = (int)(t - r * NK);
-  const double *row = w + r * N;
-  double re = 0, im = 0;
-  int m = 0;  // (k x) mod N
-  for (int x = 0; x < N; ++x) {
-    const double v = row[x];
-    re += v * tw[N + m];
-    im -= v * tw[m];
-    m += k;
-    if (m >= N) m -= N;
-  }
-  out[t * 2] = re / (double)N;
-  out[t * 2 + 1] = im / (double)N;
-}
+// and the 1/N of x2k.cxx:107-108), by the two-factor transform of lgv_dft.cuh,
+// whose chains the measurer's DFT shares, so the transform of a measured wall
+// reproduces the measurer's k wall bit for bit.
+//
+// A block takes R rows (a power of two; lanes are rows, so a twiddle is read
+// once for the whole warp and the row strides, odd, keep the lanes on distinct
+// banks).  Rows come in and modes leave through shared memory in whole lines;
+// kB columns (or k2's) per thread share each row value.  STAGE = false (N above
+// kX2kStageMaxN, one row per block): the table of N twiddles takes the room of
+// the row, which is read and written in global memory.  33 792 rows of 256: 84
+// us (139 MB in and out take 21), against 653 us for the direct sums, which
+// shared-memory bandwidth bound; now the phases between barriers do (36 % of
+// the warps resident, 46 % issue).  Measured at 16 rows and three blocks per
+// SM; 8 rows and four: 138 us, 16 rows and two: 90 us.
+constexpr int kX2kThreads = 256, kX2kB1 = 5, kX2kB2 = 5, kX2kStageMaxN = 4096;
+constexpr int kX2kLogRows = 4;  // 16 rows per block where they fit
+constexpr int kX2kBlocks = 3;   // blocks per SM
 
-// Same transform for N <= kX2kTileMaxN with 32 rows per block staged in shared
-// memory (row stride N + 1, odd, so the 32 lanes -- one row each -- read
-// distinct banks) and the lanes of a warp sharing one k, so every twiddle read
-// is a broadcast.  Warp w of the block takes k = w, w + 8, ...; the sum over x
-// runs in the same order with the same table, so results equal x2k_kernel's.
-constexpr int kX2kTileRows = 32, kX2kTileMaxN = 512;
+constexpr size_t kX2kSmem = 226 * 1024 / kX2kBlocks - 1024;
 
-__global__ void __launch_bounds__(256) x2k_tile_kernel(const double *__restrict__ w, long long rows, int N,
-                                                       double *__restrict__ out) {
-  extern __shared__ double sm[];
-  double *tw = sm;            // 2N: sin, cos
-  double *tile = sm + 2 * N;  // [32][N + 1]
-  const int S = N + 1, NK = N / 2 + 1;
-  for (int m = threadIdx.x; m < N; m += blockDim.x) sincospi(2.0 * (double)m / (double)N, &tw[m], &tw[N + m]);
-  const long long r0 = (long long)blockIdx.x * kX2kTileRows;
-  const int nr = (int)min((long long)kX2kTileRows, rows - r0);
-  for (int e = threadIdx.x; e < nr * N; e += blockDim.x) {
-    const int rr = e / N, x = e - rr * N;
-    tile[rr * S + x] = w[(r0 + rr) * N + x];
-  }
-  __syncthreads();
+struct X2kShape {
+  dft::Plan p;
+  int R, logR;  // rows per block
+  int SA, SZ;   // strides of a row of walls / modes (doubles) and of Z (double2), odd
+};
+
+template <bool STAGE>
+__global__ void __launch_bounds__(kX2kThreads, kX2kBlocks) x2k_kernel(const double *__restrict__ w, long long rows, X2kShape s,
+                                                          double *__restrict__ out) {
+  extern __shared__ __align__(16) double2 sm2[];
+  const dft::Plan p = s.p;
+  const int N = p.N, NK = N / 2 + 1, R = s.R;
+  double2 *tw = sm2, *Z = sm2 + N;
+  double *A = (double *)(Z + (size_t)R * s.SZ);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane >= nr) return;
-  const double *row = tile + lane * S;
-  double *o = out + (r0 + lane) * NK * 2;
-  // four k per pass over the row (k, k + 8, k + 16, k + 24): each row value
-  // read from shared memory serves eight multiply-adds
-  for (int k0 = warp; k0 < NK; k0 += 32) {
-    double re[4] = {0, 0, 0, 0}, im[4] = {0, 0, 0, 0};
-    int m[4] = {0, 0, 0, 0}, dk[4];
+  dft::fill_twiddles(tw, N);
+  for (long long r0 = (long long)blockIdx.x * R; r0 < rows; r0 += (long long)gridDim.x * R) {
+  const int nr = (int)min((long long)R, rows - r0);
+  if (STAGE)
+    for (int rr = warp; rr < nr; rr += kX2kThreads / 32)
+      for (int x = lane; x < N; x += 32) A[rr * s.SA + x] = w[(r0 + rr) * N + x];
+  __syncthreads();
+  const int rr = threadIdx.x & (R - 1), u0 = threadIdx.x >> s.logR, nu = kX2kThreads >> s.logR;
+  const bool live = rr < nr;
+  const double *row = STAGE ? A + rr * s.SA : w + r0 * N;
+  double2 *Zr = Z + (size_t)rr * s.SZ;
+  const int nb1 = (p.K1 + kX2kB1 - 1) / kX2kB1;
+  for (int u = u0; u < p.N2 * nb1; u += nu) {
+    const int n2 = u / nb1, c0 = (u - n2 * nb1) * kX2kB1;
+    int k1[kX2kB1];
+    double2 z[kX2kB1];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) dk[q] = (k0 + 8 * q) % N;  // k itself for every k < NK; keeps m < N beyond
-    for (int x = 0; x < N; ++x) {
-      const double v = row[x];
+    for (int b = 0; b < kX2kB1; ++b) k1[b] = min(c0 + b, p.K1 - 1);
+    if (live) {
+      dft::inner<kX2kB1>(row + n2, p, tw, n2, k1, z);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        re[q] += v * tw[N + m[q]];
-        im[q] -= v * tw[m[q]];
-        m[q] += dk[q];
-        if (m[q] >= N) m[q] -= N;
+      for (int b = 0; b < kX2kB1; ++b)
+        if (c0 + b < p.K1) Zr[(c0 + b) * p.N2 + n2] = z[b];
+    }
+  }
+  __syncthreads();
+  double *o = STAGE ? A + rr * s.SA : out + r0 * NK * 2;
+  const int n2h = p.N2 / 2 + 1, nb2 = (n2h + kX2kB2 - 1) / kX2kB2;
+  for (int u = u0; u < p.K1 * nb2; u += nu) {
+    const int k1 = u / nb2, c0 = (u - k1 * nb2) * kX2kB2;
+    int k2[kX2kB2];
+    double2 W[kX2kB2], M[kX2kB2];
+#pragma unroll
+    for (int b = 0; b < kX2kB2; ++b) k2[b] = min(c0 + b, n2h - 1);
+    if (live) {
+      dft::outer<kX2kB2>(Zr + k1 * p.N2, p, tw, k2, W, M);
+#pragma unroll
+      for (int b = 0; b < kX2kB2; ++b) {
+        if (c0 + b >= n2h) continue;
+        dft::store(p, k1, k2[b], W[b], o);
+        if (k2[b] > 0 && 2 * k2[b] < p.N2) dft::store(p, k1, p.N2 - k2[b], M[b], o);
       }
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k = k0 + 8 * q;
-      if (k < NK) {
-        o[k * 2] = re[q] / (double)N;
-        o[k * 2 + 1] = im[q] / (double)N;
-      }
-    }
+  }
+  __syncthreads();
+  if (STAGE) {
+    for (int r = warp; r < nr; r += kX2kThreads / 32)
+      for (int x = lane; x < 2 * NK; x += 32) out[(r0 + r) * NK * 2 + x] = A[r * s.SA + x];
+    __syncthreads();
+  }
   }
 }
 
@@ -308,26 +319,23 @@ int lgv_x2k(const double *walls, int64_t rows, int N, double *out, void *stream)
   if (rows < 0 || N < 2 || (N & 1) || N > 8192)
     return fail(LGV_ERR_INVALID, "lgv_x2k: rows >= 0, N even in [2, 8192]");
   if (rows == 0) return LGV_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (N <= kX2kTileMaxN) {
-    const long long blocks = (rows + kX2kTileRows - 1) / kX2kTileRows;
-    if (blocks > 0x7fffffffLL) return fail(LGV_ERR_INVALID, "lgv_x2k: too many rows for one launch");
-    const size_t smem = (2 * (size_t)N + (size_t)kX2kTileRows * (N + 1)) * sizeof(double);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(x2k_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return fail(LGV_ERR_CUDA, "lgv_x2k: shared memory for the row tile");
-    x2k_tile_kernel<<<(unsigned)blocks, 256, smem, st>>>(walls, rows, N, out);
-    return launched("lgv_x2k: launch failed");
-  }
-  const long long NK = N / 2 + 1, total = rows * NK;
-  const int threads = 256;
-  const long long blocks = (total + threads - 1) / threads;
-  if (blocks > 0x7fffffffLL) return fail(LGV_ERR_INVALID, "lgv_x2k: too many rows for one launch");
-  const size_t smem = 2 * (size_t)N * sizeof(double);
+  X2kShape s;
+  s.p = dft::make_plan(N);
+  s.SA = N + 3;
+  s.SZ = (s.p.K1 * s.p.N2) | 1;
+  const bool stage = N <= kX2kStageMaxN;
+  const size_t per_row = s.SZ * sizeof(double2) + (stage ? s.SA * sizeof(double) : 0);
+  const size_t table = (size_t)N * sizeof(double2);
+  s.logR = stage ? kX2kLogRows : 0;
+  while (s.logR > 0 && table + (per_row << s.logR) > kX2kSmem) --s.logR;
+  s.R = 1 << s.logR;
+  const size_t smem = table + (per_row << s.logR);
+  const long long blocks = std::min<long long>((rows + s.R - 1) / s.R, 148LL * kX2kBlocks);
+  const auto kern = stage ? x2k_kernel<true> : x2k_kernel<false>;
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(x2k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return fail(LGV_ERR_CUDA, "lgv_x2k: shared memory for the twiddle table");
-  x2k_kernel<<<(unsigned)blocks, threads, smem, st>>>(walls, rows, N, out);
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return fail(LGV_ERR_CUDA, "lgv_x2k: shared memory for the rows");
+  kern<<<(unsigned)blocks, kX2kThreads, smem, (cudaStream_t)stream>>>(walls, rows, s, out);
   return launched("lgv_x2k: launch failed");
 }
 
