@@ -203,11 +203,9 @@ __global__ void __launch_bounds__(128) x2k_rotated_kernel(const double *__restri
 // a[t * ld + s] (real) or a[t * ld + 2 s], +1 (complex).  Output time-major too:
 // out[tau * ns + s] (complex: pairs).
 //
-// Block: 32 series (lanes) x 4 lag groups (warps); a thread owns G consecutive
-// lags and keeps their sums in registers.  For decim = 1 time runs in chunks of
-// G steps: the 2G-1 values of b the chunk needs are loaded once into registers,
-// so G^2 multiply-adds cost G + 2G - 1 loads (the same b value serves G lags).
-// Each lag's sum still runs over t in increasing order.
+// Block: 32 series (lanes) x kCorrLagWarps lag groups (warps); a thread owns G
+// consecutive lags and keeps their sums in registers.  Each lag's sum runs over
+// t in increasing order.
 template <bool CPLX>
 struct Val {
   double re, im;
@@ -232,20 +230,206 @@ __device__ __forceinline__ Val<CPLX> ld_val(const double *p) {
 template <bool CPLX>
 __device__ __forceinline__ void mac(Val<CPLX> &acc, const Val<CPLX> &x, const Val<CPLX> &y) {
   if (CPLX) {
-    acc.re += x.re * y.re - x.im * y.im;
-    acc.im += x.re * y.im + x.im * y.re;
+    acc.re = fma(x.re, y.re, acc.re);
+    acc.re = fma(-x.im, y.im, acc.re);
+    acc.im = fma(x.re, y.im, acc.im);
+    acc.im = fma(x.im, y.re, acc.im);
   } else {
-    acc.re += x.re * y.re;
+    acc.re = fma(x.re, y.re, acc.re);
   }
 }
 
 constexpr int kCorrLagWarps = 4;
 
+// mean(a_s) mean(b_s) over all T samples, each sum in increasing t.
+template <bool CPLX, bool VEC>
+__device__ __forceinline__ Val<CPLX> mean_product(const double *pa, const double *pb, long long T, long long ld) {
+  Val<CPLX> sa, sb, cc;
+  sa.re = sa.im = sb.re = sb.im = cc.re = cc.im = 0.0;
+#pragma unroll 8
+  for (long long t = 0; t < T; ++t) {
+    const Val<CPLX> x = ld_val<CPLX, VEC>(pa + t * ld), y = ld_val<CPLX, VEC>(pb + t * ld);
+    sa.re += x.re;
+    sa.im += x.im;
+    sb.re += y.re;
+    sb.im += y.im;
+  }
+  sa.re /= (double)T;
+  sa.im /= (double)T;
+  sb.re /= (double)T;
+  sb.im /= (double)T;
+  mac<CPLX>(cc, sa, sb);
+  return cc;
+}
+
+template <bool CPLX, int G>
+__device__ __forceinline__ void store_lags(const Val<CPLX> (&acc)[G], const Val<CPLX> &cc, long long tau0, long long T,
+                                           int ntmax, int decim, double *o, long long row) {
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const long long tau = tau0 + g;
+    if (tau >= ntmax) break;
+    const double cnt = (double)((T - tau + decim - 1) / decim);
+    o[tau * row] = acc[g].re / cnt - cc.re;
+    if (CPLX) o[tau * row + 1] = acc[g].im / cnt - cc.im;
+  }
+}
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+// one value (pair) of a row into shared memory, asynchronously
+template <bool CPLX, bool VEC>
+__device__ __forceinline__ void copy_val(double *dst, const double *src) {
+  if (CPLX && VEC) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    if (CPLX) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_u32(dst + 1)), "l"(src + 1) : "memory");
+  }
+}
+
+// Every sample (decim 1).  Time runs in chunks of kCorrChunk steps: the block
+// keeps the chunk's rows of a (two chunks, one arriving by cp.async while the
+// other is used) and a ring of the rows of b its lags reach, each row loaded
+// once per block.  Within a chunk a thread reads G values of a and 2G - 1 of b
+// from shared memory per G steps for G^2 multiply-adds.  What it replaces read
+// the same values from global memory and waited for them: 14.8 of 16.2 cycles
+// per issue on the load, FP64 pipe a fifth busy.  2000 samples of 1419 complex
+// series, 250 lags: 600 -> 320 us (a complex multiply-add is four fma's, 155 us
+// of FP64 pipe).  Two warps per block copy more per product (424 us), six and
+// eight leave the last wave emptier (374, 437 us).
+constexpr int kCorrChunk = 16;
+
 template <bool CPLX, bool VEC, int G>
 __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *__restrict__ a,
                                                                  const double *__restrict__ b, long long T,
-                                                                 long long ns, long long ld, int ntmax, int decim,
-                                                                 int conn, double *__restrict__ out) {
+                                                                 long long ns, long long ld, int ntmax, int conn,
+                                                                 double *__restrict__ out) {
+  constexpr int W = CPLX ? 2 : 1, C = kCorrChunk, NW = kCorrLagWarps, L = NW * G;
+  constexpr int RB = L + 2 * C;  // ring rows of b: the chunk's C + L - 1, and the C arriving
+  static_assert(RB % C == 0 && C % G == 0 && L % G == 0, "otot_kernel: ring");
+  extern __shared__ __align__(16) double sm[];
+  double *sa = sm, *sb = sm + 2 * C * 32 * W;
+  const int lane = threadIdx.x, wp = threadIdx.y;
+  const long long s = (long long)blockIdx.x * 32 + lane, tb = (long long)blockIdx.y * L, tau0 = tb + wp * G;
+  const bool live = s < ns;
+  const double *pa = a + (live ? s : 0) * W, *pb = b + (live ? s : 0) * W;
+  const long long Ta = T - tb;  // samples of a that any lag of the block uses (tb < ntmax <= T)
+  // This thread copies rows wp, wp + NW, ... of every C rows; `left` rows are
+  // left of the n asked for.  Ring rows start at multiples of C and the rings
+  // are multiples of C long, so C rows never wrap.
+  static_assert(C % NW == 0 && L % C == 0, "otot_kernel: copies");
+  const double *ga = pa + wp * ld, *gb = pb + (tb + wp) * ld;
+  const long long ldw = NW * ld;
+  auto load_rows = [&](const double *&src, double *ring, long long left) {
+    double *dst = ring + (wp * 32 + lane) * W;
+    if (live) {
+      if (left >= C) {
+#pragma unroll
+        for (int q = 0; q < C / NW; ++q) copy_val<CPLX, VEC>(dst + q * NW * 32 * W, src + q * ldw);
+      } else {
+        for (int q = 0; q < C / NW; ++q)
+          if (wp + q * NW < left) copy_val<CPLX, VEC>(dst + q * NW * 32 * W, src + q * ldw);
+      }
+    }
+    src += C * ld;
+  };
+  load_rows(ga, sa, Ta);
+#pragma unroll
+  for (int q = 0; q < C + L; q += C) load_rows(gb, sb + q * 32 * W, Ta - q);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  Val<CPLX> acc[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g) acc[g].re = acc[g].im = 0.0;
+  auto val = [&](const double *base, int row) {
+    Val<CPLX> v;
+    const double *p = base + (row * 32 + lane) * W;
+    if (CPLX) {
+      const double2 q = *reinterpret_cast<const double2 *>(p);
+      v.re = q.x;
+      v.im = q.y;
+    } else {
+      v.re = p[0];
+      v.im = 0.0;
+    }
+    return v;
+  };
+  int ra = 0, rb = 0;  // ring rows of the chunk's first a and b
+  for (long long t0 = 0; t0 < Ta; t0 += C) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    load_rows(ga, sa + (C - ra) * 32 * W, Ta - t0 - C);
+    load_rows(gb, sb + (rb >= C ? rb - C : rb + RB - C) * 32 * W, Ta - t0 - C - L);  // onto the rows before rb
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    if (t0 + C - 1 + tau0 - tb + G - 1 < Ta) {
+#pragma unroll 1
+      for (int h = 0; h < C; h += G) {
+        // the G steps' window of b: rows r .. r + 2G - 2, where the ring can end only at r + G (RB, rb, h, wp G
+        // are multiples of G)
+        int r = rb + h + wp * G;
+        if (r >= RB) r -= RB;
+        const double *w0 = sb + (r * 32 + lane) * W, *w1 = sb + ((r + G < RB ? r + G : 0) * 32 + lane) * W;
+        const double *xa = sa + ((ra + h) * 32 + lane) * W;
+        Val<CPLX> wb[2 * G - 1], sum[G];
+#pragma unroll
+        for (int i = 0; i < 2 * G - 1; ++i) wb[i] = ld_val<CPLX, true>((i < G ? w0 : w1) + (i < G ? i : i - G) * 32 * W);
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+          const Val<CPLX> x = ld_val<CPLX, true>(xa + u * 32 * W);
+          // the G steps' products are added by themselves first; the two
+          // that a complex multiply-add gives one sum are G chains apart
+#pragma unroll
+          for (int g = 0; g < G; ++g) sum[g].re = u == 0 ? x.re * wb[g].re : fma(x.re, wb[u + g].re, sum[g].re);
+          if (CPLX) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) sum[g].im = u == 0 ? x.re * wb[g].im : fma(x.re, wb[u + g].im, sum[g].im);
+#pragma unroll
+            for (int g = 0; g < G; ++g) sum[g].re = fma(-x.im, wb[u + g].im, sum[g].re);
+#pragma unroll
+            for (int g = 0; g < G; ++g) sum[g].im = fma(x.im, wb[u + g].re, sum[g].im);
+          }
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          acc[g].re += sum[g].re;
+          if (CPLX) acc[g].im += sum[g].im;
+        }
+      }
+    } else {  // some products lie past the end
+#pragma unroll 1
+      for (int u = 0; u < C; ++u) {
+        const Val<CPLX> x = val(sa, ra + u);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          int r = rb + u + wp * G + g;
+          if (r >= RB) r -= RB;
+          if (t0 + u + tau0 - tb + g < Ta) mac<CPLX>(acc[g], x, val(sb, r));
+        }
+      }
+    }
+    ra = C - ra;
+    rb += C;
+    if (rb >= RB) rb -= RB;
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (!live || tau0 >= ntmax) return;
+  Val<CPLX> cc;
+  cc.re = cc.im = 0.0;
+  if (conn) cc = mean_product<CPLX, VEC>(pa, pb, T, ld);
+  store_lags<CPLX, G>(acc, cc, tau0, T, ntmax, 1, out + s * W, ns * W);
+}
+
+template <bool CPLX, int G>
+constexpr size_t otot_smem() {
+  return (size_t)(4 * kCorrChunk + kCorrLagWarps * G) * 32 * (CPLX ? 2 : 1) * sizeof(double);
+}
+
+// Every decim-th sample (decim > 1): the rows of a chunk share little, so the
+// values come from global memory, those of all G lags of one t at a time.
+template <bool CPLX, bool VEC, int G>
+__global__ void __launch_bounds__(32 * kCorrLagWarps) otot_decim_kernel(const double *__restrict__ a,
+                                                                       const double *__restrict__ b, long long T,
+                                                                       long long ns, long long ld, int ntmax,
+                                                                       int decim, int conn, double *__restrict__ out) {
   constexpr int W = CPLX ? 2 : 1;
   const long long s = (long long)blockIdx.x * 32 + threadIdx.x;
   const long long tau0 = ((long long)blockIdx.y * kCorrLagWarps + threadIdx.y) * G;
@@ -255,57 +439,26 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *
   Val<CPLX> acc[G];
 #pragma unroll
   for (int g = 0; g < G; ++g) acc[g].re = acc[g].im = 0.0;
-  if (decim == 1) {
-    long long t0 = 0;
-    // every (t, lag) of a chunk is in range when t0 + G - 1 + tau0 + G - 1 < T
-    for (; t0 + tau0 + 2 * G - 2 < T; t0 += G) {
-      Val<CPLX> wb[2 * G - 1];
+  long long t = 0;
+#pragma unroll 2
+  for (; t + tau0 + G - 1 < T; t += decim) {
+    Val<CPLX> y[G];
+    const Val<CPLX> x = ld_val<CPLX, VEC>(pa + t * ld);
 #pragma unroll
-      for (int i = 0; i < 2 * G - 1; ++i) wb[i] = ld_val<CPLX, VEC>(pb + (t0 + tau0 + i) * ld);
+    for (int g = 0; g < G; ++g) y[g] = ld_val<CPLX, VEC>(pb + (t + tau0 + g) * ld);
 #pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const Val<CPLX> x = ld_val<CPLX, VEC>(pa + (t0 + u) * ld);
-#pragma unroll
-        for (int g = 0; g < G; ++g) mac<CPLX>(acc[g], x, wb[u + g]);
-      }
-    }
+    for (int g = 0; g < G; ++g) mac<CPLX>(acc[g], x, y[g]);
+  }
+  for (; t + tau0 < T; t += decim) {
+    const Val<CPLX> x = ld_val<CPLX, VEC>(pa + t * ld);
 #pragma unroll
     for (int g = 0; g < G; ++g)
-      for (long long t = t0; t < T - tau0 - g; ++t)
-        mac<CPLX>(acc[g], ld_val<CPLX, VEC>(pa + t * ld), ld_val<CPLX, VEC>(pb + (t + tau0 + g) * ld));
-  } else {
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-      for (long long t = 0; t < T - tau0 - g; t += decim)
-        mac<CPLX>(acc[g], ld_val<CPLX, VEC>(pa + t * ld), ld_val<CPLX, VEC>(pb + (t + tau0 + g) * ld));
+      if (t + tau0 + g < T) mac<CPLX>(acc[g], x, ld_val<CPLX, VEC>(pb + (t + tau0 + g) * ld));
   }
   Val<CPLX> cc;
   cc.re = cc.im = 0.0;
-  if (conn) {
-    Val<CPLX> sa, sb;
-    sa.re = sa.im = sb.re = sb.im = 0.0;
-    for (long long t = 0; t < T; ++t) {
-      const Val<CPLX> x = ld_val<CPLX, VEC>(pa + t * ld), y = ld_val<CPLX, VEC>(pb + t * ld);
-      sa.re += x.re;
-      sa.im += x.im;
-      sb.re += y.re;
-      sb.im += y.im;
-    }
-    sa.re /= (double)T;
-    sa.im /= (double)T;
-    sb.re /= (double)T;
-    sb.im /= (double)T;
-    mac<CPLX>(cc, sa, sb);
-  }
-#pragma unroll
-  for (int g = 0; g < G; ++g) {
-    const long long tau = tau0 + g;
-    if (tau >= ntmax) break;
-    const double cnt = (double)((T - tau + decim - 1) / decim);
-    double *o = out + (tau * ns + s) * W;
-    o[0] = acc[g].re / cnt - cc.re;
-    if (CPLX) o[1] = acc[g].im / cnt - cc.im;
-  }
+  if (conn) cc = mean_product<CPLX, VEC>(pa, pb, T, ld);
+  store_lags<CPLX, G>(acc, cc, tau0, T, ntmax, decim, out + s * W, ns * W);
 }
 
 constexpr int kGReal = 16, kGCplx = 8;
@@ -364,12 +517,24 @@ int lgv_time_correlator(const double *a, const double *b, int64_t T, int64_t nse
   const dim3 grid((unsigned)gs, (unsigned)gl), block(32, kCorrLagWarps);
   const bool vec = ((uintptr_t)a % 16 == 0) && ((uintptr_t)b % 16 == 0) && ld % 2 == 0;
   cudaStream_t st = (cudaStream_t)stream;
-  if (is_complex && vec)
-    otot_kernel<true, true, kGCplx><<<grid, block, 0, st>>>(a, b, T, nseries, ld, ntmax, decim, conn, out);
-  else if (is_complex)
-    otot_kernel<true, false, kGCplx><<<grid, block, 0, st>>>(a, b, T, nseries, ld, ntmax, decim, conn, out);
-  else
-    otot_kernel<false, false, kGReal><<<grid, block, 0, st>>>(a, b, T, nseries, ld, ntmax, decim, conn, out);
+#define LGV_OTOT(CP, VE, GG)                                                                                          \
+  if (decim == 1) {                                                                                                  \
+    constexpr size_t smem = otot_smem<CP, GG>();                                                                     \
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(otot_kernel<CP, VE, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                                 (int)smem) != cudaSuccess)                                          \
+      return fail(LGV_ERR_CUDA, "lgv_time_correlator: shared memory");                                               \
+    otot_kernel<CP, VE, GG><<<grid, block, smem, st>>>(a, b, T, nseries, ld, ntmax, conn, out);                      \
+  } else {                                                                                                           \
+    otot_decim_kernel<CP, VE, GG><<<grid, block, 0, st>>>(a, b, T, nseries, ld, ntmax, decim, conn, out);            \
+  }
+  if (is_complex && vec) {
+    LGV_OTOT(true, true, kGCplx)
+  } else if (is_complex) {
+    LGV_OTOT(true, false, kGCplx)
+  } else {
+    LGV_OTOT(false, false, kGReal)
+  }
+#undef LGV_OTOT
   return launched("lgv_time_correlator: launch failed");
 }
 
