@@ -129,9 +129,9 @@ struct lgv_handle {
   int k0 = 0, nz = 0;
   lgv_halo_fn halo_fn = nullptr;
   void *halo_ctx = nullptr;
-  // charge heat bath as three two-face launches (one per direction) instead
-  // of six single-face launches (LGV_CHARGE_FUSED=1 at lgv_create)
-  bool charge_per_face = true;
+  // charge heat bath as six single-face launches instead of three two-face
+  // launches (LGV_CHARGE_FUSED=0 at lgv_create)
+  bool charge_per_face = false;
   lgv::MonAcc *mon_dev = nullptr;  // [3]
   lgv_monitor mon_ideal{};
   uint8_t *flags_dev = nullptr;
@@ -417,7 +417,10 @@ int sub_charge(lgv_handle *h, double dt) {  // ModelGChargeHB::step (Stepper.cxx
     a.q = h->inj_ch_q;
     a.acc = h->inj_ch_acc;
   }
-  if (h->charge_per_face) {
+  // Both faces of a direction per launch; one face per launch on a slab (its
+  // ghost planes are refreshed before every z-face), with injected noise, and
+  // where single decisions are recorded.
+  if (h->charge_per_face || h->slab || a.q || a.mon || a.flags) {
     for (int p = 0; p < 6; ++p) {
       a.pass = p;
       if (h->noise_mode != LGV_NOISE_INJECTED) a.sk = lgv::sub_key(h->key, h->ctr + 1 + p);
@@ -426,25 +429,17 @@ int sub_charge(lgv_handle *h, double dt) {  // ModelGChargeHB::step (Stepper.cxx
       LGV_CK(lgv::launch_charge_pass(h->cur, pass_geo(h), xyz[p / 2], eo[p % 2], a, h->stream));
     }
   } else {
-    // both faces of a direction per launch (same streams and order as per face)
     lgv::ChargeDirPair d{};
     d.rms = a.rms;
     d.inv2chi = a.inv2chi;
-    d.q = a.q;
-    d.acc = a.acc;
-    d.flags = a.flags;
-    d.mon = a.mon;
     for (int ixyz = 0; ixyz < 3; ++ixyz) {
       for (int i = 0; i < 2; ++i) {
-        d.pass[i] = 2 * ixyz + i;
         d.eo[i] = eo[i];
-        d.sk[i] = (h->noise_mode != LGV_NOISE_INJECTED) ? lgv::sub_key(h->key, h->ctr + 1 + 2 * ixyz + i) : 0;
+        d.sk[i] = lgv::sub_key(h->key, h->ctr + 1 + 2 * ixyz + i);
       }
-      bool swapped = false;
       KTimer tm(h, LGV_KCLASS_CHARGE, 2);
-      LGV_CK(lgv::launch_charge_dir(h->cur, h->alt, h->N, xyz[ixyz], d, h->stream, &swapped));
-      if (swapped)
-        for (int L = 4; L < 10; ++L) std::swap(h->cur.c[L], h->alt.c[L]);
+      LGV_CK(lgv::launch_charge_dir(h->cur, h->alt, pass_geo(h), xyz[ixyz], d, h->stream));
+      for (int L = 4; L < 10; ++L) std::swap(h->cur.c[L], h->alt.c[L]);
     }
   }
   if (h->noise_mode == LGV_NOISE_INJECTED) h->have_ch = false;
@@ -550,10 +545,8 @@ int create_handle(const lgv_params *params, const lgv::Geo &g, bool slab, int k0
   if (!slab) {
     const char *f = std::getenv("LGV_HB_FUSED");
     h->hb_fused = f && f[0] == '1';
-    // one face per launch (the faster path on B200); LGV_CHARGE_FUSED=1 selects
-    // both faces of a direction per launch
     const char *c = std::getenv("LGV_CHARGE_FUSED");
-    h->charge_per_face = !(c && c[0] == '1');
+    h->charge_per_face = c && c[0] == '0';
   }
   int hb_slab = 4, hb_spc = 1024, hb_lag = 2;
   {

@@ -137,21 +137,46 @@ struct WordStream {
 __device__ __forceinline__ WordStream words_at(uint64_t sk, uint64_t w0) { return WordStream{sk + (w0 + 1) * kGolden}; }
 __device__ __forceinline__ uint32_t lo32(uint64_t r) { return (uint32_t)r; }
 __device__ __forceinline__ uint32_t hi32(uint64_t r) { return (uint32_t)(r >> 32); }
+// The conversions below put the random bits into the low mantissa of a power of
+// two and subtract it: exact, and two FP64 operations where an integer
+// conversion goes through the quarter-rate unit.
 // uniform in (0,1) from 32 bits: (k + 1/2) 2^-32, exact and symmetric about 1/2
-__device__ __forceinline__ double u32(uint32_t k) { return fma((double)k, 0x1p-32, 0x1p-33); }
-// variance-1 uniform in (-sqrt3, sqrt3) from 32 bits: ((k + 1/2) 2^-31 - 1) sqrt3;
-// the bracket is exact, the product rounds once
-__device__ __forceinline__ double v32(uint32_t k) {
-  return __dmul_rn(fma((double)k, 0x1p-31, 0x1p-32 - 1.0), 1.7320508075688772);
+__device__ __forceinline__ double u32(uint32_t k) {
+  return __hiloint2double(0x41300000, (int)k) - (0x1p20 - 0x1p-33);  // 2^20 + k 2^-32
 }
+// variance-1 uniform in (-sqrt3, sqrt3) from 32 bits: (2 u32 - 1) sqrt3; the
+// bracket is exact, the product rounds once
+__device__ __forceinline__ double v32(uint32_t k) { return __dmul_rn(fma(u32(k), 2.0, -1.0), 1.7320508075688772); }
 
-// uniform in [0,1) from the top 53 bits (exact conversion)
-__device__ __forceinline__ double u53(uint64_t r) { return (double)(r >> 11) * 0x1p-53; }
+// uniform in [0,1) from the top 53 bits: the top 32, then the 21 below them (exact)
+__device__ __forceinline__ double u53(uint64_t r) {
+  const double h = __hiloint2double(0x41300000, (int)(r >> 32)) - (0x1p20 + 0.5);    // top 32 bits - 1/2
+  const double l = __hiloint2double(0x43300000, (int)((uint32_t)r >> 11));           // 2^52 + the next 21
+  return fma(l, 0x1p-53, h);
+}
 // variance-1 uniform in [-sqrt3, sqrt3): (2u - 1) is exact, one rounding in the product
 __device__ __forceinline__ double var1(uint64_t r) {
-  const double t = 2.0 * u53(r) - 1.0;
-  return __dmul_rn(t, 1.7320508075688772);
+  const double h = fma(__hiloint2double(0x41300000, (int)(r >> 32)), 2.0, -(0x1p21 + 2.0));
+  const double l = __hiloint2double(0x43300000, (int)((uint32_t)r >> 11));
+  return __dmul_rn(fma(l, 0x1p-52, h), 1.7320508075688772);
 }
+
+// Metropolis test r < e^{-dS} for a uniform r whose top 32 bits are hi.  2^32
+// e^{-dS} in single precision decides every case it can: up to dS = 22 its
+// relative error is below 2^-17 (the roundings of dS and of the exponent, and
+// the hardware's 2^x), beyond that it is below the absolute slack, which also
+// covers the bits of r under hi.  `exact` decides the rest (about 1 in 10^4),
+// NaN among them, so the outcome is that of the double-precision test.
+template <typename F>
+__device__ __forceinline__ bool metropolis(uint32_t hi, double dS, F exact) {
+  const float x = fmaf(__double2float_rn(dS), -1.4426950408889634f, 32.0f), r = __uint2float_rn(hi);
+  float e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x));
+  if (r < fmaf(e, 1.0f - 0x1p-15f, -4.0f)) return true;
+  if (r > fmaf(e, 1.0f + 0x1p-15f, 4.0f)) return false;
+  return exact();
+}
+
 // Box-Muller pair, u1 = 1 - u53(ra) in (0,1], angle 2*pi*u53(rb)
 __device__ __forceinline__ void box_muller(uint64_t ra, uint64_t rb, double &z0, double &z1) {
   const double u1 = 1.0 - u53(ra);

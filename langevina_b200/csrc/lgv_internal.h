@@ -41,15 +41,11 @@ struct ChargeArgs {
   MonAcc *mon;
 };
 
-// Both faces of one direction of the charge heat bath.
+// Both faces of one direction of the charge heat bath (counter noise).
 struct ChargeDirPair {
   double rms, inv2chi;
-  uint64_t sk[2];     // sub-step keys of the two faces
-  int pass[2];        // positions of the faces in the step (0..5)
-  int eo[2];          // A-site parities, in application order
-  const double *q, *acc;  // injected [6][6][V] or null
-  uint8_t *flags;
-  MonAcc *mon;
+  uint64_t sk[2];  // sub-step keys of the two faces
+  int eo[2];       // A-site parities, in application order
 };
 
 struct EmArgs {
@@ -265,13 +261,9 @@ cudaError_t hb_plan_timeouts(const HbPlan &plan, cudaStream_t st, unsigned long 
 cudaError_t launch_hb_sweep(Fields in, Fields out, int N, const HbArgs &a, cudaStream_t st);
 cudaError_t launch_charge_pass(Fields f, int N, int dir, int eoA, const ChargeArgs &a, cudaStream_t st);
 cudaError_t launch_charge_pass(Fields f, const Geo &g, int dir, int eoA, const ChargeArgs &a, cudaStream_t st);
-// Both faces of direction dir.  x runs in place on `in`; y and z read `in`
-// and write the charges of `out` (*swapped = true: the caller swaps the
-// charge planes).
-// shared-memory slab kernel for both faces of a direction (N divisible by 32)
-bool charge_slab_supported(int N);
-cudaError_t launch_charge_dir(Fields in, Fields out, int N, int dir, const ChargeDirPair &p, cudaStream_t st,
-                              bool *swapped);
+// Both faces of direction dir of a whole lattice: reads the charges of `in`,
+// writes those of `out`.
+cudaError_t launch_charge_dir(Fields in, Fields out, const Geo &g, int dir, const ChargeDirPair &p, cudaStream_t st);
 cudaError_t launch_em(Fields in, Fields out, int N, const EmArgs &a, cudaStream_t st);
 cudaError_t launch_ideal(Fields in, Fields out, int N, const IdealArgs &a, cudaStream_t st);
 cudaError_t launch_em(Fields in, Fields out, const Geo &g, const EmArgs &a, cudaStream_t st);

@@ -7,9 +7,8 @@
 //   hb_sweep_kernel     the same, both parities in one z-marching launch (opt-in)
 //   charge_pass_kernel  ModelGChargeHB::step, one (direction, parity) face
 //                       (Stepper.cxx:471-518, modelg_update_charge_pair :419-441)
-//   charge_slab_kernel, both faces of one direction per launch (opt-in):
-//   charge_x_kernel,    shared-memory slabs for N divisible by 32, otherwise x
-//   charge_line_kernel  rows per CTA and y, z streamed lines with two-site halos
+//   charge_row_kernel,  both faces of one direction per launch: x rows per
+//   charge_run_kernel   block; y and z runs of sites per thread
 //   ideal_kernel        IdealPV2::step_no_reject fused: half rotation, charge
 //                       advection stencil, half rotation (Stepper.cxx:68-202);
 //                       the TMA-staged ideal_tma_kernel (lgv_ideal_tma.cu)
@@ -26,6 +25,7 @@
 #include "lgv_dft.cuh"
 #include "lgv_ideal_tma_cta.cuh"
 #include "lgv_internal.h"
+#include "lgv_pdl.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -323,8 +323,12 @@ __device__ __forceinline__ void hb_decide(const double po[4], const double heff[
     r.accept = true;
     r.flag = 1;
   } else {
-    const double u = INJECTED ? a.acc[nat] : u53(rng.next());
-    r.accept = u < exp(-r.dS);
+    if (INJECTED) {
+      r.accept = a.acc[nat] < exp(-r.dS);
+    } else {
+      const uint64_t w = rng.next();
+      r.accept = metropolis((uint32_t)(w >> 32), r.dS, [&] { return u53(w) < exp(-r.dS); });
+    }
     r.flag = r.accept ? 2 : 0;
   }
 }
@@ -814,6 +818,17 @@ __global__ void __launch_bounds__(HB_TM *HB_TY, 2) hb_sweep_kernel(Fields in, Fi
 }
 
 // ----------------------------------------------------------------------------
+// Action change of moving q from A to B (modelg_update_charge_pair,
+// Stepper.cxx:419-441): ((nA-q)^2 + (nB+q)^2 - nA^2 - nB^2) / (2 chi), the
+// squares multiplied out.
+__device__ __forceinline__ double charge_dS(double nA, double nB, double q, double invchi) {
+  return (q * invchi) * (q + (nB - nA));
+}
+// Accept with the 32-bit uniform of hi.
+__device__ __forceinline__ bool charge_accept(double dS, uint32_t hi) {
+  return metropolis(hi, dS, [&] { return dS < 0 || u32(hi) < exp(-dS); });
+}
+
 // Charge heat bath, one face (direction `dir`, A-site parity eoA).  One thread
 // per link (A, B = A + e_dir); the links of a face are disjoint, so the update
 // is race free and conserves each charge exactly (Stepper.cxx:493-517).
@@ -853,25 +868,16 @@ __device__ __forceinline__ void charge_link_site(const Fields &f, const Geo &g, 
       v = v32(lo32(ra));
     }
     const double q = a.rms * v;
-    const double dA = nA - q, dB = nB + q;
-    const double dS = (dA * dA + dB * dB - nA * nA - nB * nB) * a.inv2chi;
-    bool accept;
-    uint8_t fl;
-    if (dS < 0) {
-      accept = true;
-      fl = 1;
-      if (MON) mon.down(dS);
-    } else {
-      const double r = INJECTED ? a.acc[ii] : u32(hi32(ra));
-      accept = r < exp(-dS);
-      fl = accept ? 2 : 0;
-      if (MON) {
-        if (accept) mon.up_yes(dS);
-        else mon.up_no();
-      }
+    const double dS = charge_dS(nA, nB, q, 2.0 * a.inv2chi);
+    const bool accept = INJECTED ? dS < 0 || a.acc[ii] < exp(-dS) : charge_accept(dS, hi32(ra));
+    const uint8_t fl = dS < 0 ? 1 : accept ? 2 : 0;
+    if (MON) {
+      if (fl == 1) mon.down(dS);
+      else if (fl == 2) mon.up_yes(dS);
+      else mon.up_no();
     }
     if (accept) {
-      P[offA] = nA + (-q);
+      P[offA] = nA - q;
       P[offB] = nB + q;
     }
     if (a.flags) a.flags[ii] = fl;
@@ -890,347 +896,175 @@ __global__ void __launch_bounds__(128, 16) charge_pass_kernel(Fields f, Geo g, i
 }
 
 // ----------------------------------------------------------------------------
-// Charge heat bath, both parity passes of one direction in one launch
-// (ModelGChargeHB::step, Stepper.cxx:471-518): the two faces (dir, eo[0]) and
-// (dir, eo[1]) are applied in that order.  Every link update is
-// modelg_update_charge_pair (:419-441) for the six charges at once, drawing
-// from the counter stream of its pass keyed by the link's A site.
+// Charge heat bath, both faces of one direction per launch, one charge per
+// thread (ModelGChargeHB::step, Stepper.cxx:471-518).  The six charges do not
+// mix, so a thread takes one charge of a run of sites along the direction,
+// applies the first face (dir, eo[0]) and then the second (dir, eo[1]) in
+// registers and writes every site once: 16 B per site, charge and direction
+// instead of the 32 that two one-face passes move.  Reads `in`, writes `out`.
+// Links, words and outcomes are those of charge_link_site.  A charge step: 32^3
+// 37 -> 10 us, 64^3 49 -> 22, 90^3 87 -> 56, 128^3 -> 127, 160^3 400 -> 252,
+// 256^3 1684 -> 980 (5.0 TB/s of the 288 B/site that three directions move at
+// least).  Issue bounds it (74-79 % active at 160^3: 78 instructions per link
+// of one charge in y and z, 96 in x, most of them the word's two 64-bit
+// products and shifts), then DRAM.
 struct ChargeDirArgs {
-  double rms, inv2chi;
+  const double *in;  // charge 0 of six evenly spaced planes
+  double *out;
+  long long pitch_in, pitch_out;
+  double rms, invchi;
   uint64_t sk[2];
-  int pass[2];  // positions of the two faces in the step (injected indexing / flags)
   int eo[2];
-  const double *q, *acc;
-  uint8_t *flags;
-  MonAcc *mon;
 };
 
-template <bool INJECTED, bool MON>
-__device__ __forceinline__ void charge_link(double nA[6], double nB[6], const ChargeDirArgs &a, int pi,
-                                            long long natA, long long V, bool own, MonLocal &mon) {
-  WordStream ws{};
-  if (!INJECTED) ws = words_at(a.sk[pi], 6 * (uint64_t)natA);
-#pragma unroll
-  for (int L = 0; L < 6; ++L) {
-    const long long ii = (long long)(a.pass[pi] * 6 + L) * V + natA;
-    uint64_t ra = 0;
-    double v;
-    if (INJECTED) {
-      v = a.q[ii];
-    } else {
-      ra = ws.next();
-      v = v32(lo32(ra));
-    }
-    const double q = a.rms * v;
-    const double dA = nA[L] - q, dB = nB[L] + q;
-    const double dS = (dA * dA + dB * dB - nA[L] * nA[L] - nB[L] * nB[L]) * a.inv2chi;
-    bool accept;
-    uint8_t fl;
-    if (dS < 0) {
-      accept = true;
-      fl = 1;
-    } else {
-      const double r = INJECTED ? a.acc[ii] : u32(hi32(ra));
-      accept = r < exp(-dS);
-      fl = accept ? 2 : 0;
-    }
-    if (own) {
-      if (MON) {
-        if (fl == 1) mon.down(dS);
-        else if (fl == 2) mon.up_yes(dS);
-        else mon.up_no();
-      }
-      if (a.flags) a.flags[ii] = fl;
-    }
-    if (accept) {
-      nA[L] = nA[L] + (-q);
-      nB[L] = nB[L] + q;
-    }
+// One link of one charge: word z of the face's sequence gives the proposal and
+// the accept uniform; updates nA and nB.
+__device__ __forceinline__ void charge_link(double &nA, double &nB, uint64_t z, double rms, double invchi) {
+  const uint64_t r = mix64(z);
+  const double q = rms * v32(lo32(r));
+  const bool yes = charge_accept(charge_dS(nA, nB, q, invchi), hi32(r));
+  if (yes) {
+    nA -= q;
+    nB += q;
   }
 }
 
-// x direction.  A CTA owns whole rows (blockDim.x = N/2, blockDim.y rows);
-// thread m holds natural sites 2m and 2m+1 of its row (element m of both
-// parity half-rows).  Of the two x faces one pairs (2m, 2m+1) inside the
-// thread, the other pairs (2m+1, 2m+2) across threads: its A-site owner
-// computes it and hands the B site's new charges over through shared memory.
-template <bool INJECTED, bool MON>
-__global__ void __launch_bounds__(256) charge_x_kernel(Fields f, Geo g, ChargeDirArgs a) {
-  extern __shared__ double xs[];  // [6][blockDim.y][H]
-  const int H = g.H, N = g.N;
-  const int m = threadIdx.x, ty = threadIdx.y;
-  const long long R = (long long)blockIdx.x * blockDim.y + ty;
-  const bool valid = R < (long long)N * N;
-  const int j = valid ? (int)(R % N) : 0, k = valid ? (int)(R / N) : 0;
-  const int r = (j + k) & 1;  // parity of site 2m
-  const long long row = ((long long)k * N + j) * H;
-  const long long V = 2 * g.V2;
-  const long long offa = (long long)r * g.V2 + row + m, offb = (long long)(r ^ 1) * g.V2 + row + m;
-  double va[6], vb[6];
-  MonLocal mon;
-  if (valid) {
-#pragma unroll
-    for (int L = 0; L < 6; ++L) {
-      va[L] = f.c[4 + L][offa];
-      vb[L] = f.c[4 + L][offb];
-    }
-  }
-  double *sh = xs + (size_t)ty * H;
-  const size_t lstride = (size_t)blockDim.y * H;
-  const long long nat0 = ((long long)k * N + j) * N + 2 * m;
-  // Rows of a CTA differ in parity, so some take the in-thread face while
-  // others take the cross face: every thread runs the exchange barriers of
-  // both faces, and only the work between them is conditional.
-  const int mr = (m + 1 == H) ? 0 : m + 1;
-#pragma unroll
-  for (int pi = 0; pi < 2; ++pi) {
-    const bool cross = a.eo[pi] != r;
-    if (valid && !cross) charge_link<INJECTED, MON>(va, vb, a, pi, nat0, V, true, mon);
-    // cross link (2m+1, 2m+2): B is thread m+1's site 2m+2
-    if (valid && cross) {
-#pragma unroll
-      for (int L = 0; L < 6; ++L) sh[L * lstride + m] = va[L];
-    }
-    __syncthreads();
-    double nb[6];
-    if (valid && cross) {
-#pragma unroll
-      for (int L = 0; L < 6; ++L) nb[L] = sh[L * lstride + mr];
-      charge_link<INJECTED, MON>(vb, nb, a, pi, nat0 + 1, V, true, mon);
-    }
-    __syncthreads();
-    if (valid && cross) {
-#pragma unroll
-      for (int L = 0; L < 6; ++L) sh[L * lstride + mr] = nb[L];
-    }
-    __syncthreads();
-    if (valid && cross) {
-#pragma unroll
-      for (int L = 0; L < 6; ++L) va[L] = sh[L * lstride + m];
-    }
-    __syncthreads();
-  }
-  if (valid) {
-#pragma unroll
-    for (int L = 0; L < 6; ++L) {
-      f.c[4 + L][offa] = va[L];
-      f.c[4 + L][offb] = vb[L];
-    }
-  }
-  if (MON) mon_flush(mon, a.mon);
-}
-
-// y (DIR = 1) and z (DIR = 2) directions.  A thread owns element m of the
-// parity half-rows along one line (natural columns x = 2m and 2m+1) and
-// streams through a segment [s0, s1) of the line plus two sites either side.
-// Along a column the two faces alternate link by link, so as site t arrives
-// the first face's link (t-1, t) and then the second face's link (t-2, t-1)
-// are applied (three-site register window); a site is final after its second
-// face link.  Links in the halo are recomputed bit for bit by the thread that
-// owns them, so segments are independent; because halos are read while
-// neighbours write, the kernel reads `in` and writes `out`.
-template <int DIR, bool INJECTED, bool MON>
-__global__ void __launch_bounds__(128) charge_line_kernel(Fields in, Fields out, Geo g, ChargeDirArgs a, int seglen) {
-  const int H = g.H, N = g.N;
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c2 = blockIdx.y;  // k for DIR = 1, j for DIR = 2
-  const int s0 = blockIdx.z * seglen;
-  const int s1 = min(s0 + seglen, N);
-  const long long V = 2 * g.V2;
-  MonLocal mon;
-  if (m < H) {
-    double w0[2][6], w1[2][6], w2[2][6];  // sites t-2, t-1, t; [column a (x=2m) / b (x=2m+1)][charge]
-    const int e1 = a.eo[0], e2 = a.eo[1];
-    const int n = (s1 - s0) + 4;
-    int tm1 = 0, jm1 = 0, km1 = 0, tm2 = 0, jm2 = 0, km2 = 0;
-    for (int u = 0; u < n; ++u) {
-      const int t = s0 - 2 + u;  // line position (unwrapped)
-      const int tw = wrapn(t, N);
-      const int j = DIR == 1 ? tw : c2, k = DIR == 1 ? c2 : tw;
-      const int ra = (j + k) & 1;  // parity of column a's site at t
-      const long long row = ((long long)k * N + j) * H + m;
-#pragma unroll
-      for (int L = 0; L < 6; ++L) {
-        w2[0][L] = in.c[4 + L][(long long)ra * g.V2 + row];
-        w2[1][L] = in.c[4 + L][(long long)(ra ^ 1) * g.V2 + row];
-      }
-      if (u >= 1) {
-        const int rpa = (jm1 + km1) & 1;  // parity of column a at t-1
-#pragma unroll
-        for (int col = 0; col < 2; ++col) {
-          const int par = rpa ^ col;  // parity of this column's site at t-1
-          if (par == e1) {  // first face: link (t-1, t), A = t-1
-            const long long natA = ((long long)km1 * N + jm1) * N + 2 * m + col;
-            charge_link<INJECTED, MON>(w1[col], w2[col], a, 0, natA, V, (t - 1) >= s0 && (t - 1) < s1, mon);
-          }
-          if (u >= 3 && (par ^ 1) == e2) {  // second face: link (t-2, t-1), A = t-2
-            const long long natA = ((long long)km2 * N + jm2) * N + 2 * m + col;
-            charge_link<INJECTED, MON>(w0[col], w1[col], a, 1, natA, V, (t - 2) >= s0 && (t - 2) < s1, mon);
-            // sites t-2 and t-1 of this column are final
-            if ((t - 2) >= s0 && (t - 2) < s1) {
-              const long long o2 = (long long)(((jm2 + km2) & 1) ^ col) * g.V2 + ((long long)km2 * N + jm2) * H + m;
-#pragma unroll
-              for (int L = 0; L < 6; ++L) out.c[4 + L][o2] = w0[col][L];
-            }
-            if ((t - 1) >= s0 && (t - 1) < s1) {
-              const long long o1 = (long long)(rpa ^ col) * g.V2 + ((long long)km1 * N + jm1) * H + m;
-#pragma unroll
-              for (int L = 0; L < 6; ++L) out.c[4 + L][o1] = w1[col][L];
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int L = 0; L < 6; ++L) {
-          w0[c][L] = w1[c][L];
-          w1[c][L] = w2[c][L];
-        }
-      tm2 = tm1; jm2 = jm1; km2 = km1;
-      tm1 = tw; jm1 = j; km1 = k;
-    }
-    (void)tm2;
-  }
-  if (MON) mon_flush(mon, a.mon);
-}
-
-// ----------------------------------------------------------------------------
-// Both faces of one charge direction per launch, staged in shared memory.
-// The CTA copies its slab of the six charge planes to shared memory with
-// coalesced half-row loads, applies every link of the first face, then every
-// link of the second, and writes the slab back: the two faces cost one read
-// and one write of the charges instead of two of each.
-//   x (DIR 0): the slab is `nrows` whole rows (no halo: x links stay in a row).
-//   y, z (DIR 1, 2): 32 natural columns (16 elements of each parity half-row)
-//   along a segment [s0, s1) of the line at fixed k (y) or j (z), plus two
-//   sites either side; halo links are recomputed bit for bit, only links whose
-//   A site lies in the segment count in monitors and flags, and only segment
-//   sites are written, so the kernel reads `in` and writes `out`.
-// Links are the same charge_link updates, streams and order as the per-face
-// kernels (Stepper.cxx:471-518).
-constexpr int kSlabThreads = 256;
-
-template <int DIR, bool INJECTED, bool MON>
-__global__ void __launch_bounds__(kSlabThreads) charge_slab_kernel(Fields in, Fields out, Geo g, ChargeDirArgs a,
-                                                                   int seglen, int nrows) {
-  extern __shared__ double S[];
+// y (DIR 1) and z (DIR 2), one run: charge L of the sites b0 .. b0 + len - 1
+// along the direction at fixed i and o (k or j); b0 = c0 or c0 + 1, the one
+// whose site is an A site of the second face.  Its own second-face links are
+// (b0, b0 + 1), (b0 + 2, b0 + 3), ..., and the first-face links they need
+// (b0 - 1, b0), (b0 + 1, b0 + 2), ...: one more than its share, the link it has
+// in common with the next run.  Offsets (I) are in bytes.  WRAP: the run may
+// reach past N - 1.
+template <int DIR, bool WRAP, typename I>
+__device__ __forceinline__ void charge_run(const Geo &g, int L, int i, int o, int c0, int len, const ChargeDirArgs &a) {
   const int N = g.N, H = g.H;
-  const long long V2 = g.V2, V = 2 * V2;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  MonLocal mon;
-  if (DIR == 0) {
-    const long long R0 = (long long)blockIdx.x * nrows;
-    const int nr = (int)min((long long)nrows, (long long)N * N - R0);
-    // S[L][r][h][m]
-    // 16-byte cp.async: every load of the slab in flight at once
-    const int HC = H / 2;  // 16-byte chunks per half row
-#pragma unroll
-    for (int L = 0; L < 6; ++L)  // static component index: Fields stays in the parameter space
-      for (int e = tid; e < nr * H; e += kSlabThreads) {
-        const int r = e / H, cc = e - r * H;
-        const int h = cc >= HC ? 1 : 0, m = 2 * (cc - h * HC);
-        cp_async16(&S[((L * nrows + r) * 2 + h) * H + m], in.c[4 + L] + h * V2 + (R0 + r) * H + m);
-      }
-    cp_async_commit();
-    cp_async_wait_all();
-    __syncthreads();
-#pragma unroll
-    for (int pi = 0; pi < 2; ++pi) {  // static face index: the arguments stay in the parameter space
-      const int eo = a.eo[pi];
-      for (int e = tid; e < nr * H; e += kSlabThreads) {
-        const int r = e / H, u = e - r * H;
-        const long long R = R0 + r;
-        const int j = (int)(R % N), k = (int)(R / N);
-        const int sA = (eo + j + k) & 1;  // A sites at i = 2u + sA
-        {
-          const int iA = 2 * u + sA;
-          const int iB = (iA + 1 == N) ? 0 : iA + 1;
-          double *pa = S + ((size_t)r * 2 + eo) * H + u;
-          double *pb = S + ((size_t)r * 2 + (eo ^ 1)) * H + (iB >> 1);
-          const size_t ls = (size_t)nrows * 2 * H;
-          double nA[6], nB[6];
-#pragma unroll
-          for (int L = 0; L < 6; ++L) {
-            nA[L] = pa[L * ls];
-            nB[L] = pb[L * ls];
-          }
-          charge_link<INJECTED, MON>(nA, nB, a, pi, R * N + iA, V, true, mon);
-#pragma unroll
-          for (int L = 0; L < 6; ++L) {
-            pa[L * ls] = nA[L];
-            pb[L * ls] = nB[L];
-          }
-        }
-      }
-      __syncthreads();
+  const int P0 = a.eo[1];  // parity of the sites b0, b0 + 2, ...
+  const int b0 = c0 + ((P0 ^ (i + o)) & 1);
+  const I base = 8 * ((DIR == 1 ? (I)o * N * H : (I)o * H) + (i >> 1));
+  const I E = 8 * ((I)P0 * (I)g.V2) + base, O = 8 * ((I)(P0 ^ 1) * (I)g.V2) + base;
+  const I str = 8 * (DIR == 1 ? (I)H : (I)N * H), adv = 2 * str, lap = (I)N * str;
+  const double *in = a.in + L * a.pitch_in;
+  double *out = a.out + L * a.pitch_out;
+  auto ld = [&](I off) { return *(const double *)((const char *)in + off); };
+  auto st = [&](I off, double x) { *(double *)((char *)out + off) = x; };
+  auto wrap = [&](int c) { return c >= N ? c - N : c; };
+  // word of the link whose A site has coordinate c: (6 nat + L + 1) golden
+  const uint64_t ns = DIR == 1 ? (uint64_t)N : (uint64_t)N * N;
+  const uint64_t nb = DIR == 1 ? (uint64_t)o * N * N + i : (uint64_t)o * N + i;
+  const uint64_t dz = 12 * ns * kGolden, zlap = 6 * ns * N * kGolden, zb = (6 * nb + L + 1) * kGolden;
+  const int cm = b0 == 0 ? N - 1 : b0 - 1, c1 = wrap(b0 + 1), c2 = wrap(b0 + 2);
+  uint64_t z2 = a.sk[1] + zb + 6 * ns * b0 * kGolden;  // second face, A site c
+  uint64_t z1 = a.sk[0] + zb + 6 * ns * c1 * kGolden;  // first face, A site c + 1
+  const uint64_t zm = a.sk[0] + zb + 6 * ns * cm * kGolden;
+  I se = E + (I)b0 * str, so = O + (I)c1 * str;  // where this pair of sites goes
+  I le = E + (I)c2 * str;                        // the even site read last
+  const I endE = E + lap, endO = O + lap;
+  pdl_wait();
+  double vm = ld(O + (I)cm * str), p = ld(se), x = ld(so), y = ld(le);
+  charge_link(vm, p, zm, a.rms, a.invchi);
+  for (int q = len >> 1; q > 0; --q) {
+    I no = so + adv;
+    le += adv;
+    bool over = false;
+    if (WRAP) {
+      over = no >= endO;
+      if (over) no -= lap;
+      if (le >= endE) le -= lap;
     }
-#pragma unroll
-    for (int L = 0; L < 6; ++L)
-      for (int r = 0; r < nr; ++r)
-        for (int e = tid; e < 2 * H; e += kSlabThreads) {
-          const int h = e >= H ? 1 : 0, m = e - h * H;
-          out.c[4 + L][h * V2 + (R0 + r) * H + m] = S[((L * nrows + r) * 2 + h) * H + m];
-        }
-  } else {
-    const int x0 = blockIdx.x * 32, m0 = x0 >> 1;
-    const int c2 = blockIdx.y;  // k for y lines, j for z lines
-    const int s0 = blockIdx.z * seglen, s1 = min(s0 + seglen, N);
-    const int W = (s1 - s0) + 4;  // window positions t = s0 - 2 + w
-    // S[L][w][h][mm]: 32 doubles per (L, w)
-    const int h = lane >> 4, mm = lane & 15;
-    // 16-byte cp.async: every load of the slab in flight at once
-#pragma unroll
-    for (int L = 0; L < 6; ++L)
-      for (int e = tid; e < W * 16; e += kSlabThreads) {
-        const int w = e >> 4, cc = e & 15;
-        const int hc = cc >> 3, mc = 2 * (cc & 7);
-        const int t = wrapn(s0 - 2 + w, N);
-        const int j = DIR == 1 ? t : c2, k = DIR == 1 ? c2 : t;
-        cp_async16(&S[((L * W + w) * 2 + hc) * 16 + mc], in.c[4 + L] + hc * V2 + ((long long)k * N + j) * H + m0 + mc);
-      }
-    cp_async_commit();
-    cp_async_wait_all();
-    __syncthreads();
-    const size_t ls = (size_t)W * 32;
-    const int lx = lane;  // natural column x0 + lx
-#pragma unroll
-    for (int pi = 0; pi < 2; ++pi) {
-      const int eo = a.eo[pi];
-      const int w0 = (eo + lx + c2 + s0) & 1;  // A sites of this column at w = w0 + 2u
-      // first face: every link inside the window; second face: links with both ends in [1, W-2]
-      const int wlo = pi == 0 ? 0 : 1, whi = pi == 0 ? W - 1 : W - 2;
-      for (int w = w0 + 2 * warp; w + 1 <= whi; w += 2 * (kSlabThreads / 32)) {
-        if (w < wlo) continue;
-        const int tA = wrapn(s0 - 2 + w, N);
-        const int j = DIR == 1 ? tA : c2, k = DIR == 1 ? c2 : tA;
-        double *pa = S + ((size_t)w * 2 + eo) * 16 + (lx >> 1);
-        double *pb = S + ((size_t)(w + 1) * 2 + (eo ^ 1)) * 16 + (lx >> 1);
-        double nA[6], nB[6];
-#pragma unroll
-        for (int L = 0; L < 6; ++L) {
-          nA[L] = pa[L * ls];
-          nB[L] = pb[L * ls];
-        }
-        const bool own = (w - 2) >= 0 && (w - 2) < (s1 - s0);
-        charge_link<INJECTED, MON>(nA, nB, a, pi, ((long long)k * N + j) * N + x0 + lx, V, own, mon);
-#pragma unroll
-        for (int L = 0; L < 6; ++L) {
-          pa[L * ls] = nA[L];
-          pb[L * ls] = nB[L];
-        }
-      }
-      __syncthreads();
+    double xn = 0, yn = 0;
+    if (q > 1) {
+      xn = ld(no);
+      yn = ld(le);
     }
-#pragma unroll
-    for (int L = 0; L < 6; ++L)
-      for (int w = 2 + warp; w < W - 2; w += kSlabThreads / 32) {
-        const int t = s0 - 2 + w;
-        const int j = DIR == 1 ? t : c2, k = DIR == 1 ? c2 : t;
-        out.c[4 + L][h * V2 + ((long long)k * N + j) * H + m0 + mm] = S[(L * W + w) * 32 + lane];
-      }
+    charge_link(x, y, z1, a.rms, a.invchi);
+    charge_link(p, x, z2, a.rms, a.invchi);
+    st(se, p);
+    st(so, x);
+    p = y;
+    x = xn;
+    y = yn;
+    se += adv;
+    so = no;
+    z2 += dz;
+    z1 += dz;
+    if (WRAP && over) z1 -= zlap;
   }
-  if (MON) mon_flush(mon, a.mon);
+}
+
+constexpr int kRunThreads = 128;
+
+// Thread = site of the plane across the direction (lanes along m of one x
+// parity), blockIdx.y = run, blockIdx.z = charge.
+template <int DIR, typename I>
+__global__ void __launch_bounds__(kRunThreads) charge_run_kernel(Geo g, ChargeDirArgs a, int seg) {
+  pdl_launch();
+  const unsigned idx = blockIdx.x * kRunThreads + threadIdx.x;
+  const int N = g.N, L = g.zrev ? 5 - (int)blockIdx.z : (int)blockIdx.z;
+  const int q = (int)(idx / (unsigned)N), t = (int)(idx - (unsigned)q * N);
+  if (q >= N) return;
+  const int o = g.zrev ? N - 1 - q : q, s = t >= g.H ? 1 : 0, i = 2 * (t - s * g.H) + s;
+  const int c0 = (int)blockIdx.y * seg, len = min(seg, N - c0);
+  if (c0 + len < N) charge_run<DIR, false, I>(g, L, i, o, c0, len, a);
+  else charge_run<DIR, true, I>(g, L, i, o, c0, len, a);
+}
+
+// x.  A block holds whole rows (blockDim.x = N/2, blockDim.y rows) of charges
+// L0 .. L0 + nl - 1, one after the other.  Thread m of a row holds the pair of
+// sites that first-face link m joins, A and B; the second-face link joins its B
+// with the A of thread m + 1, which comes through shared memory (two slots in
+// turn, so one barrier per charge), and the thread writes both.
+__device__ __forceinline__ void charge_row(const Geo &g, int L0, int nl, int m, int row, bool valid,
+                                           const ChargeDirArgs &a, double *sh, int slot) {
+  const int N = g.N, H = g.H;
+  const int j = row % N, k = row / N, b = (a.eo[0] ^ (j + k)) & 1;  // A of link m is site 2m + b
+  const int xb = 2 * m + b + 1 == N ? 0 : 2 * m + b + 1, mn = m + 1 == H ? 0 : m + 1;
+  const long long r = (long long)row * H;
+  const long long oa = (long long)a.eo[0] * g.V2 + r, ob = (long long)a.eo[1] * g.V2 + r + (xb >> 1);
+  const uint64_t nat = (uint64_t)row * N;
+  uint64_t z1 = a.sk[0] + (6 * (nat + 2 * m + b) + L0 + 1) * kGolden;
+  uint64_t z2 = a.sk[1] + (6 * (nat + xb) + L0 + 1) * kGolden;
+  const double *ia = a.in + L0 * a.pitch_in + oa + m, *ib = a.in + L0 * a.pitch_in + ob;
+  double *wa = a.out + L0 * a.pitch_out + oa + mn, *wb = a.out + L0 * a.pitch_out + ob;
+  pdl_wait();
+  double an = 0, bn = 0;
+  if (valid) {
+    an = *ia;
+    bn = *ib;
+  }
+  for (int l = 0; l < nl; ++l) {
+    double A = an, B = bn;
+    ia += a.pitch_in;
+    ib += a.pitch_in;
+    if (valid && l + 1 < nl) {
+      an = *ia;
+      bn = *ib;
+    }
+    charge_link(A, B, z1, a.rms, a.invchi);
+    double *s = sh + (l & 1) * slot;
+    s[m] = A;
+    __syncthreads();
+    A = s[mn];
+    charge_link(B, A, z2, a.rms, a.invchi);
+    if (valid) {
+      *wb = B;
+      *wa = A;
+    }
+    wa += a.pitch_out;
+    wb += a.pitch_out;
+    z1 += kGolden;
+    z2 += kGolden;
+  }
+}
+
+__global__ void __launch_bounds__(1024) charge_row_kernel(Geo g, ChargeDirArgs a, int nl) {
+  extern __shared__ double xs[];  // [2][blockDim.y][H]
+  pdl_launch();
+  const int rows = g.N * g.N, id = blockIdx.x * blockDim.y + threadIdx.y;
+  const int L0 = nl * (g.zrev ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y);
+  const bool valid = id < rows;
+  const int row = valid ? (g.zrev ? rows - 1 - id : id) : 0;
+  charge_row(g, L0, nl, threadIdx.x, row, valid, a, xs + (size_t)threadIdx.y * g.H, blockDim.y * g.H);
 }
 
 // ----------------------------------------------------------------------------
@@ -2978,103 +2812,49 @@ cudaError_t launch_charge_pass(Fields f, const Geo &g, int dir, int eoA, const C
   return cudaGetLastError();
 }
 
-static int charge_seglen(int N) { return N >= 64 ? 32 : N; }
+// Sites per run along y and z: a run of `seg` sites repeats one of its seg
+// links, shorter runs are more threads.  The longest of 32, 16 and 8 that leaves
+// two rounds of resident threads (a charge step measured at 8 / 16 / 32 / 64:
+// 64^3 23.6 / 28.7 / - / 39 us, 128^3 143 / 138 / - / 148, 256^3 1205 / 1143 /
+// 1097 / 1106).
+static int charge_seg(int N) {
+  int seg = 32;
+  while (seg > 8 && 6LL * N * N * ((N + seg - 1) / seg) < 2LL * 148 * 2048) seg >>= 1;
+  return std::min(seg, N);
+}
 
-bool charge_slab_supported(int N) { return N >= 32 && N % 32 == 0 && N <= 2048; }
+// Charges per thread along x: all six (the row's indices are worked out once;
+// 256^3 982 us a charge step against 1152 at one each) unless that leaves the
+// chip short of threads (64^3: 22.4 us at three, 23.0 at six, 25.1 at one).
+static int charge_row_nl(const Geo &g) { return g.V2 >= 148LL * 2048 ? 6 : 3; }
 
-cudaError_t launch_charge_dir(Fields in, Fields out, int N, int dir, const ChargeDirPair &p, cudaStream_t st,
-                              bool *swapped) {
-  const Geo g = make_geo(N);
-  ChargeDirArgs a;
+cudaError_t launch_charge_dir(Fields in, Fields out, const Geo &g, int dir, const ChargeDirPair &p, cudaStream_t st) {
+  ChargeDirArgs a{};
+  a.in = in.c[4];
+  a.out = out.c[4];
+  a.pitch_in = in.c[5] - in.c[4];
+  a.pitch_out = out.c[5] - out.c[4];
+  for (int L = 0; L < 6; ++L)
+    if (in.c[4 + L] != a.in + L * a.pitch_in || out.c[4 + L] != a.out + L * a.pitch_out) return cudaErrorInvalidValue;
   a.rms = p.rms;
-  a.inv2chi = p.inv2chi;
+  a.invchi = 2.0 * p.inv2chi;
   for (int i = 0; i < 2; ++i) {
     a.sk[i] = p.sk[i];
-    a.pass[i] = p.pass[i];
     a.eo[i] = p.eo[i];
   }
-  a.q = p.q;
-  a.acc = p.acc;
-  a.flags = p.flags;
-  a.mon = p.mon;
-  const bool inj = a.q != nullptr, mon = a.mon != nullptr;
-  if (charge_slab_supported(N)) {
-    *swapped = true;
-    int sl = 0, nr = 0;
-    size_t sm = 0;
-    dim3 grid;
-    if (dir == 0) {
-      nr = (int)std::max(1, std::min(4, 512 / g.H));
-      sm = (size_t)6 * nr * 2 * g.H * sizeof(double);
-      grid = dim3((unsigned)(((long long)N * N + nr - 1) / nr));
-    } else {
-      sl = std::min(N, 32);
-      sm = (size_t)6 * (sl + 4) * 32 * sizeof(double);
-      grid = dim3(N / 32, N, (N + sl - 1) / sl);
-    }
-#define LGV_SLAB(D, I, M)                                                                   \
-  do {                                                                                      \
-    cudaError_t e_ = allow_smem(charge_slab_kernel<D, I, M>, sm);                           \
-    if (e_ != cudaSuccess) return e_;                                                       \
-    charge_slab_kernel<D, I, M><<<grid, kSlabThreads, sm, st>>>(in, out, g, a, sl, nr);     \
-  } while (0)
-#define LGV_SLAB_DIR(D) \
-  if (inj) { if (mon) LGV_SLAB(D, true, true); else LGV_SLAB(D, true, false); } \
-  else { if (mon) LGV_SLAB(D, false, true); else LGV_SLAB(D, false, false); }
-    if (dir == 0) { LGV_SLAB_DIR(0) }
-    else if (dir == 1) { LGV_SLAB_DIR(1) }
-    else { LGV_SLAB_DIR(2) }
-#undef LGV_SLAB_DIR
-#undef LGV_SLAB
-    return cudaGetLastError();
-  }
-  if (dir == 0 && g.H > 256) {
-    // rows longer than one 256-thread CTA: the two faces as separate launches
-    *swapped = false;
-    for (int i = 0; i < 2; ++i) {
-      ChargeArgs c{};
-      c.rms = p.rms;
-      c.inv2chi = p.inv2chi;
-      c.sk = p.sk[i];
-      c.pass = p.pass[i];
-      c.q = p.q;
-      c.acc = p.acc;
-      c.flags = p.flags;
-      c.mon = p.mon;
-      cudaError_t e = launch_charge_pass(in, N, 0, p.eo[i], c, st);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-  }
   if (dir == 0) {
-    *swapped = false;
-    const int H = g.H;
-    const int by = H >= 256 ? 1 : 256 / H;
-    const long long rows = (long long)N * N;
-    dim3 block(H, by), grid((unsigned)((rows + by - 1) / by));
-    const size_t sm = (size_t)6 * by * H * sizeof(double);
-    if (inj) {
-      if (mon) charge_x_kernel<true, true><<<grid, block, sm, st>>>(in, g, a);
-      else charge_x_kernel<true, false><<<grid, block, sm, st>>>(in, g, a);
-    } else {
-      if (mon) charge_x_kernel<false, true><<<grid, block, sm, st>>>(in, g, a);
-      else charge_x_kernel<false, false><<<grid, block, sm, st>>>(in, g, a);
-    }
-    return cudaGetLastError();
+    const int by = std::max(1, kRunThreads / g.H), nl = charge_row_nl(g);
+    const dim3 block(g.H, by), grid((unsigned)(((long long)g.N * g.N + by - 1) / by), 6 / nl);
+    return launch_pdl(charge_row_kernel, grid, block, 2 * (size_t)by * g.H * sizeof(double), st, g, a, nl);
   }
-  *swapped = true;
-  const int sl = charge_seglen(N);
-  dim3 grid((g.H + 127) / 128, N, (N + sl - 1) / sl);
-#define LGV_LINE(D, I, M) charge_line_kernel<D, I, M><<<grid, 128, 0, st>>>(in, out, g, a, sl)
-  if (dir == 1) {
-    if (inj) { if (mon) LGV_LINE(1, true, true); else LGV_LINE(1, true, false); }
-    else { if (mon) LGV_LINE(1, false, true); else LGV_LINE(1, false, false); }
-  } else {
-    if (inj) { if (mon) LGV_LINE(2, true, true); else LGV_LINE(2, true, false); }
-    else { if (mon) LGV_LINE(2, false, true); else LGV_LINE(2, false, false); }
-  }
-#undef LGV_LINE
-  return cudaGetLastError();
+  const bool i32 = 16 * g.V2 <= 0xffffffffLL;  // byte offsets within a plane
+  const int seg = charge_seg(g.N);
+  const dim3 grid(nblocks((long long)g.N * g.N, kRunThreads), (g.N + seg - 1) / seg, 6);
+#define LGV_RUN(D)                                                                                                  \
+  launch_pdl(i32 ? charge_run_kernel<D, unsigned> : charge_run_kernel<D, long long>, grid, dim3(kRunThreads), 0, st, g, \
+             a, seg)
+  return dir == 1 ? LGV_RUN(1) : LGV_RUN(2);
+#undef LGV_RUN
 }
 
 cudaError_t launch_em(Fields in, Fields out, int N, const EmArgs &a, cudaStream_t st) {
