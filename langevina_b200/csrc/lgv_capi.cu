@@ -156,10 +156,11 @@ struct lgv_handle {
     int S = 0, b = 0, K = 1;
     uint64_t ctr0 = 0;
     std::vector<double> tn, avg;
+    // partial: the slots of block rows and launch_sum_rows' scratch; gs: the
+    // parameter sums of every adjoint launch
     double *ckpt = nullptr, *seg = nullptr, *lam = nullptr, *work = nullptr, *avg_dev = nullptr, *partial = nullptr,
-           *g4 = nullptr;
-    unsigned *done = nullptr;  // grid_sum4 counter, zero between launches
-    size_t ckpt_len = 0, seg_len = 0, avg_len = 0, lam_len = 0, work_len = 0;
+           *gs = nullptr, *g4 = nullptr;
+    size_t ckpt_len = 0, seg_len = 0, avg_len = 0, lam_len = 0, work_len = 0, gs_len = 0;
   } adj;
 };
 
@@ -588,12 +589,12 @@ int create_handle(const lgv_params *params, const lgv::Geo &g, bool slab, int k0
   }
   if (rc == LGV_OK) {
     if (cudaMalloc((void **)&h->waits_dev, sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMemset(h->waits_dev, 0, sizeof(unsigned long long)) != cudaSuccess)
+        cudaMemsetAsync(h->waits_dev, 0, sizeof(unsigned long long), h->stream) != cudaSuccess)
       rc = fail(LGV_ERR_NOMEM, "wait counter alloc failed");
   }
   if (rc == LGV_OK) {
     const size_t n = lgv::kMeasCounters * sizeof(unsigned);
-    if (cudaMalloc((void **)&h->meas_done, n) != cudaSuccess || cudaMemset(h->meas_done, 0, n) != cudaSuccess)
+    if (cudaMalloc((void **)&h->meas_done, n) != cudaSuccess || cudaMemsetAsync(h->meas_done, 0, n, h->stream) != cudaSuccess)
       rc = fail(LGV_ERR_NOMEM, "measurement counters alloc failed");
   }
   if (rc == LGV_OK && h->hb_ordered) {
@@ -701,9 +702,8 @@ int lgv_destroy(lgv_handle *h) {
     if (b) cudaFree(b);
   if (h->mon_dev) cudaFree(h->mon_dev);
   if (h->flags_dev) cudaFree(h->flags_dev);
-  for (double *b : {h->adj.ckpt, h->adj.seg, h->adj.lam, h->adj.work, h->adj.avg_dev, h->adj.partial, h->adj.g4})
+  for (double *b : {h->adj.ckpt, h->adj.seg, h->adj.lam, h->adj.work, h->adj.avg_dev, h->adj.partial, h->adj.gs, h->adj.g4})
     if (b) cudaFree(b);
-  if (h->adj.done) cudaFree(h->adj.done);
   lgv::hb_plan_free(h->hb_plan);
   if (h->waits_dev) cudaFree(h->waits_dev);
   if (h->meas_done) cudaFree(h->meas_done);
@@ -1017,18 +1017,34 @@ Fields planes(double *base, size_t V, size_t first, int n) {
   return f;
 }
 
-// the reduction buffers of the differentiable run: CTA partials, the
-// grid_sum4 counter (zeroed once, re-armed by the kernels) and g4
-int adj_counters(lgv_handle *h) {
-  auto &A = h->adj;
-  if (!A.partial) LGV_TRY(ensure(&A.partial, lgv::em_reduce_blocks(h->N) * 4));
-  if (!A.g4) LGV_TRY(ensure(&A.g4, 4));
-  if (!A.done) {
-    LGV_CK(cudaMalloc((void **)&A.done, sizeof(unsigned)));
-    LGV_CK(cudaMemsetAsync(A.done, 0, sizeof(unsigned), h->stream));
+// Sums over sites, one row of 4 per launch: the launches fill the slots of
+// adj.partial in turn, and flush() adds the filled slots up into rows
+// (launch_sum_rows).
+struct SiteSums {
+  lgv_handle *h;
+  double scale, *rows;
+  int nb, slots, used = 0;
+  SiteSums(lgv_handle *hh, double sc, double *r)
+      : h(hh), scale(sc), rows(r), nb(lgv::sum_blocks(hh->N)), slots(lgv::sum_slots(nb)) {}
+  static size_t doubles(int N) {
+    const int nb = lgv::sum_blocks(N);
+    return (size_t)lgv::sum_slots(nb) * 4 * ((size_t)nb + lgv::kSumSegs);
   }
-  return LGV_OK;
-}
+  int flush() {
+    if (!used) return LGV_OK;
+    double *src = h->adj.partial;
+    LGV_CK(lgv::launch_sum_rows(src, used, nb, scale, rows, src + (size_t)slots * nb * 4, h->stream));
+    rows += (size_t)used * 4;
+    used = 0;
+    return LGV_OK;
+  }
+  // the slot of the next launch
+  int next(double **slot) {
+    if (used == slots) LGV_TRY(flush());
+    *slot = h->adj.partial + (size_t)used++ * nb * 4;
+    return LGV_OK;
+  }
+};
 
 // arguments of Euler-Maruyama step number ctr at time t (counter noise), as sub_em builds them
 lgv::EmArgs em_args(const lgv_params &p, uint64_t key, uint64_t ctr, double dt, double t) {
@@ -1081,7 +1097,7 @@ int lgv_diff_forward(lgv_handle *h, int evolver, double dt, double t, int nsteps
   const size_t nck = (size_t)(S - 1) / K + 1;
   LGV_TRY(adj_realloc(&A.ckpt, &A.ckpt_len, nck * A.ncomp * V));
   LGV_TRY(adj_realloc(&A.avg_dev, &A.avg_len, (size_t)(S + 1) * 4));
-  LGV_TRY(adj_counters(h));
+  if (!A.partial) LGV_TRY(ensure(&A.partial, SiteSums::doubles(h->N)));
   A.dt = dt;
   A.S = S;
   A.b = avg_begin;
@@ -1093,13 +1109,16 @@ int lgv_diff_forward(lgv_handle *h, int evolver, double dt, double t, int nsteps
   A.tn[0] = t;
   for (int n = 0; n < S; ++n) A.tn[n + 1] = A.tn[n] + dt;
   const lgv::IdealArgs ia = ideal_args(A.p, h->N, dt, h);
-  LGV_CK(lgv::launch_phi_avg(h->cur, h->N, A.partial, A.done, A.avg_dev, h->stream));
+  SiteSums sums(h, 1.0 / (double)V, A.avg_dev);
+  double *slot = nullptr;
+  LGV_TRY(sums.next(&slot));
+  LGV_CK(lgv::launch_phi_sum(h->cur, h->N, slot, h->stream));
   for (int n = 0; n < S; ++n) {
     if (n % K == 0)
       for (int l = 0; l < A.ncomp; ++l)
         LGV_CK(cudaMemcpyAsync(A.ckpt + ((size_t)(n / K) * A.ncomp + l) * V, h->cur.c[l], V * sizeof(double),
                                cudaMemcpyDeviceToDevice, h->stream));
-    double *avg_n = A.avg_dev + (size_t)(n + 1) * 4;
+    LGV_TRY(sums.next(&slot));
     if (has_ideal(evolver)) {
       KTimer tm(h, LGV_KCLASS_IDEAL);
       LGV_CK(lgv::launch_ideal(h->cur, h->alt, h->N, ia, h->stream));
@@ -1108,12 +1127,13 @@ int lgv_diff_forward(lgv_handle *h, int evolver, double dt, double t, int nsteps
     if (has_em(evolver)) {
       KTimer tm(h, LGV_KCLASS_EM);
       const lgv::EmArgs e = em_args(A.p, A.key, A.ctr0 + (uint64_t)n, dt, A.tn[n]);
-      LGV_CK(lgv::launch_em_avg(h->cur, h->alt, h->N, e, A.partial, A.done, avg_n, h->stream));
+      LGV_CK(lgv::launch_em_sum(h->cur, h->alt, h->N, e, slot, h->stream));
       for (int l = 0; l < 4; ++l) std::swap(h->cur.c[l], h->alt.c[l]);
     } else {
-      LGV_CK(lgv::launch_phi_avg(h->cur, h->N, A.partial, A.done, avg_n, h->stream));
+      LGV_CK(lgv::launch_phi_sum(h->cur, h->N, slot, h->stream));
     }
   }
+  LGV_TRY(sums.flush());
   if (has_em(evolver)) h->ctr += (uint64_t)S;
   A.avg.assign((size_t)(S + 1) * 4, 0.0);
   LGV_CK(cudaMemcpyAsync(A.avg.data(), A.avg_dev, A.avg.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -1153,8 +1173,11 @@ int lgv_diff_backward(lgv_handle *h, const double *w, double *grad) {
   LGV_TRY(adj_realloc(&A.seg, &A.seg_len, (size_t)K * nc * V));
   LGV_TRY(adj_realloc(&A.lam, &A.lam_len, 2 * 10 * V));
   if (has_ideal(ev)) LGV_TRY(adj_realloc(&A.work, &A.work_len, 28 * V));
-  LGV_TRY(adj_counters(h));
-  LGV_CK(cudaMemsetAsync(A.g4, 0, 4 * sizeof(double), h->stream));
+  const int per_step = (has_em(ev) ? 1 : 0) + (has_ideal(ev) ? 1 : 0), nrows = S * per_step;
+  LGV_TRY(adj_realloc(&A.gs, &A.gs_len, ((size_t)nrows + lgv::kSumSegs) * 4));
+  LGV_TRY(ensure(&A.g4, 4));
+  SiteSums sums(h, 1.0, A.gs);
+  double *psum = nullptr;
   const double Vd = (double)V;
   // dJ/dphi_a(x, n) of J = w0 obs0 + w1 obs1: w0 / (M V) for a = 0, w1 2 pibar_a(n) / M for a >= 1
   auto gl = [&](int n, double out[4]) {
@@ -1210,6 +1233,7 @@ int lgv_diff_backward(lgv_handle *h, const double *w, double *grad) {
     const Fields u = slot(n - s * K);
     double gln[4];
     gl(n, gln);
+    LGV_TRY(sums.next(&psum));
     if (has_em(ev)) {
       lgv::EmAdjArgs a{};
       a.c6 = 6.0 + (A.p.mass0 + A.p.dmassdt * A.tn[n]);
@@ -1221,23 +1245,24 @@ int lgv_diff_backward(lgv_handle *h, const double *w, double *grad) {
       a.sk = lgv::sub_key(A.key, A.ctr0 + (uint64_t)n);
       if (ev == LGV_MODELA_EM) {
         for (int q = 0; q < 4; ++q) a.gl[q] = gln[q];
-        LGV_CK(lgv::launch_em_adjoint(u, lam(cur), lam(cur ^ 1), N, a, A.partial, A.done, A.g4, h->stream));
+        LGV_CK(lgv::launch_em_adjoint(u, lam(cur), lam(cur ^ 1), N, a, psum, h->stream));
       } else {
         LGV_CK(lgv::launch_ideal(u, tmp, N, ia, h->stream));
-        LGV_CK(lgv::launch_em_adjoint(tmp, lam(cur), lamx, N, a, A.partial, A.done, A.g4, h->stream));
+        LGV_CK(lgv::launch_em_adjoint(tmp, lam(cur), lamx, N, a, psum, h->stream));
         Fields lmid = lam(cur);  // charges' adjoint passes the EM step unchanged
         for (int l = 0; l < 4; ++l) lmid.c[l] = lamx.c[l];
         for (int q = 0; q < 4; ++q) iadj.gl[q] = gln[q];
-        LGV_CK(lgv::launch_ideal_adjoint(u, lmid, lam(cur ^ 1), P1, PB, QB, N, iadj, A.partial, A.done, A.g4,
-                                         h->stream));
+        LGV_TRY(sums.next(&psum));
+        LGV_CK(lgv::launch_ideal_adjoint(u, lmid, lam(cur ^ 1), P1, PB, QB, N, iadj, psum, h->stream));
       }
     } else {
       for (int q = 0; q < 4; ++q) iadj.gl[q] = gln[q];
-      LGV_CK(lgv::launch_ideal_adjoint(u, lam(cur), lam(cur ^ 1), P1, PB, QB, N, iadj, A.partial, A.done, A.g4,
-                                       h->stream));
+      LGV_CK(lgv::launch_ideal_adjoint(u, lam(cur), lam(cur ^ 1), P1, PB, QB, N, iadj, psum, h->stream));
     }
     cur ^= 1;
   }
+  LGV_TRY(sums.flush());
+  LGV_CK(lgv::launch_sum_rows(A.gs, 1, nrows, 1.0, A.g4, A.gs + (size_t)nrows * 4, h->stream));
   LGV_CK(cudaMemcpyAsync(grad, A.g4, 4 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   LGV_CK(cudaStreamSynchronize(h->stream));
   return LGV_OK;

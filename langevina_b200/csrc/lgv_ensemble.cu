@@ -109,8 +109,7 @@ struct lgv_ensemble {
     std::vector<size_t> lens;
     lgv::DiffDesc *dd = nullptr;
     double *wg = nullptr;  // [R][2] weights then [R][4] gradients
-    double *partial = nullptr;
-    unsigned *done = nullptr;  // one counter per replica
+    double *partial = nullptr;  // slots of block rows (lgv::sum_slots)
     size_t partial_len = 0;
   } diff;
 };
@@ -406,7 +405,7 @@ int enqueue_step(lgv_ensemble *e, int ev, int inner, int outer, double dt) {
     case LGV_CHARGE_HB: ETRY(charge(dt)); break;
     case LGV_MODELA_EM:
       ECK(lgv::launch_batch_em(e->dd, e->dyn, e->plane_map.rep, e->plane_map.first, nb_p, e->phase_phi, dt, off,
-                               e->stream));
+                               e->idx32, e->stream));
       e->phase_phi ^= 1;
       off += 1;
       break;
@@ -533,7 +532,6 @@ int lgv_ensemble_destroy(lgv_ensemble *e) {
   if (e->diff.dd) cudaFree(e->diff.dd);
   if (e->diff.wg) cudaFree(e->diff.wg);
   if (e->diff.partial) cudaFree(e->diff.partial);
-  if (e->diff.done) cudaFree(e->diff.done);
   if (e->waits) cudaFree(e->waits);
   if (e->bar) cudaFree(e->bar);
   if (e->side) {
@@ -697,10 +695,9 @@ int lgv_ensemble_diff_forward(lgv_ensemble *e, double dt, double t, int nsteps, 
     D.hd.assign(R, lgv::DiffDesc{});
     ECK(cudaMalloc((void **)&D.dd, R * sizeof(lgv::DiffDesc)));
     ECK(cudaMalloc((void **)&D.wg, (size_t)R * 6 * sizeof(double)));
-    ECK(cudaMalloc((void **)&D.done, R * sizeof(unsigned)));
-    ECK(cudaMemsetAsync(D.done, 0, R * sizeof(unsigned), e->stream));
   }
-  const size_t need_partial = (size_t)e->plane_map.nblocks * 4 + 16;
+  const int slots = lgv::sum_slots(e->plane_map.nblocks);
+  const size_t need_partial = (size_t)slots * e->plane_map.nblocks * 4;
   if (D.partial_len < need_partial) {
     if (D.partial) cudaFree(D.partial);
     D.partial = nullptr;
@@ -710,8 +707,8 @@ int lgv_ensemble_diff_forward(lgv_ensemble *e, double dt, double t, int nsteps, 
   }
   for (int r = 0; r < R; ++r) {
     const size_t V = (size_t)e->p[r].N * e->p[r].N * e->p[r].N;
-    // checkpoints, segment states, two adjoint states, averages
-    const size_t need = (nck + (size_t)K + 2) * 4 * V + (size_t)(S + 1) * 4;
+    // checkpoints, segment states, two adjoint states, averages, parameter sums
+    const size_t need = (nck + (size_t)K + 2) * 4 * V + (size_t)(2 * S + 1) * 4;
     if (D.lens[r] < need) {
       if (D.bufs[r]) cudaFree(D.bufs[r]);
       D.bufs[r] = nullptr;
@@ -725,6 +722,7 @@ int lgv_ensemble_diff_forward(lgv_ensemble *e, double dt, double t, int nsteps, 
     d.seg = d.ckpt + nck * 4 * V;
     d.lam = d.seg + (size_t)K * 4 * V;
     d.avg = d.lam + 8 * V;
+    d.gs = d.avg + (size_t)(S + 1) * 4;
     d.w = D.wg + 2 * r;
     d.grad = D.wg + 2 * R + 4 * r;
   }
@@ -738,16 +736,28 @@ int lgv_ensemble_diff_forward(lgv_ensemble *e, double dt, double t, int nsteps, 
   D.tn[0] = t;
   for (int n = 0; n < S; ++n) D.tn[n + 1] = D.tn[n] + dt;
   const BlockMap &pm = e->plane_map;
-  for (int r = 0; r < R; ++r)
-    ECK(lgv::launch_phi_avg(cur_fields(e, r), e->p[r].N, D.partial, D.done, D.hd[r].avg, e->stream));
+  // the slots of D.partial, filled from row `row` on, are added up when all are
+  int used = 0, row = 0;
+  auto slot = [&]() { return D.partial + (size_t)used++ * pm.nblocks * 4; };
+  auto flush = [&](bool last) -> int {
+    if (used == slots || (last && used)) {
+      ECK(lgv::launch_batch_sum(D.dd, pm.first, pm.count, R, 0, D.partial, pm.nblocks, row, used, e->stream));
+      row += used;
+      used = 0;
+    }
+    return LGV_OK;
+  };
+  ECK(lgv::launch_batch_phi_sum(e->dd, pm.rep, pm.first, pm.nblocks, e->phase_phi, slot(), e->stream));
   for (int n = 0; n < S; ++n) {
+    ETRY(flush(false));
     if (n % K == 0)
       ECK(lgv::launch_batch_diff_copy(e->dd, D.dd, pm.rep, pm.first, pm.nblocks, 0, e->phase_phi, n / K, avg_begin, S,
                                       e->stream));
-    ECK(lgv::launch_batch_em_fwd(e->dd, D.dd, pm.rep, pm.first, pm.count, pm.nblocks, e->phase_phi, D.ctr0 + n,
-                                 D.tn[n], dt, n, D.partial, D.done, e->stream));
+    ECK(lgv::launch_batch_em_fwd(e->dd, pm.rep, pm.first, pm.nblocks, e->phase_phi, D.ctr0 + n, D.tn[n], dt, slot(),
+                                 e->idx32, e->stream));
     e->phase_phi ^= 1;
   }
+  ETRY(flush(true));
   e->ctr += (unsigned long long)S;
   std::vector<double> avg((size_t)(S + 1) * 4);
   for (int r = 0; r < R; ++r) {
@@ -774,9 +784,9 @@ int lgv_ensemble_diff_backward(lgv_ensemble *e, const double *w, double *grad) {
   const int R = e->R, S = D.S, K = D.K;
   const BlockMap &pm = e->plane_map;
   ECK(cudaMemcpyAsync(D.wg, w, (size_t)R * 2 * sizeof(double), cudaMemcpyHostToDevice, e->stream));
-  ECK(cudaMemsetAsync(D.wg + 2 * R, 0, (size_t)R * 4 * sizeof(double), e->stream));
   ECK(lgv::launch_batch_diff_copy(e->dd, D.dd, pm.rep, pm.first, pm.nblocks, 2, 0, 0, D.b, S, e->stream));
-  int cur = 0, loaded = -1;
+  const int slots = lgv::sum_slots(pm.nblocks);
+  int cur = 0, loaded = -1, used = 0, row = 0;
   for (int n = S - 1; n >= 0; --n) {
     const int s = n / K;
     if (s != loaded) {
@@ -784,13 +794,19 @@ int lgv_ensemble_diff_backward(lgv_ensemble *e, const double *w, double *grad) {
       const int last = std::min(s * K + K - 1, S - 1);
       for (int m = s * K; m < last; ++m)
         ECK(lgv::launch_batch_em_seg(e->dd, D.dd, pm.rep, pm.first, pm.nblocks, m - s * K, D.ctr0 + m, D.tn[m], D.dt,
-                                     e->stream));
+                                     e->idx32, e->stream));
       loaded = s;
     }
-    ECK(lgv::launch_batch_em_adj(e->dd, D.dd, pm.rep, pm.first, pm.count, pm.nblocks, n - s * K, cur, n, D.b, S,
-                                 D.ctr0 + n, D.tn[n], D.dt, D.partial, D.done, e->stream));
+    ECK(lgv::launch_batch_em_adj(e->dd, D.dd, pm.rep, pm.first, pm.nblocks, n - s * K, cur, n, D.b, S, D.ctr0 + n,
+                                 D.tn[n], D.dt, D.partial + (size_t)used * pm.nblocks * 4, e->idx32, e->stream));
+    if (++used == slots || n == 0) {
+      ECK(lgv::launch_batch_sum(D.dd, pm.first, pm.count, R, 1, D.partial, pm.nblocks, row, used, e->stream));
+      row += used;
+      used = 0;
+    }
     cur ^= 1;
   }
+  ECK(lgv::launch_batch_sum(D.dd, pm.first, pm.count, R, 2, nullptr, 0, S, 1, e->stream));
   ECK(cudaMemcpyAsync(grad, D.wg + 2 * R, (size_t)R * 4 * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
   ECK(cudaStreamSynchronize(e->stream));
   return ens_check_waits(e);

@@ -96,24 +96,33 @@ struct EnsDyn {
 // Differentiable Euler-Maruyama runs of an ensemble: per-replica buffers of
 // V-double planes.  ckpt: checkpoint slots of 4 planes; seg: the K states of
 // the segment being differentiated; lam: two 4-plane adjoint states; avg:
-// (S+1) x 4 volume averages; w: the replica's observable weights.
+// (S+1) x 4 volume averages; gs: S x 4 parameter sums of the steps; w: the
+// replica's observable weights.
 struct DiffDesc {
-  double *ckpt, *seg, *lam, *avg, *w, *grad;
+  double *ckpt, *seg, *lam, *avg, *gs, *w, *grad;
   long long V;
 };
 
-// forward step n: phi of the lattice buffer `phase` -> phase ^ 1, averages into avg[n+1]
-cudaError_t launch_batch_em_fwd(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first,
-                                const int *count, int nblocks, int phase, unsigned long long ctr, double t, double dt,
-                                int n, double *partial, unsigned *done, cudaStream_t st);
+// forward step: phi of the lattice buffer `phase` -> phase ^ 1; the sums of the
+// new phi leave as a row of 4 per block in partial
+cudaError_t launch_batch_em_fwd(const RepDesc *d, const int *rep, const int *first, int nblocks, int phase,
+                                unsigned long long ctr, double t, double dt, double *partial, bool i32,
+                                cudaStream_t st);
 // recompute: seg slot m -> m + 1
 cudaError_t launch_batch_em_seg(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first, int nblocks,
-                                int m, unsigned long long ctr, double t, double dt, cudaStream_t st);
-// adjoint of step n at seg slot m: lam[cur] -> lam[cur ^ 1], gradients into grad
-cudaError_t launch_batch_em_adj(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first,
-                                const int *count, int nblocks, int m, int cur, int n, int b, int S,
-                                unsigned long long ctr, double t, double dt, double *partial, unsigned *done,
-                                cudaStream_t st);
+                                int m, unsigned long long ctr, double t, double dt, bool i32, cudaStream_t st);
+// adjoint of step n at seg slot m: lam[cur] -> lam[cur ^ 1], parameter sums as rows in partial
+cudaError_t launch_batch_em_adj(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first, int nblocks,
+                                int m, int cur, int n, int b, int S, unsigned long long ctr, double t, double dt,
+                                double *partial, bool i32, cudaStream_t st);
+// rows of the sums of phi of buffer `phase`
+cudaError_t launch_batch_phi_sum(const RepDesc *d, const int *rep, const int *first, int nblocks, int phase,
+                                 double *partial, cudaStream_t st);
+// the rows of nslot slots [slot][nblocks][4] of src, per replica, into rows
+// row0 .. row0 + nslot - 1 of its averages (what 0) or of its gs (1); what 2:
+// its row0 rows of gs into grad
+cudaError_t launch_batch_sum(const DiffDesc *dd, const int *first, const int *count, int nrep, int what,
+                             const double *src, int nblocks, int row0, int nslot, cudaStream_t st);
 // phi planes: lattice buffer `phase` -> ckpt slot s (dir 0); ckpt slot s -> seg slot 0 (dir 1);
 // lam[0] = dJ/dphi(S) from avg and w (dir 2)
 cudaError_t launch_batch_diff_copy(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first,
@@ -135,7 +144,7 @@ cudaError_t launch_batch_hb(const RepDesc *d, const EnsDyn *dyn, const int *rep,
 cudaError_t launch_batch_charge(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
                                 int phase_q, int pass, double dt, int ctr_off_order, bool i32, cudaStream_t st);
 cudaError_t launch_batch_em(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
-                            int phase_phi, double dt, int ctr_off, cudaStream_t st);
+                            int phase_phi, double dt, int ctr_off, bool i32, cudaStream_t st);
 cudaError_t launch_ens_set(EnsDyn *dyn, unsigned long long ctr, double t, cudaStream_t st);
 cudaError_t launch_ens_advance(EnsDyn *dyn, unsigned long long dctr, double dt, cudaStream_t st);
 // volume averages (the 11 OAverage observables) of every replica: partial[nblocks][11], out[nrep][11]
@@ -192,8 +201,6 @@ struct EmAdjArgs {
   double gl[4];   // uniform loss gradient dL/dphi_a added to the adjoint of this state
   uint64_t sk;    // the step's noise key (regenerates xi)
 };
-// lam_out = J^T lam_in + gl at state phi; per-block parameter-gradient partial
-// sums (dm2, dlambda, dH, dgamma) into partial[nblocks][4]
 struct IdealAdjArgs {
   double k;   // (dt / 2) / chi
   double dt;
@@ -202,24 +209,29 @@ struct IdealAdjArgs {
   double gl[4];  // added to the phi adjoint at every site
 };
 
-// Adjoint of one ideal step at state u (10 planes): lam_in (10 planes) ->
-// lam_out (10 planes); adds dL/dH into g4[2].  P1, PB: 4 planes, QB: 6 planes
-// of scratch; partial / done as for launch_em_avg.
-cudaError_t launch_ideal_adjoint(Fields u, Fields lam_in, Fields lam_out, Fields P1, Fields PB, Fields QB, int N,
-                                 const IdealAdjArgs &a, double *partial, unsigned *done, double *g4,
-                                 cudaStream_t st);
-
-// Euler-Maruyama step that also writes the volume averages of the new phi
-// to avg_out[0..3]; partial holds em_reduce_blocks(N) * 4 doubles and *done
-// is a zeroed counter (left zeroed).
-cudaError_t launch_em_avg(Fields in, Fields out, int N, const EmArgs &a, double *partial, unsigned *done,
-                          double *avg_out, cudaStream_t st);
-size_t em_reduce_blocks(int N);
-// adjoint of one Euler-Maruyama step; adds dL/d(m^2, lambda, H, Gamma) of the step into g4[0..3]
+// Sums over sites.  The kernels below leave them as rows of 4 doubles, one per
+// block (sum_blocks(N) of them) in a slot of `partial`; a buffer of
+// sum_slots(blocks) slots is filled step after step and then added up, slot by
+// slot, by launch_sum_rows: rows[slot][4] = scale times the sum of the nb rows of
+// src[slot], in a fixed order.  tmp: nslot * kSumSegs * 4 doubles.
+constexpr int kSumSegs = 16;
+int sum_blocks(int N);
+int sum_slots(int nblocks);
+cudaError_t launch_sum_rows(const double *src, int nslot, int nb, double scale, double *rows, double *tmp,
+                            cudaStream_t st);
+// Euler-Maruyama step that also sums the new phi
+cudaError_t launch_em_sum(Fields in, Fields out, int N, const EmArgs &a, double *partial, cudaStream_t st);
+// sums of phi_0..3
+cudaError_t launch_phi_sum(Fields f, int N, double *partial, cudaStream_t st);
+// adjoint of one Euler-Maruyama step: lam_out = J^T lam_in + gl at state phi,
+// and the step's share of dL/d(m^2, lambda, H, Gamma)
 cudaError_t launch_em_adjoint(Fields phi, Fields lam_in, Fields lam_out, int N, const EmAdjArgs &a, double *partial,
-                              unsigned *done, double *g4, cudaStream_t st);
-// volume averages of phi_0..3 -> out[4]
-cudaError_t launch_phi_avg(Fields f, int N, double *partial, unsigned *done, double *out, cudaStream_t st);
+                              cudaStream_t st);
+// Adjoint of one ideal step at state u (10 planes): lam_in (10 planes) ->
+// lam_out (10 planes), and the step's share of dL/dH (sum 2).  P1, PB: 4
+// planes, QB: 6 planes of scratch.
+cudaError_t launch_ideal_adjoint(Fields u, Fields lam_in, Fields lam_out, Fields P1, Fields PB, Fields QB, int N,
+                                 const IdealAdjArgs &a, double *partial, cudaStream_t st);
 // phi planes of f set to the constants v[4]
 cudaError_t launch_fill_phi(Fields f, int N, const double v[4], cudaStream_t st);
 

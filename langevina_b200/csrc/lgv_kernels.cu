@@ -48,17 +48,14 @@ __device__ __forceinline__ void warp_sum(unsigned long long &v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
 }
 
-// Sums v[0..3] over the CTA into partial[blockIdx.x][0..3]; the last CTA of
-// the grid to finish then adds the CTA partials in block order (fixed, so the
-// result does not depend on which CTA ends last), scaled, into out[0..3]
-// (accumulating when add) and re-arms the counter.  `done` is zero on entry.
+// Sums v[0..3] over the CTA into out[0..3], a row of its own for every CTA:
+// sum_rows_kernel adds the rows in a fixed order.  (Adding them in the launch
+// itself, by the CTA that ends last, left the chip idle for 4 us of a 10 us
+// step at 48^3.)
 template <int NT>
-__device__ __forceinline__ void grid_sum4(double (&v)[4], double *partial, unsigned *done, double *out, double scale,
-                                          bool add) {
-  static_assert(NT % 32 == 0 && NT >= 128, "grid_sum4: NT");
+__device__ __forceinline__ void block_sum4(double (&v)[4], double *out) {
   constexpr int NW = NT / 32;
   __shared__ double sm[4][NW];
-  __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -66,37 +63,36 @@ __device__ __forceinline__ void grid_sum4(double (&v)[4], double *partial, unsig
     if (lane == 0) sm[q][warp] = v[q];
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      double t = 0;
-#pragma unroll
-      for (int w = 0; w < NW; ++w) t += sm[q][w];
-      partial[(size_t)blockIdx.x * 4 + q] = t;
-    }
-    __threadfence();
-    last = atomicAdd(done, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (warp < 4) {
+  if (threadIdx.x < 4) {
     double t = 0;
-    for (unsigned b = lane; b < gridDim.x; b += 32) t += __ldcg(partial + (size_t)b * 4 + warp);
-    warp_sum(t);
-    if (lane == 0) out[warp] = add ? out[warp] + t * scale : t * scale;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) t += sm[threadIdx.x][w];
+    out[threadIdx.x] = t;
   }
-  if (threadIdx.x == 0) *done = 0u;
 }
 
-// Flat site-pair index -> (m, j, k) of the red-black half rows: idx = (k N + j) H + m.
-// 32-bit unsigned divisions (64-bit ones are emulated); idx < V/2 <= 2^32 for N <= 2048.
-__device__ __forceinline__ void pair_coords(long long idx, const Geo &g, int &m, int &j, int &k) {
-  const unsigned u = (unsigned)idx, H = (unsigned)g.H, N = (unsigned)g.N;
-  const unsigned row = u / H;
-  m = (int)(u - row * H);
-  k = (int)(row / N);
-  j = (int)(row - (unsigned)k * N);
+// Block (slot, seg): rows n of src[slot][nb][4] with n in segment seg of
+// gridDim.y, summed in a fixed order, scaled, into out[slot][gridDim.y][4].
+constexpr int kSumThreads = 256;
+
+__device__ __forceinline__ void sum_rows(const double *src, int n0, int n1, double scale, double *out) {
+  __shared__ double sm[kSumThreads];
+  double t = 0;
+#pragma unroll 8
+  for (int n = n0 + (threadIdx.x >> 2); n < n1; n += kSumThreads / 4) t += src[(size_t)n * 4 + (threadIdx.x & 3)];
+  sm[threadIdx.x] = t;
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double u = 0;
+#pragma unroll 16
+    for (int w = 0; w < kSumThreads / 4; ++w) u += sm[w * 4 + threadIdx.x];
+    out[threadIdx.x] = u * scale;
+  }
+}
+
+__global__ void __launch_bounds__(kSumThreads) sum_rows_kernel(const double *src, int nb, double scale, double *out) {
+  const int slot = blockIdx.x, seg = blockIdx.y, ns = gridDim.y, per = (nb + ns - 1) / ns;
+  sum_rows(src + (size_t)slot * nb * 4, seg * per, min(nb, (seg + 1) * per), scale, out + ((size_t)slot * ns + seg) * 4);
 }
 
 // Per-thread monitor tally, reduced per block and added once per block.
@@ -290,26 +286,37 @@ struct HbDecision {
   uint8_t flag;
 };
 
-// GAUSS (counter noise): the proposals are the four normals of two
-// Box-Muller pairs from the site's first four draws (as Euler-Maruyama's
-// noise) instead of the reference's U(-sqrt3, sqrt3), Stepper.cxx:343; both
-// are symmetric with variance one, so detailed balance and the proposal scale
-// are the same.  The accept uniform is the next draw either way.
-template <bool INJECTED, bool GAUSS = false>
-__device__ __forceinline__ void hb_decide(const double po[4], const double heff[4], const HbArgs &a, long long nat,
-                                          long long V, HbDecision &r) {
+// The counter noise of one heat-bath site: four proposals of variance one and
+// the stream, whose next draw is the accept uniform.  GAUSS: the proposals are
+// the four normals of two Box-Muller pairs from the site's first four draws (as
+// Euler-Maruyama's noise) instead of the reference's U(-sqrt3, sqrt3),
+// Stepper.cxx:343; both are symmetric with variance one, so detailed balance
+// and the proposal scale are the same.
+struct HbNoise {
+  double v[4];
   Xoro rng;
-  if (!INJECTED) rng = stream_at(a.sk, (uint64_t)nat);
-  double z[4] = {0., 0., 0., 0.};
-  if (!INJECTED && GAUSS) {
-    const uint64_t r1 = rng.next(), r2 = rng.next(), r3 = rng.next(), r4 = rng.next();
-    box_muller(r1, r2, z[0], z[1]);
-    box_muller(r3, r4, z[2], z[3]);
+};
+
+template <bool GAUSS>
+__device__ __forceinline__ void hb_noise(uint64_t sk, long long nat, HbNoise &r) {
+  r.rng = stream_at(sk, (uint64_t)nat);
+  if (GAUSS) {
+    const uint64_t r1 = r.rng.next(), r2 = r.rng.next(), r3 = r.rng.next(), r4 = r.rng.next();
+    box_muller(r1, r2, r.v[0], r.v[1]);
+    box_muller(r3, r4, r.v[2], r.v[3]);
+  } else {
+#pragma unroll
+    for (int l = 0; l < 4; ++l) r.v[l] = var1(r.rng.next());
   }
+}
+
+template <bool INJECTED>
+__device__ __forceinline__ void hb_decide(const double po[4], const double heff[4], const HbArgs &a, long long nat,
+                                          long long V, HbNoise &z, HbDecision &r) {
   double hphi_o = 0., hphi_n = 0., s_o = 0., s_n = 0.;
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
-    const double v = INJECTED ? a.prop[(long long)l * V + nat] : (GAUSS ? z[l] : var1(rng.next()));
+    const double v = INJECTED ? a.prop[(long long)l * V + nat] : z.v[l];
     r.pn[l] = po[l] + a.rdtg * v;
     s_o += po[l] * po[l];
     s_n += r.pn[l] * r.pn[l];
@@ -326,7 +333,7 @@ __device__ __forceinline__ void hb_decide(const double po[4], const double heff[
     if (INJECTED) {
       r.accept = a.acc[nat] < exp(-r.dS);
     } else {
-      const uint64_t w = rng.next();
+      const uint64_t w = z.rng.next();
       r.accept = metropolis((uint32_t)(w >> 32), r.dS, [&] { return u53(w) < exp(-r.dS); });
     }
     r.flag = r.accept ? 2 : 0;
@@ -368,7 +375,8 @@ __device__ __forceinline__ I nat_index_t(const Geo &g, int i, int j, int k) {
   return ((I)kk * g.N + j) * g.N + i;
 }
 
-template <bool INJECTED, bool MON, bool CG = false, typename I = long long, bool GAUSS = false>
+// EARLY: the noise is drawn before the wait for the previous kernel.
+template <bool INJECTED, bool MON, bool CG = false, typename I = long long, bool GAUSS = false, bool EARLY = false>
 __device__ __forceinline__ void hb_site(const Fields &f, const Geo &g, int parity, const HbArgs &a, int m, int j,
                                         int k, MonLocal &mon) {
   const int H = g.H, N = g.N;
@@ -384,6 +392,12 @@ __device__ __forceinline__ void hb_site(const Fields &f, const Geo &g, int parit
   const I okp = ob + ((I)wrap_inc(k, g.Nz) * N + j) * H + m;
   const I okm = ob + ((I)wrap_dec(k, g.Nz) * N + j) * H + m;
   const I own = (I)parity * (I)g.V2 + row + m;
+  const long long nat = (long long)nat_index_t<I>(g, 2 * m + s, j, k);
+  HbNoise z;
+  if (!INJECTED && EARLY) {
+    hb_noise<GAUSS>(a.sk, nat, z);
+    pdl_wait();
+  }
   double po[4], heff[4];
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
@@ -393,9 +407,9 @@ __device__ __forceinline__ void hb_site(const Fields &f, const Geo &g, int parit
               (ld_phi<CG>(P + okp) + ld_phi<CG>(P + okm));
     po[l] = ld_phi<CG>(P + own);
   }
-  const long long nat = (long long)nat_index_t<I>(g, 2 * m + s, j, k);
+  if (!INJECTED && !EARLY) hb_noise<GAUSS>(a.sk, nat, z);
   HbDecision d;
-  hb_decide<INJECTED, GAUSS>(po, heff, a, nat, global_sites(g), d);
+  hb_decide<INJECTED>(po, heff, a, nat, global_sites(g), z, d);
   if (d.accept) {
 #pragma unroll
     for (int l = 0; l < 4; ++l) f.c[l][own] = d.pn[l];
@@ -429,11 +443,17 @@ __host__ __forceinline__ dim3 pass_grid(const Geo &g, bool rows) {
   return rows ? dim3(g.H / 128, g.N, g.Nz) : dim3((unsigned)(((long long)g.N * g.H + 127) / 128), g.Nz);
 }
 
-template <bool INJECTED, bool MON, bool ROWS, typename I, bool GAUSS = false>
+// The noise is drawn before the wait for the previous kernel, at every size (a
+// sweep of two passes: 64^3 12.3 us launched plainly, 10.0 with the wait first,
+// 9.1 with the noise first; 256^3 342 with the wait first, 329).
+template <bool INJECTED, bool MON, bool ROWS, typename I, bool GAUSS>
 __global__ void __launch_bounds__(128) hb_pass_kernel(Fields f, Geo g, int parity, HbArgs a) {
+  pdl_launch();
+  if (INJECTED) pdl_wait();
   int m, j, k;
   MonLocal mon;
-  if (pass_site<ROWS>(g, m, j, k)) hb_site<INJECTED, MON, false, I, GAUSS>(f, g, parity, a, m, j, k, mon);
+  if (pass_site<ROWS>(g, m, j, k))
+    hb_site<INJECTED, MON, false, I, GAUSS, true>(f, g, parity, a, m, j, k, mon);
   if (MON) mon_flush(mon, a.mon);
 }
 
@@ -525,7 +545,9 @@ __global__ void __launch_bounds__(ZP_NT) hb_zpass_kernel(Fields f, Geo g, int pa
       }
       const long long nat = ((long long)k * N + j) * N + 2 * m + s;
       HbDecision d;
-      hb_decide<INJECTED>(po, heff, a, nat, 2 * g.V2, d);
+      HbNoise z;
+      if (!INJECTED) hb_noise<false>(a.sk, nat, z);
+      hb_decide<INJECTED>(po, heff, a, nat, 2 * g.V2, z, d);
       if (d.accept) {
 #pragma unroll
         for (int l = 0; l < 4; ++l) f.c[l][offp] = d.pn[l];
@@ -767,7 +789,9 @@ __global__ void __launch_bounds__(HB_TM *HB_TY, 2) hb_sweep_kernel(Fields in, Fi
       }
       const long long nat = ((long long)p * N + j) * N + 2 * m + s0;
       HbDecision d;
-      hb_decide<INJECTED>(po, heff, a, nat, V, d);
+      HbNoise z;
+      if (!INJECTED) hb_noise<false>(a.sk, nat, z);
+      hb_decide<INJECTED>(po, heff, a, nat, V, z, d);
 #pragma unroll
       for (int l = 0; l < 4; ++l) nec[l * HB_EP + e] = d.accept ? d.pn[l] : po[l];
       const bool own = in_chunk_e && qm >= 1 && qm <= HB_TM && qj >= 1 && qj <= HB_TY && mr < H && jr < N;
@@ -801,7 +825,9 @@ __global__ void __launch_bounds__(HB_TM *HB_TY, 2) hb_sweep_kernel(Fields in, Fi
       }
       const long long nat = ((long long)q * N + j) * N + 2 * m + s1;
       HbDecision d;
-      hb_decide<INJECTED>(po, heff, a, nat, V, d);
+      HbNoise z;
+      if (!INJECTED) hb_noise<false>(a.sk, nat, z);
+      hb_decide<INJECTED>(po, heff, a, nat, V, z, d);
       if (act) {
         const long long row = ((long long)q * N + j) * H + m;
 #pragma unroll
@@ -889,6 +915,8 @@ __device__ __forceinline__ void charge_link_site(const Fields &f, const Geo &g, 
 // integer / FP64 chains, and full occupancy hides them best
 template <bool INJECTED, bool MON, bool ROWS, typename I>
 __global__ void __launch_bounds__(128, 16) charge_pass_kernel(Fields f, Geo g, int dir, int eoA, ChargeArgs a) {
+  pdl_launch();
+  pdl_wait();
   int m, j, k;
   MonLocal mon;
   if (pass_site<ROWS>(g, m, j, k)) charge_link_site<INJECTED, MON, I>(f, g, dir, eoA, a, m, j, k, mon);
@@ -1068,129 +1096,134 @@ __global__ void __launch_bounds__(1024) charge_row_kernel(Geo g, ChargeDirArgs a
 }
 
 // ----------------------------------------------------------------------------
-// Euler-Maruyama Model A step (Jacobi: reads `in`, writes phi of `out`).
-// One thread per element m of both parity half-rows of row (j, k).  I: the
-// element offset type (int when idx32 holds, as the heat-bath pass).
-template <bool INJECTED, typename I = long long>
-__device__ __forceinline__ void em_pair(const Fields &in, const Fields &out, const Geo &g, const EmArgs &a, int m,
-                                        int j, int k, double (&acc)[4]) {
-  const int H = g.H, N = g.N;
-  const I row = ((I)k * N + j) * H;
-  const I rjp = ((I)k * N + wrap_inc(j, N)) * H + m;
-  const I rjm = ((I)k * N + wrap_dec(j, N)) * H + m;
-  const I rkp = ((I)wrap_inc(k, g.Nz) * N + j) * H + m;
-  const I rkm = ((I)wrap_dec(k, g.Nz) * N + j) * H + m;
+// Blocks of the kernels that visit all sites: 256 threads cover 128 consecutive
+// (j, m) elements of a plane, threads 0..127 in the even and 128..255 in the odd
+// half.  Grid (ceil(N H / 128), planes).
+constexpr int kSiteThreads = 256;
+// resident blocks per SM of the Euler-Maruyama step, its adjoint and the ideal step's adjoint (48, 80 and 86-128 registers)
+#ifdef EMB
+constexpr int kEmBlocks = EMB, kEmAdjBlocks = AJB, kIdealAdjBlocks = 2;
+#else
+constexpr int kEmBlocks = 5, kEmAdjBlocks = 3, kIdealAdjBlocks = 2;
+#endif
+
+__device__ __forceinline__ bool all_site(const Geo &g, int chunk, int &parity, int &m, int &j) {
+  parity = threadIdx.x >> 7;
+  const unsigned t = chunk * 128 + (threadIdx.x & 127), H = (unsigned)g.H;
+  const unsigned jj = t / H;
+  m = (int)(t - jj * H);
+  j = (int)jj;
+  return j < g.N;
+}
+
+inline dim3 site_grid(const Geo &g) { return dim3((unsigned)(((long long)g.N * g.H + 127) / 128), g.Nz); }
+
+// The six neighbours of a site as offsets in a component plane.
+template <typename I>
+struct Nbrs {
+  I own, xp, xm, jp, jm, kp, km;
+};
+template <typename I>
+__device__ __forceinline__ Nbrs<I> nbrs_of(const Geo &g, int parity, int m, int j, int k) {
+  const int H = g.H, N = g.N, s = (parity + j + k) & 1;
+  int xm = m - 1 + s, xp = m + s;
+  if (xm < 0) xm += H;
+  if (xp == H) xp = 0;
+  const I ob = (I)(parity ^ 1) * (I)g.V2, row = ((I)k * N + j) * H;
+  Nbrs<I> r;
+  r.own = (I)parity * (I)g.V2 + row + m;
+  r.xp = ob + row + xp;
+  r.xm = ob + row + xm;
+  r.jp = ob + ((I)k * N + wrap_inc(j, N)) * H + m;
+  r.jm = ob + ((I)k * N + wrap_dec(j, N)) * H + m;
+  r.kp = ob + ((I)wrap_inc(k, g.Nz) * N + j) * H + m;
+  r.km = ob + ((I)wrap_dec(k, g.Nz) * N + j) * H + m;
+  return r;
+}
+template <typename I>
+__device__ __forceinline__ double nbr_sum(const double *P, const Nbrs<I> &o) {
+  return (P[o.xp] + P[o.xm]) + (P[o.jp] + P[o.jm]) + (P[o.kp] + P[o.km]);
+}
+
+// The four normals of site nat in the sub-step of key sk.
+__device__ __forceinline__ void site_normals(uint64_t sk, long long nat, double (&xi)[4]) {
+  Xoro rng = stream_at(sk, (uint64_t)nat);
+  const uint64_t r1 = rng.next(), r2 = rng.next(), r3 = rng.next(), r4 = rng.next();
+  box_muller(r1, r2, xi[0], xi[1]);
+  box_muller(r3, r4, xi[2], xi[3]);
+}
+
+// Euler-Maruyama Model A step at one site (Jacobi: reads `in`, writes phi of
+// `out`); acc: the new phi.  The noise is drawn before the wait for the previous
+// kernel.  I: the element offset type (int when idx32 holds).
+template <bool INJECTED, typename I>
+__device__ __forceinline__ void em_site(const Fields &in, const Fields &out, const Geo &g, const EmArgs &a, int parity,
+                                        int m, int j, int k, double (&acc)[4]) {
+  const long long nat = (long long)nat_index_t<I>(g, 2 * m + ((parity + j + k) & 1), j, k);
+  double xi[4];
+  if (!INJECTED) site_normals(a.sk, nat, xi);
+  const Nbrs<I> o = nbrs_of<I>(g, parity, m, j, k);
+  pdl_wait();
+  if (INJECTED) {
 #pragma unroll
-  for (int parity = 0; parity < 2; ++parity) {
-    const int s = (parity + j + k) & 1;
-    const int i = 2 * m + s;
-    int xm = m - 1 + s, xp = m + s;
-    if (xm < 0) xm += H;
-    if (xp == H) xp = 0;
-    const I own = (I)parity * (I)g.V2 + row + m;
-    const I ob = (I)(parity ^ 1) * (I)g.V2;
-    const I orow = ob + row;
-    const long long nat = (long long)nat_index_t<I>(g, i, j, k);
-    double xi[4];
-    if (INJECTED) {
+    for (int l = 0; l < 4; ++l) xi[l] = a.xi[(long long)l * global_sites(g) + nat];
+  }
+  double c[4];
 #pragma unroll
-      for (int l = 0; l < 4; ++l) xi[l] = a.xi[(long long)l * global_sites(g) + nat];
-    } else {
-      Xoro rng = stream_at(a.sk, (uint64_t)nat);
-      const uint64_t r1 = rng.next(), r2 = rng.next(), r3 = rng.next(), r4 = rng.next();
-      box_muller(r1, r2, xi[0], xi[1]);
-      box_muller(r3, r4, xi[2], xi[3]);
-    }
-    double c[4];
+  for (int l = 0; l < 4; ++l) c[l] = in.c[l][o.own];
+  const double p2 = c[0] * c[0] + c[1] * c[1] + c[2] * c[2] + c[3] * c[3];
 #pragma unroll
-    for (int l = 0; l < 4; ++l) c[l] = in.c[l][own];
-    const double p2 = c[0] * c[0] + c[1] * c[1] + c[2] * c[2] + c[3] * c[3];
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      const double *P = in.c[l];
-      const double heff = (P[orow + xp] + P[orow + xm]) + (P[ob + rjp] + P[ob + rjm]) + (P[ob + rkp] + P[ob + rkm]);
-      double fo = -heff + a.c6 * c[l] + a.lambda * p2 * c[l];
-      if (l == 0) fo -= a.H;
-      const double v = c[l] - a.dtg * fo + a.sq * xi[l];
-      out.c[l][own] = v;
-      acc[l] += v;
-    }
+  for (int l = 0; l < 4; ++l) {
+    double fo = -nbr_sum(in.c[l], o) + a.c6 * c[l] + a.lambda * p2 * c[l];
+    if (l == 0) fo -= a.H;
+    acc[l] = c[l] - a.dtg * fo + a.sq * xi[l];
+    out.c[l][o.own] = acc[l];
   }
 }
 
-// One thread per site pair (element m of both parity half rows of row (j, k)),
-// flat over the V/2 pairs.  AVG: also the volume averages of the new phi into
-// avg_out[0..3] (grid_sum4).  Six 256-thread CTAs per SM (40 registers): the
-// step is bound by issue and its loads' latency, and measured fastest there
-// (0.399 ms per 256^3 step against 0.404 at five, 0.420 at four, 0.399 at
-// seven or eight with more spill).
-template <bool INJECTED, bool AVG, typename I>
-__global__ void __launch_bounds__(kThreads, 6) em_kernel(Fields in, Fields out, Geo g, EmArgs a, double *partial,
-                                                      unsigned *done, double *avg_out) {
-  const long long idx = (long long)blockIdx.x * kThreads + threadIdx.x;
+// SUM: also the sums of the new phi, a row per block.
+template <bool INJECTED, bool SUM, typename I>
+__global__ void __launch_bounds__(kSiteThreads, kEmBlocks) em_kernel(Fields in, Fields out, Geo g, EmArgs a, double *partial) {
+  pdl_launch();
+  int parity, m, j;
   double acc[4] = {0, 0, 0, 0};
-  if (idx < g.V2) {
-    int m, j, k;
-    pair_coords(idx, g, m, j, k);
-    em_pair<INJECTED, I>(in, out, g, a, m, j, k, acc);
-  }
-  if (AVG) grid_sum4<kThreads>(acc, partial, done, avg_out, 1.0 / (2.0 * (double)g.V2), false);
+  if (all_site(g, blockIdx.x, parity, m, j)) em_site<INJECTED, I>(in, out, g, a, parity, m, j, blockIdx.y, acc);
+  if (SUM) block_sum4<kSiteThreads>(acc, partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 4);
 }
 
-// Adjoint of the Euler-Maruyama step for one site pair (see em_adjoint_kernel).
-// Both parities of site pair (m, j, k); adds the parameter sums into v[0..3].
-template <typename I = long long>
-__device__ __forceinline__ void em_adjoint_pair(const Fields &phi, const Fields &lin, const Fields &lout, const Geo &g,
-                                                const EmAdjArgs &a, int m, int j, int k, double (&v)[4]) {
-  const int H = g.H, N = g.N;
-  const I row = ((I)k * N + j) * H;
-  const I rjp = ((I)k * N + wrap_inc(j, N)) * H + m;
-  const I rjm = ((I)k * N + wrap_dec(j, N)) * H + m;
-  const I rkp = ((I)wrap_inc(k, N) * N + j) * H + m;
-  const I rkm = ((I)wrap_dec(k, N) * N + j) * H + m;
-  double gm = 0, gla = 0, gh = 0, gg = 0;
+// Adjoint of the Euler-Maruyama step at one site (see em_adjoint_kernel); v: its
+// shares of the parameter sums.  gl: the loss gradient added to the adjoint.
+template <typename I, typename GL>
+__device__ __forceinline__ void em_adjoint_site(const Fields &phi, const Fields &lin, const Fields &lout, const Geo &g,
+                                                const EmAdjArgs &a, int parity, int m, int j, int k, GL gl,
+                                                double (&v)[4]) {
+  const long long nat = (long long)nat_index_t<I>(g, 2 * m + ((parity + j + k) & 1), j, k);
+  double xi[4];
+  site_normals(a.sk, nat, xi);
+  const Nbrs<I> o = nbrs_of<I>(g, parity, m, j, k);
+  pdl_wait();
+  double c[4], l[4];
 #pragma unroll
-  for (int parity = 0; parity < 2; ++parity) {
-    const int s = (parity + j + k) & 1;
-    int xm = m - 1 + s, xp = m + s;
-    if (xm < 0) xm += H;
-    if (xp == H) xp = 0;
-    const I own = (I)parity * (I)g.V2 + row + m;
-    const I ob = (I)(parity ^ 1) * (I)g.V2;
-    const I orow = ob + row;
-    const long long nat = (long long)(((I)k * N + j) * N + 2 * m + s);
-    double c[4], l[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      c[b] = phi.c[b][own];
-      l[b] = lin.c[b][own];
-    }
-    Xoro rng = stream_at(a.sk, (uint64_t)nat);
-    double xi[4];
-    const uint64_t r1 = rng.next(), r2 = rng.next(), r3 = rng.next(), r4 = rng.next();
-    box_muller(r1, r2, xi[0], xi[1]);
-    box_muller(r3, r4, xi[2], xi[3]);
-    const double p2 = c[0] * c[0] + c[1] * c[1] + c[2] * c[2] + c[3] * c[3];
-    const double dot = c[0] * l[0] + c[1] * l[1] + c[2] * l[2] + c[3] * l[3];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const double *P = phi.c[b], *Lm = lin.c[b];
-      const double hf = (P[orow + xp] + P[orow + xm]) + (P[ob + rjp] + P[ob + rjm]) + (P[ob + rkp] + P[ob + rkm]);
-      const double nl = (Lm[orow + xp] + Lm[orow + xm]) + (Lm[ob + rjp] + Lm[ob + rjm]) + (Lm[ob + rkp] + Lm[ob + rkm]);
-      const double jl = a.c6 * l[b] + a.lambda * (p2 * l[b] + 2.0 * c[b] * dot) - nl;
-      lout.c[b][own] = l[b] - a.dtg * jl + a.gl[b];
-      double F = -hf + a.c6 * c[b] + a.lambda * p2 * c[b];
-      if (b == 0) F -= a.H;
-      gg += l[b] * (-a.dt * F + a.cxi * xi[b]);
-    }
-    gm += -a.dtg * dot;
-    gla += -a.dtg * p2 * dot;
-    gh += a.dtg * l[0];
+  for (int b = 0; b < 4; ++b) {
+    c[b] = phi.c[b][o.own];
+    l[b] = lin.c[b][o.own];
   }
-  v[0] += gm;
-  v[1] += gla;
-  v[2] += gh;
-  v[3] += gg;
+  const double p2 = c[0] * c[0] + c[1] * c[1] + c[2] * c[2] + c[3] * c[3];
+  const double dot = c[0] * l[0] + c[1] * l[1] + c[2] * l[2] + c[3] * l[3];
+  double gg = 0;
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const double hf = nbr_sum(phi.c[b], o), nl = nbr_sum(lin.c[b], o);
+    const double jl = a.c6 * l[b] + a.lambda * (p2 * l[b] + 2.0 * c[b] * dot) - nl;
+    lout.c[b][o.own] = l[b] - a.dtg * jl + gl(b);
+    double F = -hf + a.c6 * c[b] + a.lambda * p2 * c[b];
+    if (b == 0) F -= a.H;
+    gg += l[b] * (-a.dt * F + a.cxi * xi[b]);
+  }
+  v[0] = -a.dtg * dot;
+  v[1] = -a.dtg * p2 * dot;
+  v[2] = a.dtg * l[0];
+  v[3] = gg;
 }
 
 // ----------------------------------------------------------------------------
@@ -1970,41 +2003,6 @@ __global__ void __launch_bounds__(128, 16) batch_charge_kernel(const RepDesc *__
 }
 
 // ---- differentiable Euler-Maruyama runs of an ensemble ---------------------
-// Per-replica sums of v[0..3] over the replica's blocks first[r] ..
-// first[r] + count[r] - 1 (contiguous in the grid): the replica's last block to
-// finish adds the block partials in block order into out[0..3] (accumulating
-// when add).  done[r] is zero on entry and re-armed.
-__device__ __forceinline__ void rep_sum4(double (&v)[4], int r, int local, int nloc, double *partial, unsigned *done,
-                                         double *out, double scale, bool add) {
-  constexpr int NW = 4;  // 128 threads
-  __shared__ double sm[4][NW];
-  __shared__ bool last;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    warp_sum(v[q]);
-    if (lane == 0) sm[q][warp] = v[q];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) partial[(size_t)blockIdx.x * 4 + q] = ((sm[q][0] + sm[q][1]) + sm[q][2]) + sm[q][3];
-    __threadfence();
-    last = atomicAdd(done + r, 1u) == (unsigned)(nloc - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  const size_t b0 = (size_t)(blockIdx.x - local);
-  if (warp < 4) {
-    double t = 0;
-    for (int b = lane; b < nloc; b += 32) t += __ldcg(partial + (b0 + b) * 4 + warp);
-    warp_sum(t);
-    if (lane == 0) out[warp] = add ? out[warp] + t * scale : t * scale;
-  }
-  if (threadIdx.x == 0) done[r] = 0u;
-}
-
 __device__ __forceinline__ Fields diff_planes(double *base, long long V, long long first) {
   Fields f{};
 #pragma unroll
@@ -2023,57 +2021,102 @@ __device__ __forceinline__ EmArgs rep_em_args(const RepDesc &R, unsigned long lo
   return a;
 }
 
-__global__ void __launch_bounds__(128) batch_em_fwd_kernel(const RepDesc *__restrict__ d, const DiffDesc *__restrict__ dd,
-                                                           const int *__restrict__ rep, const int *__restrict__ first,
-                                                           const int *__restrict__ count, int phase,
-                                                           unsigned long long ctr, double t, double dt, int n,
-                                                           double *partial, unsigned *done) {
-  const int r = rep[blockIdx.x];
-  const RepDesc &R = d[r];
-  const DiffDesc &D = dd[r];
-  const int local = blockIdx.x - first[r];
-  int m, j, k;
-  double acc[4] = {0, 0, 0, 0};
-  if (plane_coords(R, local, m, j, k))
-    em_pair<false>(rep_fields(R, phase, phase), rep_fields(R, phase ^ 1, phase ^ 1), R.g, rep_em_args(R, ctr, t, dt), m,
-                   j, k, acc);
-  rep_sum4(acc, r, local, count[r], partial, done, D.avg + (size_t)(n + 1) * 4, 1.0 / (double)D.V, false);
+// Blocks of the plane map: 256 threads, both halves of 128 elements (as all_site).
+__device__ __forceinline__ bool rep_site(const RepDesc &R, int local, int &parity, int &m, int &j, int &k) {
+  k = local / R.nchunk;
+  return all_site(R.g, local - k * R.nchunk, parity, m, j);
 }
 
-__global__ void __launch_bounds__(128) batch_em_seg_kernel(const RepDesc *__restrict__ d, const DiffDesc *__restrict__ dd,
-                                                           const int *__restrict__ rep, const int *__restrict__ first,
-                                                           int slot, unsigned long long ctr, double t, double dt) {
+// Forward step: phi of the lattice buffer `phase` -> phase ^ 1, the sums of the
+// new phi into the block's row of `partial`.
+template <typename I>
+__global__ void __launch_bounds__(kSiteThreads, kEmBlocks) batch_em_fwd_kernel(const RepDesc *__restrict__ d,
+                                                                    const int *__restrict__ rep,
+                                                                    const int *__restrict__ first, int phase,
+                                                                    unsigned long long ctr, double t, double dt,
+                                                                    double *partial) {
+  pdl_launch();
+  const int r = rep[blockIdx.x];
+  const RepDesc &R = d[r];
+  int parity, m, j, k;
+  double acc[4] = {0, 0, 0, 0};
+  if (rep_site(R, blockIdx.x - first[r], parity, m, j, k))
+    em_site<false, I>(rep_fields(R, phase, phase), rep_fields(R, phase ^ 1, phase ^ 1), R.g, rep_em_args(R, ctr, t, dt),
+                      parity, m, j, k, acc);
+  block_sum4<kSiteThreads>(acc, partial + (size_t)blockIdx.x * 4);
+}
+
+template <typename I>
+__global__ void __launch_bounds__(kSiteThreads, kEmBlocks) batch_em_seg_kernel(const RepDesc *__restrict__ d,
+                                                                    const DiffDesc *__restrict__ dd,
+                                                                    const int *__restrict__ rep,
+                                                                    const int *__restrict__ first, int slot,
+                                                                    unsigned long long ctr, double t, double dt) {
+  pdl_launch();
   const int r = rep[blockIdx.x];
   const RepDesc &R = d[r];
   const DiffDesc &D = dd[r];
-  int m, j, k;
-  if (!plane_coords(R, blockIdx.x - first[r], m, j, k)) return;
-  double acc[4] = {0, 0, 0, 0};
-  em_pair<false>(diff_planes(D.seg, D.V, 4LL * slot), diff_planes(D.seg, D.V, 4LL * (slot + 1)), R.g,
-                 rep_em_args(R, ctr, t, dt), m, j, k, acc);
+  int parity, m, j, k;
+  if (!rep_site(R, blockIdx.x - first[r], parity, m, j, k)) return;
+  double acc[4];
+  em_site<false, I>(diff_planes(D.seg, D.V, 4LL * slot), diff_planes(D.seg, D.V, 4LL * (slot + 1)), R.g,
+                    rep_em_args(R, ctr, t, dt), parity, m, j, k, acc);
+}
+
+// Sums of phi of the lattice buffer `phase`, a row per block.
+__global__ void __launch_bounds__(kSiteThreads) batch_phi_sum_kernel(const RepDesc *__restrict__ d,
+                                                                     const int *__restrict__ rep,
+                                                                     const int *__restrict__ first, int phase,
+                                                                     double *partial) {
+  const int r = rep[blockIdx.x];
+  const RepDesc &R = d[r];
+  int parity, m, j, k;
+  double v[4] = {0, 0, 0, 0};
+  if (rep_site(R, blockIdx.x - first[r], parity, m, j, k)) {
+    const long long o = (long long)parity * R.g.V2 + ((long long)k * R.g.N + j) * R.g.H + m;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) v[l] = R.base[phase][(long long)l * R.pstride + o];
+  }
+  block_sum4<kSiteThreads>(v, partial + (size_t)blockIdx.x * 4);
+}
+
+// Block (replica r, slot): the rows of r's blocks in src[slot][nblocks][4] into
+// row row0 + slot of r's averages (WHAT 0, scaled by 1 / V) or of its gradient
+// rows (1); WHAT 2: r's n gradient rows into its gradient.
+template <int WHAT>
+__global__ void __launch_bounds__(kSumThreads) batch_sum_kernel(const DiffDesc *__restrict__ dd,
+                                                                const int *__restrict__ first,
+                                                                const int *__restrict__ count, const double *src,
+                                                                int nblocks, int row0, int n) {
+  const int r = blockIdx.x;
+  const DiffDesc &D = dd[r];
+  if (WHAT == 2) {
+    sum_rows(D.gs, 0, n, 1.0, D.grad);
+    return;
+  }
+  const size_t row = ((size_t)row0 + blockIdx.y) * 4;
+  sum_rows(src + (size_t)blockIdx.y * nblocks * 4, first[r], first[r] + count[r], WHAT == 0 ? 1.0 / (double)D.V : 1.0,
+           (WHAT == 0 ? D.avg : D.gs) + row);
 }
 
 // dJ/dphi_a(n) of J = w0 obs0 + w1 obs1 (the per-replica averages of the run)
-__device__ __forceinline__ void rep_gl(const DiffDesc &D, int n, int b, int S, double gl[4]) {
-  gl[0] = gl[1] = gl[2] = gl[3] = 0.0;
-  if (n <= b) return;
+__device__ __forceinline__ double rep_gl(const DiffDesc &D, int n, int b, int S, int a) {
+  if (n <= b) return 0.0;
   const double M = (double)(S - b);
-  gl[0] = D.w[0] / ((double)D.V * M);
-#pragma unroll
-  for (int a = 1; a < 4; ++a) gl[a] = D.w[1] * 2.0 * D.avg[(size_t)n * 4 + a] / M;
+  return a == 0 ? D.w[0] / ((double)D.V * M) : D.w[1] * 2.0 * D.avg[(size_t)n * 4 + a] / M;
 }
 
-__global__ void __launch_bounds__(128, 4) batch_em_adj_kernel(const RepDesc *__restrict__ d,
-                                                              const DiffDesc *__restrict__ dd,
-                                                              const int *__restrict__ rep,
-                                                              const int *__restrict__ first,
-                                                              const int *__restrict__ count, int slot, int cur, int n,
-                                                              int b, int S, unsigned long long ctr, double t, double dt,
-                                                              double *partial, unsigned *done) {
+template <typename I>
+__global__ void __launch_bounds__(kSiteThreads, kEmAdjBlocks) batch_em_adj_kernel(const RepDesc *__restrict__ d,
+                                                                    const DiffDesc *__restrict__ dd,
+                                                                    const int *__restrict__ rep,
+                                                                    const int *__restrict__ first, int slot, int cur,
+                                                                    int n, int b, int S, unsigned long long ctr,
+                                                                    double t, double dt, double *partial) {
+  pdl_launch();
   const int r = rep[blockIdx.x];
   const RepDesc &R = d[r];
   const DiffDesc &D = dd[r];
-  const int local = blockIdx.x - first[r];
   EmAdjArgs a{};
   a.c6 = 6.0 + __dadd_rn(R.mass0, __dmul_rn(R.dmassdt, t));
   a.dtg = dt * R.gamma;
@@ -2081,14 +2124,14 @@ __global__ void __launch_bounds__(128, 4) batch_em_adj_kernel(const RepDesc *__r
   a.lambda = R.lambda;
   a.H = R.H;
   a.cxi = sqrt(2.0 * dt) / (2.0 * sqrt(R.gamma));
-  rep_gl(D, n, b, S, a.gl);
   a.sk = sub_key(R.key, ctr);
   double v[4] = {0, 0, 0, 0};
-  int m, j, k;
-  if (plane_coords(R, local, m, j, k))
-    em_adjoint_pair(diff_planes(D.seg, D.V, 4LL * slot), diff_planes(D.lam, D.V, 4LL * cur),
-                    diff_planes(D.lam, D.V, 4LL * (cur ^ 1)), R.g, a, m, j, k, v);
-  rep_sum4(v, r, local, count[r], partial, done, D.grad, 1.0, true);
+  int parity, m, j, k;
+  if (rep_site(R, blockIdx.x - first[r], parity, m, j, k))
+    em_adjoint_site<I>(diff_planes(D.seg, D.V, 4LL * slot), diff_planes(D.lam, D.V, 4LL * cur),
+                       diff_planes(D.lam, D.V, 4LL * (cur ^ 1)), R.g, a, parity, m, j, k,
+                       [&](int q) { return rep_gl(D, n, b, S, q); }, v);
+  block_sum4<kSiteThreads>(v, partial + (size_t)blockIdx.x * 4);
 }
 
 __global__ void __launch_bounds__(128) batch_diff_copy_kernel(const RepDesc *__restrict__ d,
@@ -2102,8 +2145,9 @@ __global__ void __launch_bounds__(128) batch_diff_copy_kernel(const RepDesc *__r
   int m, j, k;
   if (!plane_coords(R, blockIdx.x - first[r], m, j, k)) return;
   const long long row = ((long long)k * R.g.N + j) * R.g.H + m;
-  double gl[4];
-  if (dir == 2) rep_gl(D, S, b, S, gl);
+  double gl[4] = {0, 0, 0, 0};
+  if (dir == 2)
+    for (int l = 0; l < 4; ++l) gl[l] = rep_gl(D, S, b, S, l);
 #pragma unroll
   for (int l = 0; l < 4; ++l)
 #pragma unroll
@@ -2115,23 +2159,20 @@ __global__ void __launch_bounds__(128) batch_diff_copy_kernel(const RepDesc *__r
     }
 }
 
-__global__ void __launch_bounds__(128) batch_em_kernel(const RepDesc *__restrict__ d, const EnsDyn *__restrict__ dyn,
-                                                       const int *__restrict__ rep, const int *__restrict__ first,
-                                                       int phase_in, double dt, int ctr_off) {
+template <typename I>
+__global__ void __launch_bounds__(kSiteThreads, kEmBlocks) batch_em_kernel(const RepDesc *__restrict__ d,
+                                                                const EnsDyn *__restrict__ dyn,
+                                                                const int *__restrict__ rep,
+                                                                const int *__restrict__ first, int phase_in, double dt,
+                                                                int ctr_off) {
   const int r = rep[blockIdx.x];
   const RepDesc &R = d[r];
   const EnsDyn y = *dyn;
-  int m, j, k;
-  if (!plane_coords(R, blockIdx.x - first[r], m, j, k)) return;
-  EmArgs a{};
-  a.c6 = 6.0 + rep_mass(R, y);
-  a.dtg = dt * R.gamma;
-  a.sq = sqrt(2.0 * R.gamma * dt);
-  a.lambda = R.lambda;
-  a.H = R.H;
-  a.sk = sub_key(R.key, y.ctr + (unsigned long long)ctr_off);
-  double acc[4] = {0, 0, 0, 0};
-  em_pair<false>(rep_fields(R, phase_in, phase_in), rep_fields(R, phase_in ^ 1, phase_in ^ 1), R.g, a, m, j, k, acc);
+  int parity, m, j, k;
+  if (!rep_site(R, blockIdx.x - first[r], parity, m, j, k)) return;
+  double acc[4];
+  em_site<false, I>(rep_fields(R, phase_in, phase_in), rep_fields(R, phase_in ^ 1, phase_in ^ 1), R.g,
+                    rep_em_args(R, y.ctr + (unsigned long long)ctr_off, y.t, dt), parity, m, j, k, acc);
 }
 
 template <int TX, int TY>
@@ -2349,23 +2390,16 @@ __global__ void batch_oavg_final_kernel(const RepDesc *__restrict__ d, const int
 // (the lattice Laplacian is symmetric), and the parameter sensitivities are
 //   dL/dm^2 += -dtG (phi . lam),  dL/dlambda += -dtG phi^2 (phi . lam),
 //   dL/dH += dtG lam_0,  dL/dG += lam . (-dt F + sqrt(2dt)/(2 sqrt G) xi).
-// One thread per site pair, flat over the V/2 pairs; the parameter sums are
-// accumulated into g4[0..3] (grid_sum4).
-// One thread per site pair, flat over the V/2 pairs; the parameter sums are
-// accumulated into g4[0..3] (grid_sum4).
-constexpr int kAdjThreads = 128;
+// One thread per site; the parameter sums leave as a row per block.
 template <typename I>
-__global__ void __launch_bounds__(kAdjThreads, 4) em_adjoint_kernel(Fields phi, Fields lin, Fields lout, Geo g,
-                                                                    EmAdjArgs a, double *partial, unsigned *done,
-                                                                    double *g4) {
-  const long long idx = (long long)blockIdx.x * kAdjThreads + threadIdx.x;
+__global__ void __launch_bounds__(kSiteThreads, kEmAdjBlocks) em_adjoint_kernel(Fields phi, Fields lin, Fields lout, Geo g,
+                                                                  EmAdjArgs a, double *partial) {
+  pdl_launch();
   double v[4] = {0, 0, 0, 0};
-  if (idx < g.V2) {
-    int m, j, k;
-    pair_coords(idx, g, m, j, k);
-    em_adjoint_pair<I>(phi, lin, lout, g, a, m, j, k, v);
-  }
-  grid_sum4<kAdjThreads>(v, partial, done, g4, 1.0, true);
+  int parity, m, j;
+  if (all_site(g, blockIdx.x, parity, m, j))
+    em_adjoint_site<I>(phi, lin, lout, g, a, parity, m, j, blockIdx.y, [&](int q) { return a.gl[q]; }, v);
+  block_sum4<kSiteThreads>(v, partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 4);
 }
 
 // ----------------------------------------------------------------------------
@@ -2383,30 +2417,9 @@ __global__ void __launch_bounds__(kAdjThreads, 4) em_adjoint_kernel(Fields phi, 
 __host__ __device__ constexpr int pair_a(int c) { return c < 3 ? 0 : (c == 3 ? 2 : (c == 4 ? 3 : 1)); }
 __host__ __device__ constexpr int pair_b(int c) { return c < 3 ? c + 1 : (c == 3 ? 3 : (c == 4 ? 1 : 2)); }
 
-struct SiteNbrs {
-  long long own, o[6];  // x+, x-, y+, y-, z+, z-
-};
-
-__device__ __forceinline__ SiteNbrs site_nbrs(const Geo &g, int m, int j, int k, int parity) {
-  const int H = g.H, N = g.N;
-  const long long row = ((long long)k * N + j) * H;
-  const int s = (parity + j + k) & 1;
-  int xm = m - 1 + s, xp = m + s;
-  if (xm < 0) xm += H;
-  if (xp == H) xp = 0;
-  const long long ob = (long long)(parity ^ 1) * g.V2;
-  SiteNbrs r;
-  r.own = (long long)parity * g.V2 + row + m;
-  r.o[0] = ob + row + xp;
-  r.o[1] = ob + row + xm;
-  r.o[2] = ob + ((long long)k * N + wrap_inc(j, N)) * H + m;
-  r.o[3] = ob + ((long long)k * N + wrap_dec(j, N)) * H + m;
-  r.o[4] = ob + ((long long)wrap_inc(k, N) * N + j) * H + m;
-  r.o[5] = ob + ((long long)wrap_dec(k, N) * N + j) * H + m;
-  return r;
-}
-
 __global__ void __launch_bounds__(kThreads) rot_phi_kernel(Fields u, Fields P1, long long V, double k) {
+  pdl_launch();
+  pdl_wait();
   const long long n = (long long)blockIdx.x * kThreads + threadIdx.x;
   if (n >= V) return;
   double ph[4], q[6];
@@ -2419,116 +2432,102 @@ __global__ void __launch_bounds__(kThreads) rot_phi_kernel(Fields u, Fields P1, 
   for (int l = 0; l < 4; ++l) P1.c[l][n] = ph[l];
 }
 
-__global__ void __launch_bounds__(128) ideal_adj_a_kernel(Fields u, Fields lin, Fields P1, Fields PB, Fields QB, Geo g,
-                                                          IdealAdjArgs a, double *partial, unsigned *done,
-                                                          double *g4) {
-  const long long idx = (long long)blockIdx.x * 128 + threadIdx.x;
-  double hb = 0;
-  if (idx < g.V2) {
-    int m, j, k;
-    pair_coords(idx, g, m, j, k);
-#pragma unroll 1
-    for (int parity = 0; parity < 2; ++parity) {
-      const SiteNbrs sn = site_nbrs(g, m, j, k, parity);
-      double c[4], xp[4], xm[4], yp[4], ym[4], zp[4], zm[4];
+__global__ void __launch_bounds__(kSiteThreads, kIdealAdjBlocks) ideal_adj_a_kernel(Fields u, Fields lin, Fields P1, Fields PB, Fields QB,
+                                                                   Geo g, IdealAdjArgs a, double *partial) {
+  pdl_launch();
+  pdl_wait();
+  double v[4] = {0, 0, 0, 0};
+  int parity, m, j;
+  if (all_site(g, blockIdx.x, parity, m, j)) {
+    const Nbrs<long long> o = nbrs_of<long long>(g, parity, m, j, blockIdx.y);
+    // n' exactly as the forward computes it (ideal_tile, ideal_tma_kernel)
+    double c[4], q2[6], S[4];
 #pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        const double *P = P1.c[l];
-        c[l] = P[sn.own];
-        xp[l] = P[sn.o[0]];
-        xm[l] = P[sn.o[1]];
-        yp[l] = P[sn.o[2]];
-        ym[l] = P[sn.o[3]];
-        zp[l] = P[sn.o[4]];
-        zm[l] = P[sn.o[5]];
-      }
-      // n' exactly as the forward computes it (ideal_tile, ideal_tma_kernel)
-      double q2[6], S[4];
-#pragma unroll
-      for (int l = 0; l < 4; ++l) S[l] = ((xp[l] + xm[l]) + (yp[l] + ym[l])) + (zp[l] + zm[l]);
-#pragma unroll
-      for (int s = 0; s < 6; ++s) q2[s] = u.c[4 + s][sn.own];
-      charge_currents(c, S, a.dt, a.a2, a.H, q2);
-      double ob[4], pb[4], qb[6];
-#pragma unroll
-      for (int l = 0; l < 4; ++l) ob[l] = lin.c[l][sn.own];
-      rotate_site_adj(c, q2, a.k, ob, pb, qb);
-#pragma unroll
-      for (int l = 0; l < 4; ++l) PB.c[l][sn.own] = pb[l];
-#pragma unroll
-      for (int s = 0; s < 6; ++s) {
-        const double Q = lin.c[4 + s][sn.own] + qb[s];
-        QB.c[s][sn.own] = Q;
-        if (s < 3) hb += -a.dt * Q * c[s + 1];
-      }
+    for (int l = 0; l < 4; ++l) {
+      c[l] = P1.c[l][o.own];
+      S[l] = nbr_sum(P1.c[l], o);
     }
+#pragma unroll
+    for (int s = 0; s < 6; ++s) q2[s] = u.c[4 + s][o.own];
+    charge_currents(c, S, a.dt, a.a2, a.H, q2);
+    double ob[4], pb[4], qb[6];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) ob[l] = lin.c[l][o.own];
+    rotate_site_adj(c, q2, a.k, ob, pb, qb);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) PB.c[l][o.own] = pb[l];
+    double hb = 0;
+#pragma unroll
+    for (int s = 0; s < 6; ++s) {
+      const double Q = lin.c[4 + s][o.own] + qb[s];
+      QB.c[s][o.own] = Q;
+      if (s < 3) hb += -a.dt * Q * c[s + 1];
+    }
+    v[2] = hb;
   }
-  double v[4] = {0.0, 0.0, hb, 0.0};
-  grid_sum4<128>(v, partial, done, g4, 1.0, true);
+  block_sum4<kSiteThreads>(v, partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 4);
 }
 
-__global__ void __launch_bounds__(128) ideal_adj_b_kernel(Fields u, Fields lout, Fields P1, Fields PB, Fields QB, Geo g,
-                                                          IdealAdjArgs a) {
-  const long long idx = (long long)blockIdx.x * 128 + threadIdx.x;
-  if (idx >= g.V2) return;
-  int m, j, k;
-  pair_coords(idx, g, m, j, k);
-#pragma unroll 1
-  for (int parity = 0; parity < 2; ++parity) {
-    const SiteNbrs sn = site_nbrs(g, m, j, k, parity);
-    double S[4] = {0, 0, 0, 0}, Na[6] = {0, 0, 0, 0, 0, 0}, Nb[6] = {0, 0, 0, 0, 0, 0};
+__global__ void __launch_bounds__(kSiteThreads, kIdealAdjBlocks) ideal_adj_b_kernel(Fields u, Fields lout, Fields P1, Fields PB, Fields QB,
+                                                                   Geo g, IdealAdjArgs a) {
+  pdl_launch();
+  pdl_wait();
+  int parity, m, j;
+  if (!all_site(g, blockIdx.x, parity, m, j)) return;
+  const Nbrs<long long> o = nbrs_of<long long>(g, parity, m, j, blockIdx.y);
+  const long long od[6] = {o.xp, o.xm, o.jp, o.jm, o.kp, o.km};
+  double S[4] = {0, 0, 0, 0}, Na[6] = {0, 0, 0, 0, 0, 0}, Nb[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
-    for (int d = 0; d < 6; ++d) {
-      double P[4], Q[6];
+  for (int d = 0; d < 6; ++d) {
+    double P[4], Q[6];
 #pragma unroll
-      for (int l = 0; l < 4; ++l) P[l] = P1.c[l][sn.o[d]];
+    for (int l = 0; l < 4; ++l) P[l] = P1.c[l][od[d]];
 #pragma unroll
-      for (int s = 0; s < 6; ++s) Q[s] = QB.c[s][sn.o[d]];
+    for (int s = 0; s < 6; ++s) Q[s] = QB.c[s][od[d]];
 #pragma unroll
-      for (int l = 0; l < 4; ++l) S[l] += P[l];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        Na[c] += Q[c] * P[pair_b(c)];
-        Nb[c] += Q[c] * P[pair_a(c)];
-      }
-    }
-    double pb[4], Qc[6];
-#pragma unroll
-    for (int l = 0; l < 4; ++l) pb[l] = PB.c[l][sn.own];
-#pragma unroll
-    for (int s = 0; s < 6; ++s) Qc[s] = QB.c[s][sn.own];
-    const double da = a.dt * a.a2;
+    for (int l = 0; l < 4; ++l) S[l] += P[l];
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      const int ia = pair_a(c), ib = pair_b(c);
-      pb[ia] += da * (Qc[c] * S[ib] - Na[c]);
-      pb[ib] += da * (Nb[c] - Qc[c] * S[ia]);
+      Na[c] += Q[c] * P[pair_b(c)];
+      Nb[c] += Q[c] * P[pair_a(c)];
     }
-#pragma unroll
-    for (int l = 0; l < 3; ++l) pb[l + 1] += -a.dt * a.H * Qc[l];
-    double ph[4], q[6], phb[4], qb[6];
-#pragma unroll
-    for (int l = 0; l < 4; ++l) ph[l] = u.c[l][sn.own];
-#pragma unroll
-    for (int s = 0; s < 6; ++s) q[s] = u.c[4 + s][sn.own];
-    rotate_site_adj(ph, q, a.k, pb, phb, qb);
-#pragma unroll
-    for (int l = 0; l < 4; ++l) lout.c[l][sn.own] = phb[l] + a.gl[l];
-#pragma unroll
-    for (int s = 0; s < 6; ++s) lout.c[4 + s][sn.own] = Qc[s] + qb[s];
   }
+  double pb[4], Qc[6];
+#pragma unroll
+  for (int l = 0; l < 4; ++l) pb[l] = PB.c[l][o.own];
+#pragma unroll
+  for (int s = 0; s < 6; ++s) Qc[s] = QB.c[s][o.own];
+  const double da = a.dt * a.a2;
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    const int ia = pair_a(c), ib = pair_b(c);
+    pb[ia] += da * (Qc[c] * S[ib] - Na[c]);
+    pb[ib] += da * (Nb[c] - Qc[c] * S[ia]);
+  }
+#pragma unroll
+  for (int l = 0; l < 3; ++l) pb[l + 1] += -a.dt * a.H * Qc[l];
+  double ph[4], q[6], phb[4], qb[6];
+#pragma unroll
+  for (int l = 0; l < 4; ++l) ph[l] = u.c[l][o.own];
+#pragma unroll
+  for (int s = 0; s < 6; ++s) q[s] = u.c[4 + s][o.own];
+  rotate_site_adj(ph, q, a.k, pb, phb, qb);
+#pragma unroll
+  for (int l = 0; l < 4; ++l) lout.c[l][o.own] = phb[l] + a.gl[l];
+#pragma unroll
+  for (int s = 0; s < 6; ++s) lout.c[4 + s][o.own] = Qc[s] + qb[s];
 }
 
-// volume averages of phi_0..3 into out[0..3]
-__global__ void __launch_bounds__(kThreads) phi_avg_kernel(Fields f, Geo g, double *partial, unsigned *done,
-                                                           double *out) {
-  const long long idx = (long long)blockIdx.x * kThreads + threadIdx.x;
+// sums of phi_0..3, a row per block
+__global__ void __launch_bounds__(kSiteThreads) phi_sum_kernel(Fields f, Geo g, double *partial) {
+  int parity, m, j;
   double v[4] = {0, 0, 0, 0};
-  if (idx < g.V2) {
+  if (all_site(g, blockIdx.x, parity, m, j)) {
+    const long long o = (long long)parity * g.V2 + ((long long)blockIdx.y * g.N + j) * g.H + m;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) v[b] = f.c[b][idx] + f.c[b][g.V2 + idx];
+    for (int b = 0; b < 4; ++b) v[b] = f.c[b][o];
   }
-  grid_sum4<kThreads>(v, partial, done, out, 1.0 / (2.0 * (double)g.V2), false);
+  block_sum4<kSiteThreads>(v, partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 4);
 }
 
 __global__ void fill_phi_kernel(Fields f, long long V, double v0, double v1, double v2, double v3) {
@@ -2630,17 +2629,27 @@ cudaError_t launch_hb_pass(Fields f, const Geo &g, int parity, const HbArgs &a, 
   const bool rows = g.H % 128 == 0;
   const dim3 grid = pass_grid(g, rows);
   const bool i32 = idx32(g);
-#define LGV_HBP1(I, M, T, G)                                                                                 \
-  if (rows) hb_pass_kernel<I, M, true, T, G><<<grid, 128, 0, st>>>(f, g, parity, a);                        \
-  else hb_pass_kernel<I, M, false, T, G><<<grid, 128, 0, st>>>(f, g, parity, a)
-#define LGV_HBP(I, M, G)                                                                                     \
-  if (i32) { LGV_HBP1(I, M, int, G); } else { LGV_HBP1(I, M, long long, G); }
-  if (inj) { if (mon) { LGV_HBP(true, true, false); } else { LGV_HBP(true, false, false); } }
-  else if (gauss) { if (mon) { LGV_HBP(false, true, true); } else { LGV_HBP(false, false, true); } }
-  else { if (mon) { LGV_HBP(false, true, false); } else { LGV_HBP(false, false, false); } }
+#define LGV_HBP(I, M, R, T, G) \
+  return launch_pdl(hb_pass_kernel<I, M, R, T, G>, grid, dim3(128), 0, st, f, g, parity, a)
+#define LGV_HBP_T(I, M, G)                                     \
+  if (i32) {                                                   \
+    if (rows) LGV_HBP(I, M, true, int, G);                     \
+    else LGV_HBP(I, M, false, int, G);                         \
+  } else if (rows) LGV_HBP(I, M, true, long long, G);          \
+  else LGV_HBP(I, M, false, long long, G)
+  if (inj) {
+    if (mon) LGV_HBP_T(true, true, false);
+    else LGV_HBP_T(true, false, false);
+  } else if (gauss) {
+    if (mon) LGV_HBP_T(false, true, true);
+    else LGV_HBP_T(false, false, true);
+  } else if (mon) {
+    LGV_HBP_T(false, true, false);
+  } else {
+    LGV_HBP_T(false, false, false);
+  }
+#undef LGV_HBP_T
 #undef LGV_HBP
-#undef LGV_HBP1
-  return cudaGetLastError();
 }
 
 // ---- ordered sweeps ---------------------------------------------------------
@@ -2801,8 +2810,8 @@ cudaError_t launch_charge_pass(Fields f, const Geo &g, int dir, int eoA, const C
   const bool inj = a.q != nullptr, mon = a.mon != nullptr;
   const bool i32 = idx32(g);
 #define LGV_CHP1(I, M, T)                                                                                    \
-  if (rows) charge_pass_kernel<I, M, true, T><<<grid, 128, 0, st>>>(f, g, dir, eoA, a);                     \
-  else charge_pass_kernel<I, M, false, T><<<grid, 128, 0, st>>>(f, g, dir, eoA, a)
+  return launch_pdl(rows ? charge_pass_kernel<I, M, true, T> : charge_pass_kernel<I, M, false, T>, grid, dim3(128), 0, \
+                    st, f, g, dir, eoA, a)
 #define LGV_CHP(I, M)                                                                                        \
   if (i32) { LGV_CHP1(I, M, int); } else { LGV_CHP1(I, M, long long); }
   if (inj) { if (mon) { LGV_CHP(true, true); } else { LGV_CHP(true, false); } }
@@ -2862,30 +2871,16 @@ cudaError_t launch_em(Fields in, Fields out, int N, const EmArgs &a, cudaStream_
 }
 
 cudaError_t launch_em(Fields in, Fields out, const Geo &g, const EmArgs &a, cudaStream_t st) {
-  const unsigned nb = nblocks(g.V2, kThreads);
   const bool i32 = idx32(g);
-  if (a.xi) {
-    if (i32) em_kernel<true, false, int><<<nb, kThreads, 0, st>>>(in, out, g, a, nullptr, nullptr, nullptr);
-    else em_kernel<true, false, long long><<<nb, kThreads, 0, st>>>(in, out, g, a, nullptr, nullptr, nullptr);
-  } else {
-    if (i32) em_kernel<false, false, int><<<nb, kThreads, 0, st>>>(in, out, g, a, nullptr, nullptr, nullptr);
-    else em_kernel<false, false, long long><<<nb, kThreads, 0, st>>>(in, out, g, a, nullptr, nullptr, nullptr);
-  }
-  return cudaGetLastError();
+  const auto kern = a.xi ? (i32 ? em_kernel<true, false, int> : em_kernel<true, false, long long>)
+                         : (i32 ? em_kernel<false, false, int> : em_kernel<false, false, long long>);
+  return launch_pdl(kern, site_grid(g), dim3(kSiteThreads), 0, st, in, out, g, a, nullptr);
 }
 
-cudaError_t launch_em_avg(Fields in, Fields out, int N, const EmArgs &a, double *partial, unsigned *done,
-                          double *avg_out, cudaStream_t st) {
+cudaError_t launch_em_sum(Fields in, Fields out, int N, const EmArgs &a, double *partial, cudaStream_t st) {
   const Geo g = make_geo(N);
-  const unsigned nb = nblocks(g.V2, kThreads);
-  if (idx32(g)) {
-    if (a.xi) em_kernel<true, true, int><<<nb, kThreads, 0, st>>>(in, out, g, a, partial, done, avg_out);
-    else em_kernel<false, true, int><<<nb, kThreads, 0, st>>>(in, out, g, a, partial, done, avg_out);
-  } else {
-    if (a.xi) em_kernel<true, true, long long><<<nb, kThreads, 0, st>>>(in, out, g, a, partial, done, avg_out);
-    else em_kernel<false, true, long long><<<nb, kThreads, 0, st>>>(in, out, g, a, partial, done, avg_out);
-  }
-  return cudaGetLastError();
+  const auto kern = idx32(g) ? em_kernel<false, true, int> : em_kernel<false, true, long long>;
+  return launch_pdl(kern, site_grid(g), dim3(kSiteThreads), 0, st, in, out, g, a, partial);
 }
 
 cudaError_t launch_ideal(Fields in, Fields out, int N, const IdealArgs &a, cudaStream_t st) {
@@ -3076,29 +3071,44 @@ cudaError_t launch_ens_persistent(const PersistPlan &plan, const PersistPtrs &q,
 }
 
 cudaError_t launch_batch_em(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
-                            int phase_in, double dt, int ctr_off, cudaStream_t st) {
-  batch_em_kernel<<<nblocks, 128, 0, st>>>(d, dyn, rep, first, phase_in, dt, ctr_off);
+                            int phase_in, double dt, int ctr_off, bool i32, cudaStream_t st) {
+  if (i32) batch_em_kernel<int><<<nblocks, kSiteThreads, 0, st>>>(d, dyn, rep, first, phase_in, dt, ctr_off);
+  else batch_em_kernel<long long><<<nblocks, kSiteThreads, 0, st>>>(d, dyn, rep, first, phase_in, dt, ctr_off);
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_em_fwd(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first,
-                                const int *count, int nblocks, int phase, unsigned long long ctr, double t, double dt,
-                                int n, double *partial, unsigned *done, cudaStream_t st) {
-  batch_em_fwd_kernel<<<nblocks, 128, 0, st>>>(d, dd, rep, first, count, phase, ctr, t, dt, n, partial, done);
-  return cudaGetLastError();
+cudaError_t launch_batch_em_fwd(const RepDesc *d, const int *rep, const int *first, int nblocks, int phase,
+                                unsigned long long ctr, double t, double dt, double *partial, bool i32,
+                                cudaStream_t st) {
+  return launch_pdl(i32 ? batch_em_fwd_kernel<int> : batch_em_fwd_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
+                    0, st, d, rep, first, phase, ctr, t, dt, partial);
 }
 
 cudaError_t launch_batch_em_seg(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first, int nblocks,
-                                int m, unsigned long long ctr, double t, double dt, cudaStream_t st) {
-  batch_em_seg_kernel<<<nblocks, 128, 0, st>>>(d, dd, rep, first, m, ctr, t, dt);
+                                int m, unsigned long long ctr, double t, double dt, bool i32, cudaStream_t st) {
+  return launch_pdl(i32 ? batch_em_seg_kernel<int> : batch_em_seg_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
+                    0, st, d, dd, rep, first, m, ctr, t, dt);
+}
+
+cudaError_t launch_batch_em_adj(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first, int nblocks,
+                                int m, int cur, int n, int b, int S, unsigned long long ctr, double t, double dt,
+                                double *partial, bool i32, cudaStream_t st) {
+  return launch_pdl(i32 ? batch_em_adj_kernel<int> : batch_em_adj_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
+                    0, st, d, dd, rep, first, m, cur, n, b, S, ctr, t, dt, partial);
+}
+
+cudaError_t launch_batch_phi_sum(const RepDesc *d, const int *rep, const int *first, int nblocks, int phase,
+                                 double *partial, cudaStream_t st) {
+  batch_phi_sum_kernel<<<nblocks, kSiteThreads, 0, st>>>(d, rep, first, phase, partial);
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_em_adj(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first,
-                                const int *count, int nblocks, int m, int cur, int n, int b, int S,
-                                unsigned long long ctr, double t, double dt, double *partial, unsigned *done,
-                                cudaStream_t st) {
-  batch_em_adj_kernel<<<nblocks, 128, 0, st>>>(d, dd, rep, first, count, m, cur, n, b, S, ctr, t, dt, partial, done);
+cudaError_t launch_batch_sum(const DiffDesc *dd, const int *first, const int *count, int nrep, int what,
+                             const double *src, int nblocks, int row0, int nslot, cudaStream_t st) {
+  const dim3 grid(nrep, nslot);
+  if (what == 0) batch_sum_kernel<0><<<grid, kSumThreads, 0, st>>>(dd, first, count, src, nblocks, row0, 0);
+  else if (what == 1) batch_sum_kernel<1><<<grid, kSumThreads, 0, st>>>(dd, first, count, src, nblocks, row0, 0);
+  else batch_sum_kernel<2><<<nrep, kSumThreads, 0, st>>>(dd, first, count, nullptr, 0, 0, row0);
   return cudaGetLastError();
 }
 
@@ -3134,37 +3144,46 @@ cudaError_t launch_batch_oavg_final(const RepDesc *d, const int *first, const in
 
 // ---------------------------------------------------------------------------
 // Euler-Maruyama adjoint launchers.
-size_t em_reduce_blocks(int N) {
-  const Geo g = make_geo(N);
-  return std::max<size_t>(nblocks(g.V2, kThreads), nblocks(g.V2, std::min(kAdjThreads, 128)));
+int sum_blocks(int N) {
+  const dim3 g = site_grid(make_geo(N));
+  return (int)(g.x * g.y);
+}
+
+int sum_slots(int nblocks) { return (int)std::max<long long>(1, std::min<long long>(32, (8LL << 20) / (32LL * nblocks))); }
+
+cudaError_t launch_sum_rows(const double *src, int nslot, int nb, double scale, double *rows, double *tmp,
+                            cudaStream_t st) {
+  if (nb <= 4096) {
+    sum_rows_kernel<<<nslot, kSumThreads, 0, st>>>(src, nb, scale, rows);
+  } else {
+    sum_rows_kernel<<<dim3(nslot, kSumSegs), kSumThreads, 0, st>>>(src, nb, 1.0, tmp);
+    sum_rows_kernel<<<nslot, kSumThreads, 0, st>>>(tmp, kSumSegs, scale, rows);
+  }
+  return cudaGetLastError();
 }
 
 cudaError_t launch_em_adjoint(Fields phi, Fields lam_in, Fields lam_out, int N, const EmAdjArgs &a, double *partial,
-                              unsigned *done, double *g4, cudaStream_t st) {
+                              cudaStream_t st) {
   const Geo g = make_geo(N);
-  if (idx32(g))
-    em_adjoint_kernel<int><<<nblocks(g.V2, kAdjThreads), kAdjThreads, 0, st>>>(phi, lam_in, lam_out, g, a, partial,
-                                                                              done, g4);
-  else
-    em_adjoint_kernel<long long><<<nblocks(g.V2, kAdjThreads), kAdjThreads, 0, st>>>(phi, lam_in, lam_out, g, a,
-                                                                                    partial, done, g4);
-  return cudaGetLastError();
+  return launch_pdl(idx32(g) ? em_adjoint_kernel<int> : em_adjoint_kernel<long long>, site_grid(g), dim3(kSiteThreads), 0,
+                    st, phi, lam_in, lam_out, g, a, partial);
 }
 
 cudaError_t launch_ideal_adjoint(Fields u, Fields lam_in, Fields lam_out, Fields P1, Fields PB, Fields QB, int N,
-                                 const IdealAdjArgs &a, double *partial, unsigned *done, double *g4,
-                                 cudaStream_t st) {
+                                 const IdealAdjArgs &a, double *partial, cudaStream_t st) {
   const Geo g = make_geo(N);
   const long long V = 2 * g.V2;
-  rot_phi_kernel<<<nblocks(V, kThreads), kThreads, 0, st>>>(u, P1, V, a.k);
-  ideal_adj_a_kernel<<<nblocks(g.V2, 128), 128, 0, st>>>(u, lam_in, P1, PB, QB, g, a, partial, done, g4);
-  ideal_adj_b_kernel<<<nblocks(g.V2, 128), 128, 0, st>>>(u, lam_out, P1, PB, QB, g, a);
-  return cudaGetLastError();
+  cudaError_t e = launch_pdl(rot_phi_kernel, dim3(nblocks(V, kThreads)), dim3(kThreads), 0, st, u, P1, V, a.k);
+  if (e == cudaSuccess)
+    e = launch_pdl(ideal_adj_a_kernel, site_grid(g), dim3(kSiteThreads), 0, st, u, lam_in, P1, PB, QB, g, a, partial);
+  if (e == cudaSuccess)
+    e = launch_pdl(ideal_adj_b_kernel, site_grid(g), dim3(kSiteThreads), 0, st, u, lam_out, P1, PB, QB, g, a);
+  return e;
 }
 
-cudaError_t launch_phi_avg(Fields f, int N, double *partial, unsigned *done, double *out, cudaStream_t st) {
+cudaError_t launch_phi_sum(Fields f, int N, double *partial, cudaStream_t st) {
   const Geo g = make_geo(N);
-  phi_avg_kernel<<<nblocks(g.V2, kThreads), kThreads, 0, st>>>(f, g, partial, done, out);
+  phi_sum_kernel<<<site_grid(g), kSiteThreads, 0, st>>>(f, g, partial);
   return cudaGetLastError();
 }
 
