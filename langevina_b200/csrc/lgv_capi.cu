@@ -296,6 +296,18 @@ lgv::Geo pass_geo(lgv_handle *h) {
   return g;
 }
 
+// One ideal step of the current state; the result is current afterwards.
+int ideal_step(lgv_handle *h, const lgv::IdealArgs &a) {
+  KTimer tm(h, LGV_KCLASS_IDEAL);
+  if (lgv::ideal_flat(h->N)) {  // in place, phi' in the alternate buffer
+    LGV_CK(lgv::launch_ideal_flat(h->cur, h->alt, h->cur, h->geo, a, h->stream));
+    return LGV_OK;
+  }
+  LGV_CK(lgv::launch_ideal(h->cur, h->alt, pass_geo(h), a, h->stream));
+  std::swap(h->cur, h->alt);
+  return LGV_OK;
+}
+
 int sub_ideal(lgv_handle *h, double dt) {  // IdealPV2::step (Stepper.cxx:23-66)
   double Eold = 0, Enew = 0;
   if (h->mon_on) LGV_TRY(energy_now(h, &Eold));
@@ -308,11 +320,7 @@ int sub_ideal(lgv_handle *h, double dt) {  // IdealPV2::step (Stepper.cxx:23-66)
   a.waits = h->waits_dev;
   a.wait_limit = h->wait_limit;
   LGV_TRY(halo(h, LGV_HALO_ALL));
-  {
-    KTimer tm(h, LGV_KCLASS_IDEAL);
-    LGV_CK(lgv::launch_ideal(h->cur, h->alt, pass_geo(h), a, h->stream));
-  }
-  std::swap(h->cur, h->alt);
+  LGV_TRY(ideal_step(h, a));
   if (h->mon_on) {
     LGV_TRY(energy_now(h, &Enew));
     const double dE = Enew - Eold;
@@ -1119,11 +1127,7 @@ int lgv_diff_forward(lgv_handle *h, int evolver, double dt, double t, int nsteps
         LGV_CK(cudaMemcpyAsync(A.ckpt + ((size_t)(n / K) * A.ncomp + l) * V, h->cur.c[l], V * sizeof(double),
                                cudaMemcpyDeviceToDevice, h->stream));
     LGV_TRY(sums.next(&slot));
-    if (has_ideal(evolver)) {
-      KTimer tm(h, LGV_KCLASS_IDEAL);
-      LGV_CK(lgv::launch_ideal(h->cur, h->alt, h->N, ia, h->stream));
-      std::swap(h->cur, h->alt);
-    }
+    if (has_ideal(evolver)) LGV_TRY(ideal_step(h, ia));
     if (has_em(evolver)) {
       KTimer tm(h, LGV_KCLASS_EM);
       const lgv::EmArgs e = em_args(A.p, A.key, A.ctr0 + (uint64_t)n, dt, A.tn[n]);
@@ -1198,6 +1202,11 @@ int lgv_diff_backward(lgv_handle *h, const double *w, double *grad) {
                PB = planes(A.work, V, 18, 4), QB = planes(A.work, V, 22, 6);
   auto lam = [&](int which) { return planes(A.lam, V, (size_t)which * 10, 10); };
   auto slot = [&](int m) { return planes(A.seg, V, (size_t)m * nc, nc); };
+  // one ideal step of state a into b (P1 is free between adjoint steps)
+  auto ideal = [&](const Fields &a, const Fields &b) {
+    return lgv::ideal_flat(N) ? lgv::launch_ideal_flat(a, P1, b, h->geo, ia, h->stream)
+                              : lgv::launch_ideal(a, b, N, ia, h->stream);
+  };
   int cur = 0;
   {
     double v[4];
@@ -1220,11 +1229,11 @@ int lgv_diff_backward(lgv_handle *h, const double *w, double *grad) {
         if (ev == LGV_MODELA_EM) {
           LGV_CK(lgv::launch_em(a, b, N, e, h->stream));
         } else if (ev == LGV_IDEAL_PV2) {
-          LGV_CK(lgv::launch_ideal(a, b, N, ia, h->stream));
+          LGV_CK(ideal(a, b));
         } else {
           Fields mid = b;  // phi to tmp, charges straight into the next slot
           for (int l = 0; l < 4; ++l) mid.c[l] = tmp.c[l];
-          LGV_CK(lgv::launch_ideal(a, mid, N, ia, h->stream));
+          LGV_CK(ideal(a, mid));
           LGV_CK(lgv::launch_em(mid, b, N, e, h->stream));
         }
       }
@@ -1247,7 +1256,7 @@ int lgv_diff_backward(lgv_handle *h, const double *w, double *grad) {
         for (int q = 0; q < 4; ++q) a.gl[q] = gln[q];
         LGV_CK(lgv::launch_em_adjoint(u, lam(cur), lam(cur ^ 1), N, a, psum, h->stream));
       } else {
-        LGV_CK(lgv::launch_ideal(u, tmp, N, ia, h->stream));
+        LGV_CK(ideal(u, tmp));
         LGV_CK(lgv::launch_em_adjoint(tmp, lam(cur), lamx, N, a, psum, h->stream));
         Fields lmid = lam(cur);  // charges' adjoint passes the EM step unchanged
         for (int l = 0; l < 4; ++l) lmid.c[l] = lamx.c[l];

@@ -25,6 +25,7 @@
 
 #include "lgv_ideal_tma_cta.cuh"
 #include "lgv_internal.h"
+#include "lgv_pdl.cuh"
 
 namespace lgv {
 
@@ -34,6 +35,8 @@ using namespace tma;
 
 __global__ void __launch_bounds__(NT, 2)
     ideal_tma_kernel(const __grid_constant__ TmaMaps maps, Fields in, Fields out, Geo g, int zchunk, IdealArgs a) {
+  pdl_launch();
+  pdl_wait();
   ideal_tma_cta(maps.m, in, out, g, zchunk, a, blockIdx.x, blockIdx.y,
                 g.zrev ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z);
 }
@@ -106,8 +109,7 @@ cudaError_t launch_ideal_tma(Fields in, Fields out, const Geo &g, int zchunk, co
   cudaError_t e = cudaFuncSetAttribute(ideal_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
   if (e != cudaSuccess) return e;
   dim3 grid(N / TX, N / TY, (unsigned)((g.Nz + zchunk - 1) / zchunk));
-  ideal_tma_kernel<<<grid, NT, kSmemBytes, st>>>(maps, in, out, g, zchunk, a);
-  return cudaGetLastError();
+  return launch_pdl(ideal_tma_kernel, grid, dim3(NT), kSmemBytes, st, maps, in, out, g, zchunk, a);
 }
 
 int batch_tma_blocks(int N, int zchunk) { return (N / TX) * (N / TY) * ((N + zchunk - 1) / zchunk); }

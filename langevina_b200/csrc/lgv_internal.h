@@ -280,6 +280,10 @@ cudaError_t launch_em(Fields in, Fields out, int N, const EmArgs &a, cudaStream_
 cudaError_t launch_ideal(Fields in, Fields out, int N, const IdealArgs &a, cudaStream_t st);
 cudaError_t launch_em(Fields in, Fields out, const Geo &g, const EmArgs &a, cudaStream_t st);
 cudaError_t launch_ideal(Fields in, Fields out, const Geo &g, const IdealArgs &a, cudaStream_t st);
+// The ideal step in two flat launches, for lattices where ideal_flat(N): phi'
+// goes to P1 (4 planes); `out` may be `in`.
+bool ideal_flat(int N);
+cudaError_t launch_ideal_flat(Fields in, Fields P1, Fields out, const Geo &g, const IdealArgs &a, cudaStream_t st);
 // TMA-staged ideal step (lgv_ideal_tma.cu): N divisible by 32
 bool ideal_tma_supported(int N);
 cudaError_t launch_ideal_tma(Fields in, Fields out, const Geo &g, int zchunk, const IdealArgs &a, cudaStream_t st);

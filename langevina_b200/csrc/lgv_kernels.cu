@@ -1101,11 +1101,7 @@ __global__ void __launch_bounds__(1024) charge_row_kernel(Geo g, ChargeDirArgs a
 // half.  Grid (ceil(N H / 128), planes).
 constexpr int kSiteThreads = 256;
 // resident blocks per SM of the Euler-Maruyama step, its adjoint and the ideal step's adjoint (48, 80 and 86-128 registers)
-#ifdef EMB
-constexpr int kEmBlocks = EMB, kEmAdjBlocks = AJB, kIdealAdjBlocks = 2;
-#else
 constexpr int kEmBlocks = 5, kEmAdjBlocks = 3, kIdealAdjBlocks = 2;
-#endif
 
 __device__ __forceinline__ bool all_site(const Geo &g, int chunk, int &parity, int &m, int &j) {
   parity = threadIdx.x >> 7;
@@ -1367,6 +1363,8 @@ __device__ __forceinline__ void ideal_tile(const Fields &in, const Fields &out, 
 
 template <int TX, int TY>
 __global__ void __launch_bounds__(TX *TY, 2) ideal_kernel(Fields in, Fields out, Geo g, int zchunk, IdealArgs a) {
+  pdl_launch();
+  pdl_wait();
   ideal_tile<TX, TY>(in, out, g, zchunk, a, blockIdx.x, blockIdx.y,
                     g.zrev ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z);
 }
@@ -1727,6 +1725,8 @@ __device__ __forceinline__ double warp_sum25(const double (&v)[kNObs], double *t
 __global__ void __launch_bounds__(256, 2) meas_tile_kernel(Fields f, Geo g, MeasTiles mt, double *__restrict__ xp,
                                                         double *__restrict__ yp, double *__restrict__ zp) {
   extern __shared__ __align__(16) double2 sm2[];
+  pdl_launch();
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *tab = (double *)sm2 + (size_t)warp * kNObs * kMtW;       // [warp][25][kMtW]
   double *ys = (double *)sm2 + (size_t)kMtK * kNObs * kMtW;        // [warp][row][lane]
@@ -1804,7 +1804,9 @@ __global__ void __launch_bounds__(kFinishThreads) meas_finish_kernel(const doubl
   const int N = p.N, o = blockIdx.x, axis = blockIdx.y;
   const int np = mt.npart(axis), pitch = mt.pitch(axis);
   const double *src = (axis == 0 ? xp : axis == 1 ? yp : zp) + (size_t)o * np * pitch;
+  pdl_launch();
   dft::fill_twiddles(tw, N);
+  pdl_wait();
   const int P = 1 << logP, G = kFinishThreads >> logP, grp = threadIdx.x >> logP;
   double *dst = (o < 11) ? mo.wall[axis] + (size_t)o * N : mo.ph[axis] + (size_t)(o - 11) * N;
   for (int x0 = 0; x0 < N; x0 += P) {
@@ -2432,6 +2434,34 @@ __global__ void __launch_bounds__(kThreads) rot_phi_kernel(Fields u, Fields P1, 
   for (int l = 0; l < 4; ++l) P1.c[l][n] = ph[l];
 }
 
+// The ideal step of a small lattice in two launches: rot_phi_kernel writes phi'
+// to P1, and this one, a thread per site, advects the charges with the stencil
+// on phi' and rotates phi' by the second half step.  Reads the charges of `in`,
+// writes `out`, which may be `in`.
+template <typename I>
+__global__ void __launch_bounds__(kSiteThreads, 3) ideal_flat_kernel(Fields in, Fields P1, Fields out, Geo g, IdealArgs a) {
+  pdl_launch();
+  int parity, m, j;
+  const bool ok = all_site(g, blockIdx.x, parity, m, j);
+  const Nbrs<I> o = nbrs_of<I>(g, parity, m, j, blockIdx.y);
+  pdl_wait();
+  if (!ok) return;
+  double c[4], S[4], q[6];
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    c[l] = P1.c[l][o.own];
+    S[l] = nbr_sum(P1.c[l], o);
+  }
+#pragma unroll
+  for (int s = 0; s < 6; ++s) q[s] = in.c[4 + s][o.own];
+  charge_currents(c, S, a.dt, a.a2, a.H, q);
+  rotate_site(c, q, a.dto2chi);
+#pragma unroll
+  for (int l = 0; l < 4; ++l) out.c[l][o.own] = c[l];
+#pragma unroll
+  for (int s = 0; s < 6; ++s) out.c[4 + s][o.own] = q[s];
+}
+
 __global__ void __launch_bounds__(kSiteThreads, kIdealAdjBlocks) ideal_adj_a_kernel(Fields u, Fields lin, Fields P1, Fields PB, Fields QB,
                                                                    Geo g, IdealAdjArgs a, double *partial) {
   pdl_launch();
@@ -2883,6 +2913,23 @@ cudaError_t launch_em_sum(Fields in, Fields out, int N, const EmArgs &a, double 
   return launch_pdl(kern, site_grid(g), dim3(kSiteThreads), 0, st, in, out, g, a, partial);
 }
 
+// Where the march's chunks of a few planes are a chain of latencies and the
+// fields sit in L2, two flat launches are faster although phi' takes 112 B/site
+// more: 32^3 11.6 -> 5.4 us, 64^3 15.0 -> 10.4, 96^3 42.6 -> 35.0; 128^3 92.0 and
+// 91.5, 160^3 161 and 177, 256^3 601 and 748.  Sides that 32 does not divide
+// march without TMA: 90^3 45.3 -> 28.1, 120^3 96 -> 76, 150^3 175 -> 155, 200^3
+// 402 -> 348, 250^3 713 and 749.
+bool ideal_flat(int N) { return N % 32 == 0 ? N < 128 : N <= 200; }
+
+cudaError_t launch_ideal_flat(Fields in, Fields P1, Fields out, const Geo &g, const IdealArgs &a, cudaStream_t st) {
+  const long long V = 2 * g.V2;
+  const cudaError_t e =
+      launch_pdl(rot_phi_kernel, dim3(nblocks(V, kThreads)), dim3(kThreads), 0, st, in, P1, V, a.dto2chi);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(idx32(g) ? ideal_flat_kernel<int> : ideal_flat_kernel<long long>, site_grid(g), dim3(kSiteThreads), 0,
+                    st, in, P1, out, g, a);
+}
+
 cudaError_t launch_ideal(Fields in, Fields out, int N, const IdealArgs &a, cudaStream_t st) {
   return launch_ideal(in, out, make_geo(N), a, st);
 }
@@ -2904,8 +2951,7 @@ cudaError_t launch_ideal(Fields in, Fields out, const Geo &g, const IdealArgs &a
   dim3 grid((N + TX - 1) / TX, (N + TY - 1) / TY, (unsigned)((g.Nz + zc - 1) / zc));
   cudaError_t e = allow_smem(ideal_kernel<TX, TY>, T::SMEM);
   if (e != cudaSuccess) return e;
-  ideal_kernel<TX, TY><<<grid, TX * TY, T::SMEM, st>>>(in, out, g, (int)zc, a);
-  return cudaGetLastError();
+  return launch_pdl(ideal_kernel<TX, TY>, grid, dim3(TX * TY), T::SMEM, st, in, out, g, (int)zc, a);
 }
 
 size_t energy_scratch_doubles(int N) {
@@ -2949,15 +2995,17 @@ cudaError_t launch_measure(Fields f, int N, double *scratch, unsigned *done, dou
   }
   const MeasTiles t = meas_tiles(N);
   double *xp = scratch, *yp = xp + t.len(0), *zp = yp + t.len(1);
-  const cudaError_t e = allow_smem(meas_tile_kernel, kMtSmem);
+  cudaError_t e = allow_smem(meas_tile_kernel, kMtSmem);
   if (e != cudaSuccess) return e;
-  meas_tile_kernel<<<dim3(t.it, t.jt, t.kt), 256, kMtSmem, st>>>(f, g, t, xp, yp, zp);
+  if ((e = launch_pdl(meas_tile_kernel, dim3(t.it, t.jt, t.kt), dim3(256), kMtSmem, st, f, g, t, xp, yp, zp)) !=
+      cudaSuccess)
+    return e;
   const MeasOut mo = meas_layout(dev_out, N);
   const dft::Plan p = dft::make_plan(N);
   int logP = 3;
   while (logP < 8 && (1 << logP) < N) ++logP;
-  meas_finish_kernel<<<dim3(kNObs, 3), kFinishThreads, wall_smem(p), st>>>(xp, yp, zp, t, p, logP, mo, done);
-  return cudaGetLastError();
+  return launch_pdl(meas_finish_kernel, dim3(kNObs, 3), dim3(kFinishThreads), wall_smem(p), st, xp, yp, zp, t, p, logP, mo,
+                    done);
 }
 
 cudaError_t launch_measure_partials(Fields f, const Geo &g, int klo, int nk, int kout, double *T, double *U,
