@@ -70,6 +70,7 @@ struct lgv_ensemble {
   RepDesc *dd = nullptr;
   EnsDyn *dyn = nullptr;
   BlockMap ideal_map, plane_map, slab_map, tma_map;  // tma_map: ideal step of the TMA replicas
+  BlockMap run_map;                                  // charge heat bath, both faces of a direction
   std::vector<char> tma_ok;                          // replica r takes the TMA ideal kernel
   void *gmaps = nullptr;                             // their tensor maps, [R][2][2][10] x 128 B
   double *partial = nullptr, *oavg = nullptr;
@@ -89,8 +90,9 @@ struct lgv_ensemble {
   // overlap.  LGV_ENS_CONCURRENT=0 at creation keeps them in sequence.
   bool concurrent = true;
   cudaStream_t side = nullptr;
-  // every replica's element offsets fit 31 bits (set at creation)
-  bool idx32 = false;
+  // every replica's element offsets fit 31 bits, and a plane's bytes 32 (set at creation)
+  bool idx32 = false, bytes32 = false;
+  size_t run_smem = 0;  // shared memory of a run_map block
   // one cooperative launch per step instead of one launch per sub-step
   // (lgv_ensemble_use_persistent; LGV_ENS_PERSISTENT=1 at creation), and its
   // grid barrier (arrivals, generation, error flag)
@@ -223,7 +225,7 @@ int tensor_maps(lgv_ensemble *e) {
 int configure(lgv_ensemble *e) {
   int tx = 32, ty = 8;
   lgv::ideal_tile_dims(e->tile, &tx, &ty);
-  std::vector<int> ib(e->R), pb(e->R), sb(e->R), tb(e->R);
+  std::vector<int> ib(e->R), pb(e->R), sb(e->R), tb(e->R), rb(e->R);
   for (int r = 0; r < e->R; ++r) {
     RepDesc &d = e->hd[r];
     const int N = d.g.N;
@@ -235,6 +237,7 @@ int configure(lgv_ensemble *e) {
     ib[r] = e->tma_ok[r] ? 0 : d.igx * d.igy * d.igz;
     tb[r] = e->tma_ok[r] ? lgv::batch_tma_blocks(N, d.izc) : 0;
     pb[r] = d.nchunk * N;
+    rb[r] = lgv::batch_run_blocks(N);
     sb[r] = d.nchunk * ((N + lgv::kBatchPlanes - 1) / lgv::kBatchPlanes);
   }
   ECK(cudaMemcpy(e->dd, e->hd.data(), e->R * sizeof(RepDesc), cudaMemcpyHostToDevice));
@@ -242,6 +245,7 @@ int configure(lgv_ensemble *e) {
   ETRY(build_map(e, e->tma_map, tb));
   ETRY(build_map(e, e->plane_map, pb));
   ETRY(build_map(e, e->slab_map, sb));
+  ETRY(build_map(e, e->run_map, rb));
   if (e->partial) cudaFree(e->partial);
   e->partial = nullptr;
   ECK(cudaMalloc((void **)&e->partial, (size_t)e->plane_map.nblocks * 11 * sizeof(double)));
@@ -383,9 +387,11 @@ int enqueue_step(lgv_ensemble *e, int ev, int inner, int outer, double dt) {
     return LGV_OK;
   };
   auto charge = [&](double d) -> int {
-    for (int pass = 0; pass < 6; ++pass)
-      ECK(lgv::launch_batch_charge(e->dd, e->dyn, e->slab_map.rep, e->slab_map.first, nb_s, e->phase_q, pass, d,
-                                   off, e->idx32, e->stream));
+    for (int ixyz = 0; ixyz < 3; ++ixyz) {
+      ECK(lgv::launch_batch_charge_dir(e->dd, e->dyn, e->run_map.rep, e->run_map.first, e->run_map.nblocks, e->run_smem,
+                                       e->phase_q, ixyz, d, off, e->bytes32, e->stream));
+      e->phase_q ^= 1;
+    }
     off += 7;
     return LGV_OK;
   };
@@ -494,6 +500,11 @@ int lgv_ensemble_create(int nrep, const lgv_params *params, lgv_ensemble **out) 
     }
   }
   e->idx32 = lgv::batch_idx32(e->hd.data(), nrep);
+  e->bytes32 = true;
+  for (const RepDesc &d : e->hd) {
+    e->bytes32 = e->bytes32 && 16 * d.g.V2 <= 0xffffffffLL;
+    e->run_smem = std::max(e->run_smem, lgv::batch_run_smem(d.g.N));
+  }
   if (cudaMalloc((void **)&e->bar, 3 * sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(e->bar, 0, 3 * sizeof(unsigned)) != cudaSuccess)
     return bail(efail(LGV_ERR_NOMEM, "grid barrier"));
@@ -521,6 +532,7 @@ int lgv_ensemble_destroy(lgv_ensemble *e) {
   free_map(e->ideal_map);
   free_map(e->plane_map);
   free_map(e->slab_map);
+  free_map(e->run_map);
   free_map(e->tma_map);
   if (e->gmaps) cudaFree(e->gmaps);
   if (e->dd) cudaFree(e->dd);

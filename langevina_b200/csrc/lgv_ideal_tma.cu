@@ -46,6 +46,8 @@ __global__ void __launch_bounds__(NT, 2)
     batch_ideal_tma_kernel(const RepDesc *__restrict__ d, const CUtensorMap *__restrict__ gmaps,
                            const int *__restrict__ rep, const int *__restrict__ first, int pphi, int pq, double dt,
                            unsigned long long *waits, int wait_limit) {
+  pdl_launch();
+  pdl_wait();
   batch_tma_item(d, gmaps, rep, first, blockIdx.x, pphi, pq, dt, waits, wait_limit);
 }
 
@@ -125,9 +127,8 @@ cudaError_t launch_batch_ideal_tma(const RepDesc *d, const void *gmaps, const in
   cudaError_t e = cudaFuncSetAttribute(batch_ideal_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kSmemBytes);
   if (e != cudaSuccess) return e;
-  batch_ideal_tma_kernel<<<nblocks, NT, kSmemBytes, st>>>(d, reinterpret_cast<const CUtensorMap *>(gmaps), rep, first,
-                                                          phase_phi, phase_q, dt, waits, wait_limit);
-  return cudaGetLastError();
+  return launch_pdl(batch_ideal_tma_kernel, dim3(nblocks), dim3(NT), kSmemBytes, st, d,
+                    reinterpret_cast<const CUtensorMap *>(gmaps), rep, first, phase_phi, phase_q, dt, waits, wait_limit);
 }
 
 }  // namespace lgv

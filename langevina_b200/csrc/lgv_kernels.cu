@@ -893,7 +893,7 @@ __device__ __forceinline__ void charge_link_site(const Fields &f, const Geo &g, 
       ra = ws.next();
       v = v32(lo32(ra));
     }
-    const double q = a.rms * v;
+    const double q = __dmul_rn(a.rms, v);
     const double dS = charge_dS(nA, nB, q, 2.0 * a.inv2chi);
     const bool accept = INJECTED ? dS < 0 || a.acc[ii] < exp(-dS) : charge_accept(dS, hi32(ra));
     const uint8_t fl = dS < 0 ? 1 : accept ? 2 : 0;
@@ -949,7 +949,7 @@ struct ChargeDirArgs {
 // the accept uniform; updates nA and nB.
 __device__ __forceinline__ void charge_link(double &nA, double &nB, uint64_t z, double rms, double invchi) {
   const uint64_t r = mix64(z);
-  const double q = rms * v32(lo32(r));
+  const double q = __dmul_rn(rms, v32(lo32(r)));  // never contracted with the sums below: every kernel gives the same bits
   const bool yes = charge_accept(charge_dS(nA, nB, q, invchi), hi32(r));
   if (yes) {
     nA -= q;
@@ -1791,11 +1791,9 @@ __global__ void __launch_bounds__(256, 2) meas_tile_kernel(Fields f, Geo g, Meas
 // position by G groups of threads (fixed order), then its modes; the block that
 // ends last of an axis's first 11 rows then rotates that axis's modes.
 // done[3]: zero on entry, re-armed.
-__global__ void __launch_bounds__(kFinishThreads) meas_finish_kernel(const double *__restrict__ xp,
-                                                                    const double *__restrict__ yp,
-                                                                    const double *__restrict__ zp, MeasTiles mt,
-                                                                    dft::Plan p, int logP, MeasOut mo,
-                                                                    unsigned *done) {
+__global__ void __launch_bounds__(kFinishThreads) meas_finish_kernel(const double *xp, const double *yp,
+                                                                    const double *zp, MeasTiles mt, dft::Plan p,
+                                                                    int logP, MeasOut mo, unsigned *done) {
   extern __shared__ __align__(16) double2 sm2[];
   __shared__ double part[kFinishThreads];
   __shared__ bool last;
@@ -1901,6 +1899,15 @@ __device__ __forceinline__ Fields rep_fields(const RepDesc &r, int pphi, int pq)
   return f;
 }
 
+// The counter and the clock, which the kernel before this one may have written:
+// volatile, so that the read stays behind pdl_wait.
+__device__ __forceinline__ EnsDyn load_dyn(const EnsDyn *dyn) {
+  EnsDyn y;
+  y.ctr = *(const volatile unsigned long long *)&dyn->ctr;
+  y.t = *(const volatile double *)&dyn->t;
+  return y;
+}
+
 __device__ __forceinline__ double rep_mass(const RepDesc &r, const EnsDyn &dyn) {
   return __dadd_rn(r.mass0, __dmul_rn(r.dmassdt, dyn.t));
 }
@@ -1932,14 +1939,15 @@ __device__ __forceinline__ bool slab_coords(const RepDesc &r, int local, int lan
 // map, lane 0..127 of its 128 threads (a kernel of their own, or half of a
 // CTA of the persistent step).
 template <typename I>
-__device__ __forceinline__ void batch_hb_item(const RepDesc *__restrict__ d, const EnsDyn *__restrict__ dyn,
+__device__ __forceinline__ void batch_hb_item(const RepDesc *__restrict__ d, const EnsDyn *dyn,
                                               const int *__restrict__ rep, const int *__restrict__ first, int blk,
                                               int lane, int phase, int parity, double dt, int ctr_off) {
   const int r = rep[blk];
   const RepDesc &R = d[r];
-  const EnsDyn y = *dyn;
   int m, j, k0;
   if (!slab_coords(R, blk - first[r], lane, m, j, k0)) return;
+  pdl_wait();  // the previous sub-step writes the fields, the clock kernel *dyn
+  const EnsDyn y = load_dyn(dyn);
   HbArgs a{};
   a.rdtg = sqrt(2. * dt * R.gamma);
   a.Lambda2 = 0.5 * (2. * 3. + rep_mass(R, y));
@@ -1956,32 +1964,38 @@ __device__ __forceinline__ void batch_hb_item(const RepDesc *__restrict__ d, con
 }
 
 template <typename I>
-__global__ void __launch_bounds__(128) batch_hb_kernel(const RepDesc *__restrict__ d, const EnsDyn *__restrict__ dyn,
+__global__ void __launch_bounds__(128) batch_hb_kernel(const RepDesc *__restrict__ d, const EnsDyn *dyn,
                                                        const int *__restrict__ rep, const int *__restrict__ first,
                                                        int phase, int parity, double dt, int ctr_off) {
+  pdl_launch();
   batch_hb_item<I>(d, dyn, rep, first, blockIdx.x, threadIdx.x, phase, parity, dt, ctr_off);
 }
 
-template <typename I>
-__device__ __forceinline__ void batch_charge_item(const RepDesc *__restrict__ d, const EnsDyn *__restrict__ dyn,
-                                                  const int *__restrict__ rep, const int *__restrict__ first, int blk,
-                                                  int lane, int phase, int pass, double dt, int ctr_off_order) {
-  const int r = rep[blk];
-  const RepDesc &R = d[r];
-  const EnsDyn y = *dyn;
-  int m, j, k0;
-  if (!slab_coords(R, blk - first[r], lane, m, j, k0)) return;
-  // the replica's pass order (counter mode of ModelGChargeHB::step)
-  const unsigned long long c0 = y.ctr + (unsigned long long)ctr_off_order;
+// The replica's pass order (counter mode of ModelGChargeHB::step): the direction
+// in place ixyz and the first face's A-site parity.
+__device__ __forceinline__ void rep_charge_order(const RepDesc &R, unsigned long long c0, int ixyz, int &dir, int &e0) {
   const uint64_t w = split_word(sub_key(R.key, c0), 0);
   const int pi = (int)((w & 0xffffffffull) % 6ull);
   // lexicographic permutation pi of (0, 1, 2): first element pi / 2, then the
   // remaining two in order (pi even) or swapped (pi odd)
   const int p0 = pi / 2;
   const int lo = (p0 == 0) ? 1 : 0, hi = (p0 == 2) ? 1 : 2;
-  const int ixyz = pass / 2;
-  const int dir = ixyz == 0 ? p0 : (ixyz == 1 ? ((pi & 1) ? hi : lo) : ((pi & 1) ? lo : hi));
-  const int e0 = (int)(w >> 63);
+  dir = ixyz == 0 ? p0 : (ixyz == 1 ? ((pi & 1) ? hi : lo) : ((pi & 1) ? lo : hi));
+  e0 = (int)(w >> 63);
+}
+
+template <typename I>
+__device__ __forceinline__ void batch_charge_item(const RepDesc *__restrict__ d, const EnsDyn *dyn,
+                                                  const int *__restrict__ rep, const int *__restrict__ first, int blk,
+                                                  int lane, int phase, int pass, double dt, int ctr_off_order) {
+  const int r = rep[blk];
+  const RepDesc &R = d[r];
+  const EnsDyn y = load_dyn(dyn);
+  int m, j, k0;
+  if (!slab_coords(R, blk - first[r], lane, m, j, k0)) return;
+  const unsigned long long c0 = y.ctr + (unsigned long long)ctr_off_order;
+  int dir, e0;
+  rep_charge_order(R, c0, pass / 2, dir, e0);
   const int eoA = (pass & 1) ? (e0 ^ 1) : e0;
   ChargeArgs a{};
   a.rms = sqrt(2. * dt * (R.diffusion * R.chi));
@@ -1995,13 +2009,86 @@ __device__ __forceinline__ void batch_charge_item(const RepDesc *__restrict__ d,
     if (k0 + q < R.g.N) charge_link_site<false, false, I>(f, R.g, dir, eoA, a, m, j, k0 + q, mon);
 }
 
-// 32 registers, full occupancy (as charge_pass_kernel)
+// Both faces of the direction in place ixyz of every replica's order, from the
+// charges of buffer `phase` to those of the other one.  Block blk of the run
+// map, whose share of a replica is batch_run_blocks(N): along x a block holds
+// whole rows (all six charges in turn), along y and z runs of kBatchSeg sites of
+// one charge (charge_run).
+constexpr int kBatchSeg = 32;
+
+__device__ __forceinline__ void batch_charge_rows(const Geo &g, int blk, const ChargeDirArgs &a, double *sh) {
+  const int N = g.N, H = g.H, rows = N * N;
+  if (H <= kRunThreads) {  // a pair per thread, as charge_row_kernel
+    const int by = kRunThreads / H, y = (int)threadIdx.x / H, m = (int)threadIdx.x - y * H, row = blk * by + y;
+    if (blk * by >= rows) return;  // the whole block
+    const bool valid = y < by && row < rows;
+    charge_row(g, 0, 6, m, valid ? row : 0, valid, a, sh + y * H, (by + 1) * H);
+    return;
+  }
+  if (blk >= rows) return;
+  double *sA = sh, *sB = sh + H;
+  const int k = blk / N, b = (a.eo[0] ^ (blk - k * N + k)) & 1;
+  const long long ra = (long long)a.eo[0] * g.V2 + (long long)blk * H, rb = (long long)a.eo[1] * g.V2 + (long long)blk * H;
+  pdl_wait();
+  for (int L = 0; L < 6; ++L) {
+    const double *in = a.in + L * a.pitch_in;
+    double *out = a.out + L * a.pitch_out;
+    for (int m = threadIdx.x; m < H; m += kRunThreads) {
+      const int xb = 2 * m + b + 1 == N ? 0 : 2 * m + b + 1;
+      double A = in[ra + m], B = in[rb + (xb >> 1)];
+      charge_link(A, B, a.sk[0] + (6 * ((uint64_t)blk * N + 2 * m + b) + L + 1) * kGolden, a.rms, a.invchi);
+      sA[m] = A;
+      sB[m] = B;
+    }
+    __syncthreads();
+    for (int m = threadIdx.x; m < H; m += kRunThreads) {
+      const int xb = 2 * m + b + 1 == N ? 0 : 2 * m + b + 1, mn = m + 1 == H ? 0 : m + 1;
+      double A = sA[mn], B = sB[m];
+      charge_link(B, A, a.sk[1] + (6 * ((uint64_t)blk * N + xb) + L + 1) * kGolden, a.rms, a.invchi);
+      out[ra + mn] = A;
+      out[rb + (xb >> 1)] = B;
+    }
+    __syncthreads();
+  }
+}
+
 template <typename I>
-__global__ void __launch_bounds__(128, 16) batch_charge_kernel(const RepDesc *__restrict__ d,
-                                                           const EnsDyn *__restrict__ dyn, const int *__restrict__ rep,
-                                                           const int *__restrict__ first, int phase, int pass,
-                                                           double dt, int ctr_off_order) {
-  batch_charge_item<I>(d, dyn, rep, first, blockIdx.x, threadIdx.x, phase, pass, dt, ctr_off_order);
+__global__ void __launch_bounds__(kRunThreads) batch_charge_dir_kernel(const RepDesc *__restrict__ d,
+                                                                       const EnsDyn *dyn,
+                                                                       const int *__restrict__ rep,
+                                                                       const int *__restrict__ first, int phase,
+                                                                       int ixyz, double dt, int ctr_off_order) {
+  extern __shared__ double xs[];
+  pdl_launch();
+  const int r = rep[blockIdx.x];
+  const RepDesc &R = d[r];
+  const int blk = blockIdx.x - first[r], N = R.g.N;
+  pdl_wait();
+  const EnsDyn y = load_dyn(dyn);
+  const unsigned long long c0 = y.ctr + (unsigned long long)ctr_off_order;
+  int dir, e0;
+  rep_charge_order(R, c0, ixyz, dir, e0);
+  ChargeDirArgs a;
+  a.in = R.base[phase] + 4 * R.pstride;
+  a.out = R.base[phase ^ 1] + 4 * R.pstride;
+  a.pitch_in = a.pitch_out = R.pstride;
+  a.rms = sqrt(2. * dt * (R.diffusion * R.chi));
+  a.invchi = 2.0 * (1.0 / (2. * R.chi));
+  a.sk[0] = sub_key(R.key, c0 + 1 + 2 * ixyz);
+  a.sk[1] = sub_key(R.key, c0 + 2 + 2 * ixyz);
+  a.eo[0] = e0;
+  a.eo[1] = e0 ^ 1;
+  if (dir == 0) {
+    batch_charge_rows(R.g, blk, a, xs);
+    return;
+  }
+  const int nrun = (N + kBatchSeg - 1) / kBatchSeg, L = blk % 6, q = blk / 6, run = q % nrun;
+  const int idx = (q / nrun) * kRunThreads + (int)threadIdx.x, o = idx / N, t = idx - o * N;
+  if (o >= N) return;
+  const int s = t >= R.g.H ? 1 : 0, i = 2 * (t - s * R.g.H) + s;
+  const int seg0 = run * kBatchSeg, len = min(kBatchSeg, N - seg0);
+  if (dir == 1) charge_run<1, true, I>(R.g, L, i, o, seg0, len, a);
+  else charge_run<2, true, I>(R.g, L, i, o, seg0, len, a);
 }
 
 // ---- differentiable Euler-Maruyama runs of an ensemble ---------------------
@@ -2163,13 +2250,15 @@ __global__ void __launch_bounds__(128) batch_diff_copy_kernel(const RepDesc *__r
 
 template <typename I>
 __global__ void __launch_bounds__(kSiteThreads, kEmBlocks) batch_em_kernel(const RepDesc *__restrict__ d,
-                                                                const EnsDyn *__restrict__ dyn,
+                                                                const EnsDyn *dyn,
                                                                 const int *__restrict__ rep,
                                                                 const int *__restrict__ first, int phase_in, double dt,
                                                                 int ctr_off) {
+  pdl_launch();
   const int r = rep[blockIdx.x];
   const RepDesc &R = d[r];
-  const EnsDyn y = *dyn;
+  pdl_wait();
+  const EnsDyn y = load_dyn(dyn);
   int parity, m, j, k;
   if (!rep_site(R, blockIdx.x - first[r], parity, m, j, k)) return;
   double acc[4];
@@ -2197,6 +2286,8 @@ __global__ void __launch_bounds__(TX *TY, 2) batch_ideal_kernel(const RepDesc *_
                                                                 const int *__restrict__ rep,
                                                                 const int *__restrict__ first, int pphi, int pq,
                                                                 double dt) {
+  pdl_launch();
+  pdl_wait();
   batch_ideal_item<TX, TY>(d, rep, first, blockIdx.x, pphi, pq, dt);
 }
 
@@ -2328,6 +2419,8 @@ __global__ void ens_set_kernel(EnsDyn *dyn, unsigned long long ctr, double t) {
   dyn->t = t;
 }
 __global__ void ens_advance_kernel(EnsDyn *dyn, unsigned long long dctr, double dt) {
+  pdl_launch();
+  pdl_wait();
   dyn->ctr += dctr;
   dyn->t += dt;
 }
@@ -3056,13 +3149,14 @@ cudaError_t launch_batch_ideal(const RepDesc *d, const int *rep, const int *firs
   if (tile == LGV_TILE_16x16) {
     using T = IdealTile<16, 16>;
     if ((e = allow_smem(batch_ideal_kernel<16, 16>, T::SMEM)) != cudaSuccess) return e;
-    batch_ideal_kernel<16, 16><<<nblocks, 256, T::SMEM, st>>>(d, rep, first, phase_phi, phase_q, dt);
+    return launch_pdl(batch_ideal_kernel<16, 16>, dim3(nblocks), dim3(256), T::SMEM, st, d, rep, first, phase_phi, phase_q,
+                      dt);
   } else {
     using T = IdealTile<32, 8>;
     if ((e = allow_smem(batch_ideal_kernel<32, 8>, T::SMEM)) != cudaSuccess) return e;
-    batch_ideal_kernel<32, 8><<<nblocks, 256, T::SMEM, st>>>(d, rep, first, phase_phi, phase_q, dt);
+    return launch_pdl(batch_ideal_kernel<32, 8>, dim3(nblocks), dim3(256), T::SMEM, st, d, rep, first, phase_phi, phase_q,
+                      dt);
   }
-  return cudaGetLastError();
 }
 
 bool batch_idx32(const RepDesc *hd, int nrep) {
@@ -3073,16 +3167,26 @@ bool batch_idx32(const RepDesc *hd, int nrep) {
 
 cudaError_t launch_batch_hb(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
                             int phase, int parity, double dt, int ctr_off, bool i32, cudaStream_t st) {
-  if (i32) batch_hb_kernel<int><<<nblocks, 128, 0, st>>>(d, dyn, rep, first, phase, parity, dt, ctr_off);
-  else batch_hb_kernel<long long><<<nblocks, 128, 0, st>>>(d, dyn, rep, first, phase, parity, dt, ctr_off);
-  return cudaGetLastError();
+  return launch_pdl(i32 ? batch_hb_kernel<int> : batch_hb_kernel<long long>, dim3(nblocks), dim3(128), 0, st, d, dyn, rep,
+                    first, phase, parity, dt, ctr_off);
 }
 
-cudaError_t launch_batch_charge(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
-                                int phase, int pass, double dt, int ctr_off_order, bool i32, cudaStream_t st) {
-  if (i32) batch_charge_kernel<int><<<nblocks, 128, 0, st>>>(d, dyn, rep, first, phase, pass, dt, ctr_off_order);
-  else batch_charge_kernel<long long><<<nblocks, 128, 0, st>>>(d, dyn, rep, first, phase, pass, dt, ctr_off_order);
-  return cudaGetLastError();
+int batch_run_blocks(int N) {
+  const int H = N / 2, by = H <= kRunThreads ? kRunThreads / H : 1, nrun = (N + kBatchSeg - 1) / kBatchSeg;
+  const long long NN = (long long)N * N;
+  return (int)std::max<long long>((NN + by - 1) / by, 6LL * nrun * ((NN + kRunThreads - 1) / kRunThreads));
+}
+
+size_t batch_run_smem(int N) {
+  const int H = N / 2;
+  return 2 * (size_t)(H <= kRunThreads ? (kRunThreads / H + 1) * H : H) * sizeof(double);
+}
+
+cudaError_t launch_batch_charge_dir(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
+                                    size_t smem, int phase, int ixyz, double dt, int ctr_off_order, bool small,
+                                    cudaStream_t st) {
+  return launch_pdl(small ? batch_charge_dir_kernel<unsigned> : batch_charge_dir_kernel<long long>, dim3(nblocks),
+                    dim3(kRunThreads), smem, st, d, dyn, rep, first, phase, ixyz, dt, ctr_off_order);
 }
 
 int persist_grid(bool i32) {
@@ -3120,9 +3224,8 @@ cudaError_t launch_ens_persistent(const PersistPlan &plan, const PersistPtrs &q,
 
 cudaError_t launch_batch_em(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
                             int phase_in, double dt, int ctr_off, bool i32, cudaStream_t st) {
-  if (i32) batch_em_kernel<int><<<nblocks, kSiteThreads, 0, st>>>(d, dyn, rep, first, phase_in, dt, ctr_off);
-  else batch_em_kernel<long long><<<nblocks, kSiteThreads, 0, st>>>(d, dyn, rep, first, phase_in, dt, ctr_off);
-  return cudaGetLastError();
+  return launch_pdl(i32 ? batch_em_kernel<int> : batch_em_kernel<long long>, dim3(nblocks), dim3(kSiteThreads), 0, st, d,
+                    dyn, rep, first, phase_in, dt, ctr_off);
 }
 
 cudaError_t launch_batch_em_fwd(const RepDesc *d, const int *rep, const int *first, int nblocks, int phase,
@@ -3172,8 +3275,7 @@ cudaError_t launch_ens_set(EnsDyn *dyn, unsigned long long ctr, double t, cudaSt
 }
 
 cudaError_t launch_ens_advance(EnsDyn *dyn, unsigned long long dctr, double dt, cudaStream_t st) {
-  ens_advance_kernel<<<1, 1, 0, st>>>(dyn, dctr, dt);
-  return cudaGetLastError();
+  return launch_pdl(ens_advance_kernel, dim3(1), dim3(1), 0, st, dyn, dctr, dt);
 }
 
 cudaError_t launch_batch_oavg(const RepDesc *d, const int *rep, const int *first, int nblocks, int phase_phi,

@@ -9,7 +9,9 @@
 //
 // Rules the kernels keep: every thread that touches device memory calls
 // pdl_wait first, and no kernel of a chain ends without a block having waited,
-// so that completion of a kernel implies completion of all before it.
+// so that completion of a kernel implies completion of all before it.  What an
+// earlier kernel writes is never read through a const __restrict__ pointer: the
+// compiler may move such a load above the wait.
 // Anything else on the stream (copies, events, kernels launched plainly) is
 // ordered as usual.
 #pragma once
