@@ -360,11 +360,54 @@ __device__ __forceinline__ double ld_phi(const double *p) {
   return *p;
 }
 
-// I: the type of element offsets -- int when the buffer (2 V2 elements) and
-// the lattice's global site count fit in 31 bits (idx32), so that every load
-// address is one wide multiply-add of a component base; long long otherwise.
+// I: the type of the offsets in a component plane -- unsigned, in bytes, when a
+// plane is below 4 GB (idx32: N <= 812), so that an address is one 64-bit base of
+// the component and one 32-bit offset; long long, in elements, otherwise.
 __host__ __forceinline__ bool idx32(const Geo &g) {
-  return 2 * g.V2 <= 0x7fffffffLL && (long long)g.N * g.N * g.Ng <= 0x7fffffffLL;
+  return 16 * g.V2 <= 0xffffffffLL && (long long)g.N * g.N * g.Ng <= 0x7fffffffLL;
+}
+template <typename I>
+struct Unit {
+  static constexpr I of = 1;
+};
+template <>
+struct Unit<unsigned> {
+  static constexpr unsigned of = 8;
+};
+__device__ __forceinline__ const double *at(const double *P, unsigned off) {
+  return (const double *)((const char *)P + off);
+}
+__device__ __forceinline__ double *at(double *P, unsigned off) { return (double *)((char *)P + off); }
+__device__ __forceinline__ const double *at(const double *P, long long off) { return P + off; }
+__device__ __forceinline__ double *at(double *P, long long off) { return P + off; }
+
+// A site and its six neighbours as offsets in a component plane.
+template <typename I>
+struct Nbrs {
+  I own, xp, xm, jp, jm, kp, km;
+};
+template <typename I>
+__device__ __forceinline__ Nbrs<I> nbrs_of(const Geo &g, int parity, int m, int j, int k) {
+  const int N = g.N, s = (parity + j + k) & 1;
+  const I u = Unit<I>::of, H = u * (I)g.H, P = H * (I)N;  // a row, a plane
+  const I half = u * (I)g.V2, row = (I)k * P + (I)j * H, c = (parity ? (I)0 : half) + row + u * (I)m;
+  int xm = m - 1 + s, xp = m + s;
+  if (xm < 0) xm += g.H;
+  if (xp == g.H) xp = 0;
+  Nbrs<I> r;
+  r.own = (parity ? half : (I)0) + row + u * (I)m;
+  r.xp = c + u * (I)(xp - m);
+  r.xm = c + u * (I)(xm - m);
+  r.jp = c + (j + 1 == N ? H - P : H);
+  r.jm = c - (j == 0 ? H - P : H);
+  r.kp = c + (k + 1 == g.Nz ? P - P * (I)g.Nz : P);
+  r.km = c - (k == 0 ? P - P * (I)g.Nz : P);
+  return r;
+}
+template <bool CG = false, typename I = long long>
+__device__ __forceinline__ double nbr_sum(const double *P, const Nbrs<I> &o) {
+  return (ld_phi<CG>(at(P, o.xp)) + ld_phi<CG>(at(P, o.xm))) + (ld_phi<CG>(at(P, o.jp)) + ld_phi<CG>(at(P, o.jm))) +
+         (ld_phi<CG>(at(P, o.kp)) + ld_phi<CG>(at(P, o.km)));
 }
 
 template <typename I>
@@ -379,20 +422,8 @@ __device__ __forceinline__ I nat_index_t(const Geo &g, int i, int j, int k) {
 template <bool INJECTED, bool MON, bool CG = false, typename I = long long, bool GAUSS = false, bool EARLY = false>
 __device__ __forceinline__ void hb_site(const Fields &f, const Geo &g, int parity, const HbArgs &a, int m, int j,
                                         int k, MonLocal &mon) {
-  const int H = g.H, N = g.N;
-  const int s = (parity + j + k) & 1;
-  int xm = m - 1 + s, xp = m + s;
-  if (xm < 0) xm += H;
-  if (xp == H) xp = 0;
-  const I ob = (I)(parity ^ 1) * (I)g.V2;
-  const I row = ((I)k * N + j) * H;
-  const I orow = ob + row;
-  const I ojp = ob + ((I)k * N + wrap_inc(j, N)) * H + m;
-  const I ojm = ob + ((I)k * N + wrap_dec(j, N)) * H + m;
-  const I okp = ob + ((I)wrap_inc(k, g.Nz) * N + j) * H + m;
-  const I okm = ob + ((I)wrap_dec(k, g.Nz) * N + j) * H + m;
-  const I own = (I)parity * (I)g.V2 + row + m;
-  const long long nat = (long long)nat_index_t<I>(g, 2 * m + s, j, k);
+  const Nbrs<I> o = nbrs_of<I>(g, parity, m, j, k);
+  const long long nat = (long long)nat_index_t<I>(g, 2 * m + ((parity + j + k) & 1), j, k);
   HbNoise z;
   if (!INJECTED && EARLY) {
     hb_noise<GAUSS>(a.sk, nat, z);
@@ -401,18 +432,15 @@ __device__ __forceinline__ void hb_site(const Fields &f, const Geo &g, int parit
   double po[4], heff[4];
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
-    const double *P = f.c[l];
-    heff[l] = (ld_phi<CG>(P + (orow + xp)) + ld_phi<CG>(P + (orow + xm))) +
-              (ld_phi<CG>(P + ojp) + ld_phi<CG>(P + ojm)) +
-              (ld_phi<CG>(P + okp) + ld_phi<CG>(P + okm));
-    po[l] = ld_phi<CG>(P + own);
+    heff[l] = nbr_sum<CG>(f.c[l], o);
+    po[l] = ld_phi<CG>(at(f.c[l], o.own));
   }
   if (!INJECTED && !EARLY) hb_noise<GAUSS>(a.sk, nat, z);
   HbDecision d;
   hb_decide<INJECTED>(po, heff, a, nat, global_sites(g), z, d);
   if (d.accept) {
 #pragma unroll
-    for (int l = 0; l < 4; ++l) f.c[l][own] = d.pn[l];
+    for (int l = 0; l < 4; ++l) *at(f.c[l], o.own) = d.pn[l];
   }
   if (MON) mon_count(mon, d);
   if (a.flags) a.flags[nat] = d.flag;
@@ -1114,33 +1142,6 @@ __device__ __forceinline__ bool all_site(const Geo &g, int chunk, int &parity, i
 
 inline dim3 site_grid(const Geo &g) { return dim3((unsigned)(((long long)g.N * g.H + 127) / 128), g.Nz); }
 
-// The six neighbours of a site as offsets in a component plane.
-template <typename I>
-struct Nbrs {
-  I own, xp, xm, jp, jm, kp, km;
-};
-template <typename I>
-__device__ __forceinline__ Nbrs<I> nbrs_of(const Geo &g, int parity, int m, int j, int k) {
-  const int H = g.H, N = g.N, s = (parity + j + k) & 1;
-  int xm = m - 1 + s, xp = m + s;
-  if (xm < 0) xm += H;
-  if (xp == H) xp = 0;
-  const I ob = (I)(parity ^ 1) * (I)g.V2, row = ((I)k * N + j) * H;
-  Nbrs<I> r;
-  r.own = (I)parity * (I)g.V2 + row + m;
-  r.xp = ob + row + xp;
-  r.xm = ob + row + xm;
-  r.jp = ob + ((I)k * N + wrap_inc(j, N)) * H + m;
-  r.jm = ob + ((I)k * N + wrap_dec(j, N)) * H + m;
-  r.kp = ob + ((I)wrap_inc(k, g.Nz) * N + j) * H + m;
-  r.km = ob + ((I)wrap_dec(k, g.Nz) * N + j) * H + m;
-  return r;
-}
-template <typename I>
-__device__ __forceinline__ double nbr_sum(const double *P, const Nbrs<I> &o) {
-  return (P[o.xp] + P[o.xm]) + (P[o.jp] + P[o.jm]) + (P[o.kp] + P[o.km]);
-}
-
 // The four normals of site nat in the sub-step of key sk.
 __device__ __forceinline__ void site_normals(uint64_t sk, long long nat, double (&xi)[4]) {
   Xoro rng = stream_at(sk, (uint64_t)nat);
@@ -1166,14 +1167,14 @@ __device__ __forceinline__ void em_site(const Fields &in, const Fields &out, con
   }
   double c[4];
 #pragma unroll
-  for (int l = 0; l < 4; ++l) c[l] = in.c[l][o.own];
+  for (int l = 0; l < 4; ++l) c[l] = *at(in.c[l], o.own);
   const double p2 = c[0] * c[0] + c[1] * c[1] + c[2] * c[2] + c[3] * c[3];
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
     double fo = -nbr_sum(in.c[l], o) + a.c6 * c[l] + a.lambda * p2 * c[l];
     if (l == 0) fo -= a.H;
     acc[l] = c[l] - a.dtg * fo + a.sq * xi[l];
-    out.c[l][o.own] = acc[l];
+    *at(out.c[l], o.own) = acc[l];
   }
 }
 
@@ -1201,8 +1202,8 @@ __device__ __forceinline__ void em_adjoint_site(const Fields &phi, const Fields 
   double c[4], l[4];
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
-    c[b] = phi.c[b][o.own];
-    l[b] = lin.c[b][o.own];
+    c[b] = *at(phi.c[b], o.own);
+    l[b] = *at(lin.c[b], o.own);
   }
   const double p2 = c[0] * c[0] + c[1] * c[1] + c[2] * c[2] + c[3] * c[3];
   const double dot = c[0] * l[0] + c[1] * l[1] + c[2] * l[2] + c[3] * l[3];
@@ -1211,7 +1212,7 @@ __device__ __forceinline__ void em_adjoint_site(const Fields &phi, const Fields 
   for (int b = 0; b < 4; ++b) {
     const double hf = nbr_sum(phi.c[b], o), nl = nbr_sum(lin.c[b], o);
     const double jl = a.c6 * l[b] + a.lambda * (p2 * l[b] + 2.0 * c[b] * dot) - nl;
-    lout.c[b][o.own] = l[b] - a.dtg * jl + gl(b);
+    *at(lout.c[b], o.own) = l[b] - a.dtg * jl + gl(b);
     double F = -hf + a.c6 * c[b] + a.lambda * p2 * c[b];
     if (b == 0) F -= a.H;
     gg += l[b] * (-a.dt * F + a.cxi * xi[b]);
@@ -2542,17 +2543,17 @@ __global__ void __launch_bounds__(kSiteThreads, 3) ideal_flat_kernel(Fields in, 
   double c[4], S[4], q[6];
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
-    c[l] = P1.c[l][o.own];
+    c[l] = *at(P1.c[l], o.own);
     S[l] = nbr_sum(P1.c[l], o);
   }
 #pragma unroll
-  for (int s = 0; s < 6; ++s) q[s] = in.c[4 + s][o.own];
+  for (int s = 0; s < 6; ++s) q[s] = *at(in.c[4 + s], o.own);
   charge_currents(c, S, a.dt, a.a2, a.H, q);
   rotate_site(c, q, a.dto2chi);
 #pragma unroll
-  for (int l = 0; l < 4; ++l) out.c[l][o.own] = c[l];
+  for (int l = 0; l < 4; ++l) *at(out.c[l], o.own) = c[l];
 #pragma unroll
-  for (int s = 0; s < 6; ++s) out.c[4 + s][o.own] = q[s];
+  for (int s = 0; s < 6; ++s) *at(out.c[4 + s], o.own) = q[s];
 }
 
 __global__ void __launch_bounds__(kSiteThreads, kIdealAdjBlocks) ideal_adj_a_kernel(Fields u, Fields lin, Fields P1, Fields PB, Fields QB,
@@ -2567,23 +2568,23 @@ __global__ void __launch_bounds__(kSiteThreads, kIdealAdjBlocks) ideal_adj_a_ker
     double c[4], q2[6], S[4];
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-      c[l] = P1.c[l][o.own];
+      c[l] = *at(P1.c[l], o.own);
       S[l] = nbr_sum(P1.c[l], o);
     }
 #pragma unroll
-    for (int s = 0; s < 6; ++s) q2[s] = u.c[4 + s][o.own];
+    for (int s = 0; s < 6; ++s) q2[s] = *at(u.c[4 + s], o.own);
     charge_currents(c, S, a.dt, a.a2, a.H, q2);
     double ob[4], pb[4], qb[6];
 #pragma unroll
-    for (int l = 0; l < 4; ++l) ob[l] = lin.c[l][o.own];
+    for (int l = 0; l < 4; ++l) ob[l] = *at(lin.c[l], o.own);
     rotate_site_adj(c, q2, a.k, ob, pb, qb);
 #pragma unroll
-    for (int l = 0; l < 4; ++l) PB.c[l][o.own] = pb[l];
+    for (int l = 0; l < 4; ++l) *at(PB.c[l], o.own) = pb[l];
     double hb = 0;
 #pragma unroll
     for (int s = 0; s < 6; ++s) {
-      const double Q = lin.c[4 + s][o.own] + qb[s];
-      QB.c[s][o.own] = Q;
+      const double Q = *at(lin.c[4 + s], o.own) + qb[s];
+      *at(QB.c[s], o.own) = Q;
       if (s < 3) hb += -a.dt * Q * c[s + 1];
     }
     v[2] = hb;
@@ -2617,9 +2618,9 @@ __global__ void __launch_bounds__(kSiteThreads, kIdealAdjBlocks) ideal_adj_b_ker
   }
   double pb[4], Qc[6];
 #pragma unroll
-  for (int l = 0; l < 4; ++l) pb[l] = PB.c[l][o.own];
+  for (int l = 0; l < 4; ++l) pb[l] = *at(PB.c[l], o.own);
 #pragma unroll
-  for (int s = 0; s < 6; ++s) Qc[s] = QB.c[s][o.own];
+  for (int s = 0; s < 6; ++s) Qc[s] = *at(QB.c[s], o.own);
   const double da = a.dt * a.a2;
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
@@ -2631,14 +2632,14 @@ __global__ void __launch_bounds__(kSiteThreads, kIdealAdjBlocks) ideal_adj_b_ker
   for (int l = 0; l < 3; ++l) pb[l + 1] += -a.dt * a.H * Qc[l];
   double ph[4], q[6], phb[4], qb[6];
 #pragma unroll
-  for (int l = 0; l < 4; ++l) ph[l] = u.c[l][o.own];
+  for (int l = 0; l < 4; ++l) ph[l] = *at(u.c[l], o.own);
 #pragma unroll
-  for (int s = 0; s < 6; ++s) q[s] = u.c[4 + s][o.own];
+  for (int s = 0; s < 6; ++s) q[s] = *at(u.c[4 + s], o.own);
   rotate_site_adj(ph, q, a.k, pb, phb, qb);
 #pragma unroll
-  for (int l = 0; l < 4; ++l) lout.c[l][o.own] = phb[l] + a.gl[l];
+  for (int l = 0; l < 4; ++l) *at(lout.c[l], o.own) = phb[l] + a.gl[l];
 #pragma unroll
-  for (int s = 0; s < 6; ++s) lout.c[4 + s][o.own] = Qc[s] + qb[s];
+  for (int s = 0; s < 6; ++s) *at(lout.c[4 + s], o.own) = Qc[s] + qb[s];
 }
 
 // sums of phi_0..3, a row per block
@@ -2756,8 +2757,8 @@ cudaError_t launch_hb_pass(Fields f, const Geo &g, int parity, const HbArgs &a, 
   return launch_pdl(hb_pass_kernel<I, M, R, T, G>, grid, dim3(128), 0, st, f, g, parity, a)
 #define LGV_HBP_T(I, M, G)                                     \
   if (i32) {                                                   \
-    if (rows) LGV_HBP(I, M, true, int, G);                     \
-    else LGV_HBP(I, M, false, int, G);                         \
+    if (rows) LGV_HBP(I, M, true, unsigned, G);                     \
+    else LGV_HBP(I, M, false, unsigned, G);                         \
   } else if (rows) LGV_HBP(I, M, true, long long, G);          \
   else LGV_HBP(I, M, false, long long, G)
   if (inj) {
@@ -2995,14 +2996,14 @@ cudaError_t launch_em(Fields in, Fields out, int N, const EmArgs &a, cudaStream_
 
 cudaError_t launch_em(Fields in, Fields out, const Geo &g, const EmArgs &a, cudaStream_t st) {
   const bool i32 = idx32(g);
-  const auto kern = a.xi ? (i32 ? em_kernel<true, false, int> : em_kernel<true, false, long long>)
-                         : (i32 ? em_kernel<false, false, int> : em_kernel<false, false, long long>);
+  const auto kern = a.xi ? (i32 ? em_kernel<true, false, unsigned> : em_kernel<true, false, long long>)
+                         : (i32 ? em_kernel<false, false, unsigned> : em_kernel<false, false, long long>);
   return launch_pdl(kern, site_grid(g), dim3(kSiteThreads), 0, st, in, out, g, a, nullptr);
 }
 
 cudaError_t launch_em_sum(Fields in, Fields out, int N, const EmArgs &a, double *partial, cudaStream_t st) {
   const Geo g = make_geo(N);
-  const auto kern = idx32(g) ? em_kernel<false, true, int> : em_kernel<false, true, long long>;
+  const auto kern = idx32(g) ? em_kernel<false, true, unsigned> : em_kernel<false, true, long long>;
   return launch_pdl(kern, site_grid(g), dim3(kSiteThreads), 0, st, in, out, g, a, partial);
 }
 
@@ -3019,7 +3020,7 @@ cudaError_t launch_ideal_flat(Fields in, Fields P1, Fields out, const Geo &g, co
   const cudaError_t e =
       launch_pdl(rot_phi_kernel, dim3(nblocks(V, kThreads)), dim3(kThreads), 0, st, in, P1, V, a.dto2chi);
   if (e != cudaSuccess) return e;
-  return launch_pdl(idx32(g) ? ideal_flat_kernel<int> : ideal_flat_kernel<long long>, site_grid(g), dim3(kSiteThreads), 0,
+  return launch_pdl(idx32(g) ? ideal_flat_kernel<unsigned> : ideal_flat_kernel<long long>, site_grid(g), dim3(kSiteThreads), 0,
                     st, in, P1, out, g, a);
 }
 
@@ -3167,7 +3168,7 @@ bool batch_idx32(const RepDesc *hd, int nrep) {
 
 cudaError_t launch_batch_hb(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
                             int phase, int parity, double dt, int ctr_off, bool i32, cudaStream_t st) {
-  return launch_pdl(i32 ? batch_hb_kernel<int> : batch_hb_kernel<long long>, dim3(nblocks), dim3(128), 0, st, d, dyn, rep,
+  return launch_pdl(i32 ? batch_hb_kernel<unsigned> : batch_hb_kernel<long long>, dim3(nblocks), dim3(128), 0, st, d, dyn, rep,
                     first, phase, parity, dt, ctr_off);
 }
 
@@ -3206,7 +3207,7 @@ int persist_grid(bool i32) {
   c = 0;
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  const void *kern = i32 ? (const void *)ens_persistent_kernel<int> : (const void *)ens_persistent_kernel<long long>;
+  const void *kern = i32 ? (const void *)ens_persistent_kernel<unsigned> : (const void *)ens_persistent_kernel<long long>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPersistSmem) != cudaSuccess)
     return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, kPersistSmem) != cudaSuccess) return 0;
@@ -3217,34 +3218,34 @@ int persist_grid(bool i32) {
 cudaError_t launch_ens_persistent(const PersistPlan &plan, const PersistPtrs &q, bool i32, cudaStream_t st) {
   const int grid = persist_grid(i32);
   if (grid <= 0) return cudaErrorCooperativeLaunchTooLarge;
-  const void *kern = i32 ? (const void *)ens_persistent_kernel<int> : (const void *)ens_persistent_kernel<long long>;
+  const void *kern = i32 ? (const void *)ens_persistent_kernel<unsigned> : (const void *)ens_persistent_kernel<long long>;
   void *args[] = {const_cast<PersistPlan *>(&plan), const_cast<PersistPtrs *>(&q)};
   return cudaLaunchCooperativeKernel(kern, grid, 256, args, kPersistSmem, st);
 }
 
 cudaError_t launch_batch_em(const RepDesc *d, const EnsDyn *dyn, const int *rep, const int *first, int nblocks,
                             int phase_in, double dt, int ctr_off, bool i32, cudaStream_t st) {
-  return launch_pdl(i32 ? batch_em_kernel<int> : batch_em_kernel<long long>, dim3(nblocks), dim3(kSiteThreads), 0, st, d,
+  return launch_pdl(i32 ? batch_em_kernel<unsigned> : batch_em_kernel<long long>, dim3(nblocks), dim3(kSiteThreads), 0, st, d,
                     dyn, rep, first, phase_in, dt, ctr_off);
 }
 
 cudaError_t launch_batch_em_fwd(const RepDesc *d, const int *rep, const int *first, int nblocks, int phase,
                                 unsigned long long ctr, double t, double dt, double *partial, bool i32,
                                 cudaStream_t st) {
-  return launch_pdl(i32 ? batch_em_fwd_kernel<int> : batch_em_fwd_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
+  return launch_pdl(i32 ? batch_em_fwd_kernel<unsigned> : batch_em_fwd_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
                     0, st, d, rep, first, phase, ctr, t, dt, partial);
 }
 
 cudaError_t launch_batch_em_seg(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first, int nblocks,
                                 int m, unsigned long long ctr, double t, double dt, bool i32, cudaStream_t st) {
-  return launch_pdl(i32 ? batch_em_seg_kernel<int> : batch_em_seg_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
+  return launch_pdl(i32 ? batch_em_seg_kernel<unsigned> : batch_em_seg_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
                     0, st, d, dd, rep, first, m, ctr, t, dt);
 }
 
 cudaError_t launch_batch_em_adj(const RepDesc *d, const DiffDesc *dd, const int *rep, const int *first, int nblocks,
                                 int m, int cur, int n, int b, int S, unsigned long long ctr, double t, double dt,
                                 double *partial, bool i32, cudaStream_t st) {
-  return launch_pdl(i32 ? batch_em_adj_kernel<int> : batch_em_adj_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
+  return launch_pdl(i32 ? batch_em_adj_kernel<unsigned> : batch_em_adj_kernel<long long>, dim3(nblocks), dim3(kSiteThreads),
                     0, st, d, dd, rep, first, m, cur, n, b, S, ctr, t, dt, partial);
 }
 
@@ -3315,7 +3316,7 @@ cudaError_t launch_sum_rows(const double *src, int nslot, int nb, double scale, 
 cudaError_t launch_em_adjoint(Fields phi, Fields lam_in, Fields lam_out, int N, const EmAdjArgs &a, double *partial,
                               cudaStream_t st) {
   const Geo g = make_geo(N);
-  return launch_pdl(idx32(g) ? em_adjoint_kernel<int> : em_adjoint_kernel<long long>, site_grid(g), dim3(kSiteThreads), 0,
+  return launch_pdl(idx32(g) ? em_adjoint_kernel<unsigned> : em_adjoint_kernel<long long>, site_grid(g), dim3(kSiteThreads), 0,
                     st, phi, lam_in, lam_out, g, a, partial);
 }
 
