@@ -276,6 +276,17 @@ __device__ __forceinline__ void store_lags(const Val<CPLX> (&acc)[G], const Val<
 }
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+// the double at this block's address p in the shared memory of block `rank` of the cluster
+__device__ __forceinline__ double cluster_ld(const double *p, unsigned rank) {
+  unsigned addr;
+  double v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(addr) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f64 %0, [%1];\n" : "=d"(v) : "r"(addr) : "memory");
+  return v;
+}
 // one value (pair) of a row into shared memory, asynchronously
 template <bool CPLX, bool VEC>
 __device__ __forceinline__ void copy_val(double *dst, const double *src) {
@@ -294,16 +305,17 @@ __device__ __forceinline__ void copy_val(double *dst, const double *src) {
 // from shared memory per G steps for G^2 multiply-adds.  What it replaces read
 // the same values from global memory and waited for them: 14.8 of 16.2 cycles
 // per issue on the load, FP64 pipe a fifth busy.  2000 samples of 1419 complex
-// series, 250 lags: 600 -> 320 us (a complex multiply-add is four fma's, 155 us
-// of FP64 pipe).  Two warps per block copy more per product (424 us), six and
+// series, 250 lags: 600 -> 276 us (a complex multiply-add is four fma's, 155 us
+// of FP64 pipe; 320 us without the time shared by two blocks, when 360 blocks
+// left half the SMs with two and half with three).  Two warps per block copy more per product (424 us), six and
 // eight leave the last wave emptier (374, 437 us).
 constexpr int kCorrChunk = 16;
 
 template <bool CPLX, bool VEC, int G>
 __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *__restrict__ a,
                                                                  const double *__restrict__ b, long long T,
-                                                                 long long ns, long long ld, int ntmax, int conn,
-                                                                 double *__restrict__ out) {
+                                                                 long long Tz, long long ns, long long ld, int ntmax,
+                                                                 int conn, double *__restrict__ out) {
   constexpr int W = CPLX ? 2 : 1, C = kCorrChunk, NW = kCorrLagWarps, L = NW * G;
   constexpr int RB = L + 2 * C;  // ring rows of b: the chunk's C + L - 1, and the C arriving
   static_assert(RB % C == 0 && C % G == 0 && L % G == 0, "otot_kernel: ring");
@@ -314,11 +326,13 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *
   const bool live = s < ns;
   const double *pa = a + (live ? s : 0) * W, *pb = b + (live ? s : 0) * W;
   const long long Ta = T - tb;  // samples of a that any lag of the block uses (tb < ntmax <= T)
+  // this block's share of the time: blockIdx.z of the cluster's blocks takes Tz steps (a multiple of C)
+  const long long tz = blockIdx.z * Tz, te = min(Ta, tz + Tz);
   // This thread copies rows wp, wp + NW, ... of every C rows; `left` rows are
   // left of the n asked for.  Ring rows start at multiples of C and the rings
   // are multiples of C long, so C rows never wrap.
   static_assert(C % NW == 0 && L % C == 0, "otot_kernel: copies");
-  const double *ga = pa + wp * ld, *gb = pb + (tb + wp) * ld;
+  const double *ga = pa + (tz + wp) * ld, *gb = pb + (tb + tz + wp) * ld;
   const long long ldw = NW * ld;
   auto load_rows = [&](const double *&src, double *ring, long long left) {
     double *dst = ring + (wp * 32 + lane) * W;
@@ -333,9 +347,9 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *
     }
     src += C * ld;
   };
-  load_rows(ga, sa, Ta);
+  load_rows(ga, sa, Ta - tz);
 #pragma unroll
-  for (int q = 0; q < C + L; q += C) load_rows(gb, sb + q * 32 * W, Ta - q);
+  for (int q = 0; q < C + L; q += C) load_rows(gb, sb + q * 32 * W, Ta - tz - q);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   Val<CPLX> acc[G];
 #pragma unroll
@@ -354,7 +368,7 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *
     return v;
   };
   int ra = 0, rb = 0;  // ring rows of the chunk's first a and b
-  for (long long t0 = 0; t0 < Ta; t0 += C) {
+  for (long long t0 = tz; t0 < te; t0 += C) {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
     load_rows(ga, sa + (C - ra) * 32 * W, Ta - t0 - C);
@@ -411,6 +425,27 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *
     if (rb >= RB) rb -= RB;
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (gridDim.z > 1) {  // the shares of the cluster's blocks, added by its first in their order
+    __syncthreads();
+    const int tid = wp * 32 + lane;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      sm[(g * W) * 32 * NW + tid] = acc[g].re;
+      if (CPLX) sm[(g * W + 1) * 32 * NW + tid] = acc[g].im;
+    }
+    cluster_sync();
+    if (blockIdx.z == 0) {
+      for (unsigned z = 1; z < gridDim.z; ++z) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          acc[g].re += cluster_ld(sm + (g * W) * 32 * NW + tid, z);
+          if (CPLX) acc[g].im += cluster_ld(sm + (g * W + 1) * 32 * NW + tid, z);
+        }
+      }
+    }
+    cluster_sync();  // the other blocks' shared memory stays until it is read
+    if (blockIdx.z > 0) return;
+  }
   if (!live || tau0 >= ntmax) return;
   Val<CPLX> cc;
   cc.re = cc.im = 0.0;
@@ -517,13 +552,47 @@ int lgv_time_correlator(const double *a, const double *b, int64_t T, int64_t nse
   const dim3 grid((unsigned)gs, (unsigned)gl), block(32, kCorrLagWarps);
   const bool vec = ((uintptr_t)a % 16 == 0) && ((uintptr_t)b % 16 == 0) && ld % 2 == 0;
   cudaStream_t st = (cudaStream_t)stream;
+  // Blocks that share the time of a set of series and lags, a cluster: as many
+  // as make the busiest SM's share smallest, each at the cost of its own first
+  // rows; one or two blocks leave an SM at about 0.55 and 0.8 of its rate
+  // (2000 x 1419 complex, 250 lags: 330 / 276 / 296 us at 1 / 2 / 4 blocks; 4000 x
+  // 363, 300 lags: 307 / 245 / 227 / 222 at 1 / 2 / 4 / 8; 300 x 4000, 60 lags: 56 /
+  // 51 / 62).
+  int Z = 1;
+  if (decim == 1) {
+    const long long n = gs * gl, over = G * kCorrLagWarps + 4 * kCorrChunk;
+    double best = 0;
+    for (int z = 1; z <= 8; z *= 2) {
+      if (z > 1 && T / z < 4 * kCorrChunk) break;
+      const long long k = (n * z + 147) / 148;
+      const double cost = (double)(k * (T / z + over)) / (k == 1 ? 0.55 : k == 2 ? 0.8 : 1.0);
+      if (z == 1 || cost < best) {
+        best = cost;
+        Z = z;
+      }
+    }
+  }
 #define LGV_OTOT(CP, VE, GG)                                                                                          \
   if (decim == 1) {                                                                                                  \
     constexpr size_t smem = otot_smem<CP, GG>();                                                                     \
     if (smem > 48 * 1024 && cudaFuncSetAttribute(otot_kernel<CP, VE, GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                                  (int)smem) != cudaSuccess)                                          \
       return fail(LGV_ERR_CUDA, "lgv_time_correlator: shared memory");                                               \
-    otot_kernel<CP, VE, GG><<<grid, block, smem, st>>>(a, b, T, nseries, ld, ntmax, conn, out);                      \
+    cudaLaunchConfig_t lc{};                                                                                         \
+    lc.gridDim = dim3(grid.x, grid.y, (unsigned)Z);                                                                  \
+    lc.blockDim = block;                                                                                             \
+    lc.dynamicSmemBytes = smem;                                                                                      \
+    lc.stream = st;                                                                                                  \
+    cudaLaunchAttribute at{};                                                                                        \
+    at.id = cudaLaunchAttributeClusterDimension;                                                                     \
+    at.val.clusterDim.x = at.val.clusterDim.y = 1;                                                                   \
+    at.val.clusterDim.z = (unsigned)Z;                                                                               \
+    lc.attrs = &at;                                                                                                  \
+    lc.numAttrs = 1;                                                                                                 \
+    const long long Tz = ((T + Z - 1) / Z + kCorrChunk - 1) / kCorrChunk * kCorrChunk;                               \
+    if (cudaLaunchKernelEx(&lc, otot_kernel<CP, VE, GG>, a, b, (long long)T, Tz, (long long)nseries, (long long)ld,   \
+                           ntmax, conn, out) != cudaSuccess)                                                         \
+      return launched("lgv_time_correlator: launch failed");                                                         \
   } else {                                                                                                           \
     otot_decim_kernel<CP, VE, GG><<<grid, block, 0, st>>>(a, b, T, nseries, ld, ntmax, decim, conn, out);            \
   }

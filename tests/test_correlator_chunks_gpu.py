@@ -65,3 +65,12 @@ def test_samples_past_the_end_do_not_enter(lgv):
     a[T - 3], b[5] = 0.0, np.inf  # enters lags 0 .. 5
     got = call(a, b, nt, 1, False, False, False)
     assert (~np.isfinite(got[:6])).all() and np.isfinite(got[6:]).all()
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("T,ns,ntmax,shift", [(128, 3, 100, False), (130, 1, 5, True), (511, 33, 40, False),
+                                              (513, 2, 512, False), (1000, 70, 333, False), (2049, 5, 17, True)])
+def test_time_shared_by_a_cluster(lgv, cplx, T, ns, ntmax, shift):
+    """Few series: two to eight blocks share the time, with shares that end inside a chunk, hold only the tail
+    that no full chunk covers, or are empty for the largest lags."""
+    test_edges(lgv, cplx, T, ns, ntmax, 1, shift)
