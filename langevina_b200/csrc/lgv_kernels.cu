@@ -1939,6 +1939,28 @@ __device__ __forceinline__ bool slab_coords(const RepDesc &r, int local, int lan
 // Items of the batched heat-bath and charge sub-steps: block blk of the slab
 // map, lane 0..127 of its 128 threads (a kernel of their own, or half of a
 // CTA of the persistent step).
+__device__ __forceinline__ HbArgs rep_hb_args(const RepDesc &R, const EnsDyn &y, double dt, int ctr_off) {
+  HbArgs a{};
+  a.rdtg = sqrt(2. * dt * R.gamma);
+  a.Lambda2 = 0.5 * (2. * 3. + rep_mass(R, y));
+  a.lam4 = R.lambda / 4.;
+  a.H = R.H;
+  a.sk = sub_key(R.key, y.ctr + (unsigned long long)ctr_off);
+  return a;
+}
+
+// The planes of a slab block, one after the other: unrolled (the planes' loads
+// interleaved) the ensemble step measured 4 % slower.
+template <typename I>
+__device__ __forceinline__ void batch_hb_planes(const RepDesc &R, int phase, int parity, const HbArgs &a, int m, int j,
+                                                int k0) {
+  const Fields f = rep_fields(R, phase, phase);
+  MonLocal mon;
+#pragma unroll 1
+  for (int q = 0; q < kBatchPlanes; ++q)
+    if (k0 + q < R.g.N) hb_site<false, false, false, I>(f, R.g, parity, a, m, j, k0 + q, mon);
+}
+
 template <typename I>
 __device__ __forceinline__ void batch_hb_item(const RepDesc *__restrict__ d, const EnsDyn *dyn,
                                               const int *__restrict__ rep, const int *__restrict__ first, int blk,
@@ -1947,21 +1969,7 @@ __device__ __forceinline__ void batch_hb_item(const RepDesc *__restrict__ d, con
   const RepDesc &R = d[r];
   int m, j, k0;
   if (!slab_coords(R, blk - first[r], lane, m, j, k0)) return;
-  pdl_wait();  // the previous sub-step writes the fields, the clock kernel *dyn
-  const EnsDyn y = load_dyn(dyn);
-  HbArgs a{};
-  a.rdtg = sqrt(2. * dt * R.gamma);
-  a.Lambda2 = 0.5 * (2. * 3. + rep_mass(R, y));
-  a.lam4 = R.lambda / 4.;
-  a.H = R.H;
-  a.sk = sub_key(R.key, y.ctr + (unsigned long long)ctr_off);
-  const Fields f = rep_fields(R, phase, phase);
-  MonLocal mon;
-  // one plane after the other: unrolled (the planes' loads interleaved) the
-  // ensemble step measured 4 % slower, at 62 registers against 64 here
-#pragma unroll 1
-  for (int q = 0; q < kBatchPlanes; ++q)
-    if (k0 + q < R.g.N) hb_site<false, false, false, I>(f, R.g, parity, a, m, j, k0 + q, mon);
+  batch_hb_planes<I>(R, phase, parity, rep_hb_args(R, load_dyn(dyn), dt, ctr_off), m, j, k0);
 }
 
 template <typename I>
@@ -1969,7 +1977,15 @@ __global__ void __launch_bounds__(128) batch_hb_kernel(const RepDesc *__restrict
                                                        const int *__restrict__ rep, const int *__restrict__ first,
                                                        int phase, int parity, double dt, int ctr_off) {
   pdl_launch();
-  batch_hb_item<I>(d, dyn, rep, first, blockIdx.x, threadIdx.x, phase, parity, dt, ctr_off);
+  const int r = rep[blockIdx.x];
+  const RepDesc &R = d[r];
+  int m, j, k0;
+  const bool ok = slab_coords(R, blockIdx.x - first[r], threadIdx.x, m, j, k0);
+  pdl_wait();  // the previous sub-step writes the fields, the clock kernel *dyn
+  __shared__ HbArgs sa;  // once per block: a square root and a key
+  if (threadIdx.x == 0) sa = rep_hb_args(R, load_dyn(dyn), dt, ctr_off);
+  __syncthreads();
+  if (ok) batch_hb_planes<I>(R, phase, parity, sa, m, j, k0);
 }
 
 // The replica's pass order (counter mode of ModelGChargeHB::step): the direction
@@ -2065,20 +2081,25 @@ __global__ void __launch_bounds__(kRunThreads) batch_charge_dir_kernel(const Rep
   const RepDesc &R = d[r];
   const int blk = blockIdx.x - first[r], N = R.g.N;
   pdl_wait();
-  const EnsDyn y = load_dyn(dyn);
-  const unsigned long long c0 = y.ctr + (unsigned long long)ctr_off_order;
-  int dir, e0;
-  rep_charge_order(R, c0, ixyz, dir, e0);
-  ChargeDirArgs a;
-  a.in = R.base[phase] + 4 * R.pstride;
-  a.out = R.base[phase ^ 1] + 4 * R.pstride;
-  a.pitch_in = a.pitch_out = R.pstride;
-  a.rms = sqrt(2. * dt * (R.diffusion * R.chi));
-  a.invchi = 2.0 * (1.0 / (2. * R.chi));
-  a.sk[0] = sub_key(R.key, c0 + 1 + 2 * ixyz);
-  a.sk[1] = sub_key(R.key, c0 + 2 + 2 * ixyz);
-  a.eo[0] = e0;
-  a.eo[1] = e0 ^ 1;
+  __shared__ ChargeDirArgs a;  // once per block: the order, keys, a square root and a division
+  __shared__ int s_dir;
+  if (threadIdx.x == 0) {
+    const unsigned long long c0 = load_dyn(dyn).ctr + (unsigned long long)ctr_off_order;
+    int dir, e0;
+    rep_charge_order(R, c0, ixyz, dir, e0);
+    s_dir = dir;
+    a.in = R.base[phase] + 4 * R.pstride;
+    a.out = R.base[phase ^ 1] + 4 * R.pstride;
+    a.pitch_in = a.pitch_out = R.pstride;
+    a.rms = sqrt(2. * dt * (R.diffusion * R.chi));
+    a.invchi = 2.0 * (1.0 / (2. * R.chi));
+    a.sk[0] = sub_key(R.key, c0 + 1 + 2 * ixyz);
+    a.sk[1] = sub_key(R.key, c0 + 2 + 2 * ixyz);
+    a.eo[0] = e0;
+    a.eo[1] = e0 ^ 1;
+  }
+  __syncthreads();
+  const int dir = s_dir;
   if (dir == 0) {
     batch_charge_rows(R.g, blk, a, xs);
     return;
@@ -2128,10 +2149,13 @@ __global__ void __launch_bounds__(kSiteThreads, kEmBlocks) batch_em_fwd_kernel(c
   pdl_launch();
   const int r = rep[blockIdx.x];
   const RepDesc &R = d[r];
+  __shared__ EmArgs sa;  // once per block: a square root and a key
+  if (threadIdx.x == 0) sa = rep_em_args(R, ctr, t, dt);
+  __syncthreads();
   int parity, m, j, k;
   double acc[4] = {0, 0, 0, 0};
   if (rep_site(R, blockIdx.x - first[r], parity, m, j, k))
-    em_site<false, I>(rep_fields(R, phase, phase), rep_fields(R, phase ^ 1, phase ^ 1), R.g, rep_em_args(R, ctr, t, dt),
+    em_site<false, I>(rep_fields(R, phase, phase), rep_fields(R, phase ^ 1, phase ^ 1), R.g, sa,
                       parity, m, j, k, acc);
   block_sum4<kSiteThreads>(acc, partial + (size_t)blockIdx.x * 4);
 }
@@ -2145,12 +2169,15 @@ __global__ void __launch_bounds__(kSiteThreads, kEmBlocks) batch_em_seg_kernel(c
   pdl_launch();
   const int r = rep[blockIdx.x];
   const RepDesc &R = d[r];
+  __shared__ EmArgs sa;  // once per block: a square root and a key
+  if (threadIdx.x == 0) sa = rep_em_args(R, ctr, t, dt);
+  __syncthreads();
   const DiffDesc &D = dd[r];
   int parity, m, j, k;
   if (!rep_site(R, blockIdx.x - first[r], parity, m, j, k)) return;
   double acc[4];
   em_site<false, I>(diff_planes(D.seg, D.V, 4LL * slot), diff_planes(D.seg, D.V, 4LL * (slot + 1)), R.g,
-                    rep_em_args(R, ctr, t, dt), parity, m, j, k, acc);
+                    sa, parity, m, j, k, acc);
 }
 
 // Sums of phi of the lattice buffer `phase`, a row per block.
@@ -2207,20 +2234,25 @@ __global__ void __launch_bounds__(kSiteThreads, kEmAdjBlocks) batch_em_adj_kerne
   const int r = rep[blockIdx.x];
   const RepDesc &R = d[r];
   const DiffDesc &D = dd[r];
-  EmAdjArgs a{};
-  a.c6 = 6.0 + __dadd_rn(R.mass0, __dmul_rn(R.dmassdt, t));
-  a.dtg = dt * R.gamma;
-  a.dt = dt;
-  a.lambda = R.lambda;
-  a.H = R.H;
-  a.cxi = sqrt(2.0 * dt) / (2.0 * sqrt(R.gamma));
-  a.sk = sub_key(R.key, ctr);
+  __shared__ EmAdjArgs sa;  // once per block: square roots, a key, and the divisions of the loss gradient
+  if (threadIdx.x == 0) {
+    sa.c6 = 6.0 + __dadd_rn(R.mass0, __dmul_rn(R.dmassdt, t));
+    sa.dtg = dt * R.gamma;
+    sa.dt = dt;
+    sa.lambda = R.lambda;
+    sa.H = R.H;
+    sa.cxi = sqrt(2.0 * dt) / (2.0 * sqrt(R.gamma));
+    sa.sk = sub_key(R.key, ctr);
+  }
+  // avg and w were complete before the first adjoint launch
+  if (threadIdx.x >= 32 && threadIdx.x < 36) sa.gl[threadIdx.x - 32] = rep_gl(D, n, b, S, threadIdx.x - 32);
+  __syncthreads();
   double v[4] = {0, 0, 0, 0};
   int parity, m, j, k;
   if (rep_site(R, blockIdx.x - first[r], parity, m, j, k))
     em_adjoint_site<I>(diff_planes(D.seg, D.V, 4LL * slot), diff_planes(D.lam, D.V, 4LL * cur),
-                       diff_planes(D.lam, D.V, 4LL * (cur ^ 1)), R.g, a, parity, m, j, k,
-                       [&](int q) { return rep_gl(D, n, b, S, q); }, v);
+                       diff_planes(D.lam, D.V, 4LL * (cur ^ 1)), R.g, sa, parity, m, j, k,
+                       [&](int q) { return sa.gl[q]; }, v);
   block_sum4<kSiteThreads>(v, partial + (size_t)blockIdx.x * 4);
 }
 
@@ -2260,11 +2292,14 @@ __global__ void __launch_bounds__(kSiteThreads, kEmBlocks) batch_em_kernel(const
   const RepDesc &R = d[r];
   pdl_wait();
   const EnsDyn y = load_dyn(dyn);
+  __shared__ EmArgs sa;
+  if (threadIdx.x == 0) sa = rep_em_args(R, y.ctr + (unsigned long long)ctr_off, y.t, dt);
+  __syncthreads();
   int parity, m, j, k;
   if (!rep_site(R, blockIdx.x - first[r], parity, m, j, k)) return;
   double acc[4];
   em_site<false, I>(rep_fields(R, phase_in, phase_in), rep_fields(R, phase_in ^ 1, phase_in ^ 1), R.g,
-                    rep_em_args(R, y.ctr + (unsigned long long)ctr_off, y.t, dt), parity, m, j, k, acc);
+                    sa, parity, m, j, k, acc);
 }
 
 template <int TX, int TY>
