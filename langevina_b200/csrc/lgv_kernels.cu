@@ -2031,15 +2031,20 @@ __device__ __forceinline__ void batch_charge_item(const RepDesc *__restrict__ d,
 // map, whose share of a replica is batch_run_blocks(N): along x a block holds
 // whole rows (all six charges in turn), along y and z runs of kBatchSeg sites of
 // one charge (charge_run).
-constexpr int kBatchSeg = 32;
+// kBatchRowSets sets of rows per block: both forms then need about as many
+// blocks (a charge step of 52 replicas, 20^3 to 64^3: 240 us at one set and 222
+// at two with runs of 32, 236 with runs of 16, 237 at four sets).
+constexpr int kBatchSeg = 32, kBatchRowSets = 2;
 
 __device__ __forceinline__ void batch_charge_rows(const Geo &g, int blk, const ChargeDirArgs &a, double *sh) {
   const int N = g.N, H = g.H, rows = N * N;
   if (H <= kRunThreads) {  // a pair per thread, as charge_row_kernel
-    const int by = kRunThreads / H, y = (int)threadIdx.x / H, m = (int)threadIdx.x - y * H, row = blk * by + y;
-    if (blk * by >= rows) return;  // the whole block
-    const bool valid = y < by && row < rows;
-    charge_row(g, 0, 6, m, valid ? row : 0, valid, a, sh + y * H, (by + 1) * H);
+    const int by = kRunThreads / H, y = (int)threadIdx.x / H, m = (int)threadIdx.x - y * H;
+    for (int r0 = blk * kBatchRowSets * by; r0 < min(rows, (blk + 1) * kBatchRowSets * by); r0 += by) {
+      const bool valid = y < by && r0 + y < rows;
+      charge_row(g, 0, 6, m, valid ? r0 + y : 0, valid, a, sh + y * H, (by + 1) * H);
+      __syncthreads();
+    }
     return;
   }
   if (blk >= rows) return;
@@ -3208,7 +3213,7 @@ cudaError_t launch_batch_hb(const RepDesc *d, const EnsDyn *dyn, const int *rep,
 }
 
 int batch_run_blocks(int N) {
-  const int H = N / 2, by = H <= kRunThreads ? kRunThreads / H : 1, nrun = (N + kBatchSeg - 1) / kBatchSeg;
+  const int H = N / 2, by = H <= kRunThreads ? kBatchRowSets * (kRunThreads / H) : 1, nrun = (N + kBatchSeg - 1) / kBatchSeg;
   const long long NN = (long long)N * N;
   return (int)std::max<long long>((NN + by - 1) / by, 6LL * nrun * ((NN + kRunThreads - 1) / kRunThreads));
 }
