@@ -45,14 +45,16 @@ int launched(const char *where) {
 // A block takes R rows (a power of two; lanes are rows, so a twiddle is read
 // once for the whole warp and the row strides, odd, keep the lanes on distinct
 // banks).  Rows come in and modes leave through shared memory in whole lines;
-// kB columns (or k2's) per thread share each row value.  STAGE = false (N above
-// kX2kStageMaxN, one row per block): the table of N twiddles takes the room of
-// the row, which is read and written in global memory.  33 792 rows of 256: 84
-// us (139 MB in and out take 21), against 653 us for the direct sums, which
-// shared-memory bandwidth bound; now the phases between barriers do (36 % of
-// the warps resident, 46 % issue).  Measured at 16 rows and three blocks per
-// SM; 8 rows and four: 138 us, 16 rows and two: 90 us.
-constexpr int kX2kThreads = 256, kX2kB1 = 5, kX2kB2 = 5, kX2kStageMaxN = 4096;
+// kX2kB1 columns, then kX2kB2 k2's, per thread share each row value: more read
+// fewer values, fewer leave less of the last threads' work to waste.  STAGE =
+// false (N above kX2kStageMaxN, one row per block): the table of N twiddles takes
+// the room of the row, which is read and written in global memory.  33 792 rows
+// of 256: 70 us (139 MB in and out take 21), against 653 us for the direct sums,
+// which shared-memory bandwidth bound; now the phases between barriers do.  The
+// choice: 3 columns and 2 k2's 70 us, 3 and 3 72, 2 and 2 78, 5 and 5 84, 4 and 4
+// 92 (rows of 90, 500, 24 and 166: the first is the fastest too); at 5 and 5, 8
+// rows and four blocks per SM 138 us, 16 rows and two blocks 90.
+constexpr int kX2kThreads = 256, kX2kB1 = 3, kX2kB2 = 2, kX2kStageMaxN = 4096;
 constexpr int kX2kLogRows = 4;  // 16 rows per block where they fit
 constexpr int kX2kBlocks = 3;   // blocks per SM
 
