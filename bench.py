@@ -39,9 +39,11 @@ sys.path.insert(0, REPO)
 ALG_BYTES = {  # algorithmic bytes per site, per launch (each input read once, each output written once)
     "ideal": 160.0,    # 10 doubles in, 10 out
     "phi_hb": 32.0,    # one parity pass: 64 B/site per full sweep, half the sites per launch
-    "charge": 96.0,    # one (direction, parity) face: 6 charges in and out for every site
+    "charge": 48.0,    # one (direction, parity) face: both faces of a direction share one launch, which takes the
+                       # 6 charges in and out once (96 B per site)
     "em": 64.0,
 }
+# bytes of a step with every sub-step as the reference sequences it, six charge faces at 96 B each
 STEP_BYTES = {"PV2HBSplit23": 1440.0, "PV2HBSplit11": 800.0}
 NOMINAL_HBM_GBS = 7700.0  # B200 HBM3e, HGX figure
 KCLASS = {"ideal": 0, "phi_hb": 1, "charge": 2, "em": 3, "measure": 4}
@@ -805,10 +807,12 @@ def run_ours(a):
         L.check(lib.lgv_timing_read(h, c, C.byref(tot), C.byref(n)), "timing_read")
         kern[k] = (tot.value, n.value)
     L.check(lib.lgv_timing_enable(h, 0), "timing off")
-    # launches of the timed region: the split pass's count per step (the
-    # measurement every MEASURE_EVERY steps is 5 launches)
-    per_step = sum(n for k, (tot, n) in kern.items() if k != "measure") / split_steps
-    launches = int(round(per_step * a.steps)) + 5 * n_meas
+    # launches of the timed region: the split pass's count per step, where a
+    # charge launch counts as two faces and an ideal step on a small lattice is
+    # two launches, and the measurement's two (five beyond N = 512)
+    per = {"charge": 0.5, "ideal": 2.0 if (N < 128 if N % 32 == 0 else N <= 200) else 1.0, "measure": 0.0}
+    per_step = sum(n * per.get(k, 1.0) for k, (tot, n) in kern.items()) / split_steps
+    launches = int(round(per_step * a.steps)) + (2 if N <= 512 else 5) * n_meas
 
     value = whole_job_rate(V * a.steps, world, ms / 1e3)
     peak, peak_kind = peaks()

@@ -212,8 +212,10 @@ int lgv_synchronize(lgv_handle *h);
  * synchronizes, adds the elapsed times of all pairs recorded so far and
  * returns the running total and launch count of one class.  Enabling (or
  * re-enabling) resets the totals.  A "launch" of LGV_KCLASS_PHI_HB is one
- * checkerboard parity pass; of LGV_KCLASS_CHARGE one (direction, parity) face;
- * of LGV_KCLASS_MEASURE one full measurement (five small kernels). */
+ * checkerboard parity pass; of LGV_KCLASS_CHARGE one (direction, parity) face
+ * (two per kernel where a kernel updates both faces of a direction); of
+ * LGV_KCLASS_MEASURE one full measurement (two kernels up to N = 512, five
+ * beyond); of LGV_KCLASS_IDEAL one ideal step (two kernels on small lattices). */
 #define LGV_KCLASS_IDEAL 0
 #define LGV_KCLASS_PHI_HB 1
 #define LGV_KCLASS_CHARGE 2

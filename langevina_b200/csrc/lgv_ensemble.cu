@@ -195,7 +195,7 @@ int build_map(lgv_ensemble *e, BlockMap &m, const std::vector<int> &blocks_per_r
 // Replicas with N divisible by 32 take the TMA ideal kernel: encode the
 // tensor maps of their component planes for every (phi buffer, charge
 // buffer) pairing once, since the buffers never move.  LGV_IDEAL_TMA=0 keeps
-// every replica on the cp.async kernel, as for single lattices.
+// every replica on the cp.async kernel.
 int tensor_maps(lgv_ensemble *e) {
   const char *env = std::getenv("LGV_IDEAL_TMA");
   const bool off = env && env[0] == '0';

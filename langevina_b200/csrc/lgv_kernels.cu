@@ -5,18 +5,25 @@
 //   hb_pass_kernel      EulerLangevinHB::step, one checkerboard parity per
 //                       launch (Stepper.cxx:287-389)
 //   hb_sweep_kernel     the same, both parities in one z-marching launch (opt-in)
-//   charge_pass_kernel  ModelGChargeHB::step, one (direction, parity) face
-//                       (Stepper.cxx:471-518, modelg_update_charge_pair :419-441)
-//   charge_row_kernel,  both faces of one direction per launch: x rows per
-//   charge_run_kernel   block; y and z runs of sites per thread
+//   charge_row_kernel,  ModelGChargeHB::step, both faces of one direction per
+//   charge_run_kernel   launch (Stepper.cxx:471-518, modelg_update_charge_pair
+//                       :419-441): x rows per block; y and z runs of sites per
+//                       thread
+//   charge_pass_kernel  the same, one face per launch (slabs, decision flags,
+//                       injected noise, LGV_CHARGE_FUSED=0)
 //   ideal_kernel        IdealPV2::step_no_reject fused: half rotation, charge
 //                       advection stencil, half rotation (Stepper.cxx:68-202);
 //                       the TMA-staged ideal_tma_kernel (lgv_ideal_tma.cu)
-//                       replaces it for N divisible by 32
+//                       replaces it for N divisible by 32, and rot_phi_kernel
+//                       and ideal_flat_kernel, one thread per site, on small
+//                       lattices (ideal_flat)
 //   em_kernel           Euler-Maruyama Model A step (action of Stepper.cxx:354-355)
 //   energy_*            IdealPV2::computeEnergy (Stepper.cxx:204-268)
 //   meas_*              Measurer::computeSliceAverage / ...Phase /
-//                       computeDerivedObs (measurer.cxx:10-317)
+//                       computeDerivedObs (measurer.cxx:10-317): one pass over
+//                       the state and one kernel for the rest up to
+//                       kMeasTileMaxN, five kernels beyond
+//   sum_rows_kernel     adds the block rows of site sums in a fixed order
 //   batch_*             the same steps for every replica of an ensemble in one
 //                       launch (no counterpart: the reference runs one lattice)
 //   em_adjoint_kernel, rot_phi_kernel, ideal_adj_a/b_kernel, batch_em_*
@@ -264,10 +271,6 @@ __global__ void charge_sub_kernel(Fields f, long long V, const double *mean) {
 __device__ __forceinline__ void cp_async8(double *smem, const double *gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async16(double *smem, const double *gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
