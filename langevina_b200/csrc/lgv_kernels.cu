@@ -2036,7 +2036,9 @@ __device__ __forceinline__ void batch_charge_item(const RepDesc *__restrict__ d,
 // one charge (charge_run).
 // kBatchRowSets sets of rows per block: both forms then need about as many
 // blocks (a charge step of 52 replicas, 20^3 to 64^3: 240 us at one set and 222
-// at two with runs of 32, 236 with runs of 16, 237 at four sets).
+// at two with runs of 32, 236 with runs of 16, 237 at four sets).  Twelve blocks
+// per SM (40 registers, 40 bytes of spill): 222 -> 207 us, since the step waits
+// on its replicas' memory; 48 registers 213, 32 registers 219.
 constexpr int kBatchSeg = 32, kBatchRowSets = 2;
 
 __device__ __forceinline__ void batch_charge_rows(const Geo &g, int blk, const ChargeDirArgs &a, double *sh) {
@@ -2078,7 +2080,7 @@ __device__ __forceinline__ void batch_charge_rows(const Geo &g, int blk, const C
 }
 
 template <typename I>
-__global__ void __launch_bounds__(kRunThreads) batch_charge_dir_kernel(const RepDesc *__restrict__ d,
+__global__ void __launch_bounds__(kRunThreads, 12) batch_charge_dir_kernel(const RepDesc *__restrict__ d,
                                                                        const EnsDyn *dyn,
                                                                        const int *__restrict__ rep,
                                                                        const int *__restrict__ first, int phase,
