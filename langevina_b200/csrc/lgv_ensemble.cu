@@ -78,7 +78,7 @@ struct lgv_ensemble {
   cudaStream_t own = nullptr, stream = nullptr;
   int phase_phi = 0, phase_q = 0;
   unsigned long long ctr = 0;
-  int tile = LGV_TILE_32x8, zchunk = 16, order = LGV_PACK_GIVEN;
+  int tile = LGV_TILE_32x8, zchunk = 16, order = LGV_PACK_GIVEN;  // of the ideal step (choose_tuning)
   bool graphs = true;
   std::map<std::tuple<int, int, int, double, int, int>, cudaGraphExec_t> cache;
   // bounded device waits of this ensemble's TMA ideal launches that gave up,
@@ -221,6 +221,44 @@ int tensor_maps(lgv_ensemble *e) {
   return LGV_OK;
 }
 
+// Tile and z-chunk of the ideal step until the caller chooses (lgv_ensemble_tune
+// or _autotune).  Tile: the one that covers the replicas without a tensor map
+// with fewer columns (an ideal step of 16 replicas of 48^3 110 us at 32 x 8, 94
+// at 16 x 16, which divides 48; of 56^3 133 and 150).  Chunk: a block of n planes
+// marches n + 3, and two blocks per SM are resident, so the step takes about the
+// longer of one block's march and the sum of all marches over 296: the longest of
+// 16, 8 and 4 that makes this least (at 16, 8 and 4: 32 of 24^3 41, 30 and 34 us;
+// two of 48^3 37, 22 and 19; 16 of 48^3 94, 96 and 106; 48 of 20^3 35, 46 and 42).
+// Before, every ensemble had 32 x 8 and 16: 51, 37, 110 and 51 us.
+void choose_tuning(lgv_ensemble *e) {
+  const int tiles[2] = {LGV_TILE_32x8, LGV_TILE_16x16}, zcs[3] = {16, 8, 4};
+  long long cols[2] = {0, 0};
+  for (int t = 0; t < 2; ++t)
+    for (int r = 0; r < e->R; ++r) {
+      int tx = 0, ty = 0;
+      lgv::ideal_tile_dims(tiles[t], &tx, &ty);
+      const long long N = e->hd[r].g.N;
+      if (!e->tma_ok[r]) cols[t] += N * ((N + tx - 1) / tx * tx) * ((N + ty - 1) / ty * ty);
+    }
+  e->tile = tiles[cols[1] < cols[0]];
+  int tx = 0, ty = 0;
+  lgv::ideal_tile_dims(e->tile, &tx, &ty);
+  double best = 0;
+  for (int zc : zcs) {
+    long long sum = 0, longest = 0;
+    for (int r = 0; r < e->R; ++r) {
+      const int N = e->hd[r].g.N, nz = (N + zc - 1) / zc, march = (N + nz - 1) / nz + 3;
+      sum += (long long)(e->tma_ok[r] ? lgv::batch_tma_blocks(N, zc) : (N + tx - 1) / tx * ((N + ty - 1) / ty) * nz) * march;
+      longest = std::max<long long>(longest, march);
+    }
+    const double t = std::max((double)longest, sum / 296.0);
+    if (best == 0 || t < best) {
+      best = t;
+      e->zchunk = zc;
+    }
+  }
+}
+
 // (Re)derive the per-replica launch geometry for the current tuning and
 // upload the descriptors and block maps.
 int configure(lgv_ensemble *e) {
@@ -233,8 +271,8 @@ int configure(lgv_ensemble *e) {
     d.nchunk = (int)(((long long)N * d.g.H + 127) / 128);
     d.igx = (N + tx - 1) / tx;
     d.igy = (N + ty - 1) / ty;
-    d.izc = std::min(e->zchunk, N);
-    d.igz = (N + d.izc - 1) / d.izc;
+    d.igz = (N + std::min(e->zchunk, N) - 1) / std::min(e->zchunk, N);
+    d.izc = (N + d.igz - 1) / d.igz;  // as many chunks, evenly long
     ib[r] = e->tma_ok[r] ? 0 : d.igx * d.igy * d.igz;
     tb[r] = e->tma_ok[r] ? lgv::batch_tma_blocks(N, d.izc) : 0;
     pb[r] = d.nchunk * N;
@@ -532,6 +570,7 @@ int lgv_ensemble_create(int nrep, const lgv_params *params, lgv_ensemble **out) 
       cudaMalloc((void **)&e->oavg, (size_t)nrep * 11 * sizeof(double)) != cudaSuccess)
     return bail(efail(LGV_ERR_NOMEM, "ensemble tables"));
   if ((rc = tensor_maps(e)) != LGV_OK) return bail(rc);
+  choose_tuning(e);
   if ((rc = configure(e)) != LGV_OK) return bail(rc);
   if (lgv::launch_ens_set(e->dyn, 0, 0.0, e->stream) != cudaSuccess || cudaStreamSynchronize(e->stream) != cudaSuccess)
     return bail(efail(LGV_ERR_CUDA, "ensemble init"));
