@@ -4,6 +4,7 @@
 // Kernel map (reference loop each one replaces):
 //   hb_pass_kernel      EulerLangevinHB::step, one checkerboard parity per
 //                       launch (Stepper.cxx:287-389)
+//   hb_pass_small_kernel  the same compiled for small lattices
 //   hb_sweep_kernel     the same, both parities in one z-marching launch (opt-in)
 //   charge_row_kernel,  ModelGChargeHB::step, both faces of one direction per
 //   charge_run_kernel   launch (Stepper.cxx:471-518, modelg_update_charge_pair
@@ -478,7 +479,7 @@ __host__ __forceinline__ dim3 pass_grid(const Geo &g, bool rows) {
 // sweep of two passes: 64^3 12.3 us launched plainly, 10.0 with the wait first,
 // 9.1 with the noise first; 256^3 342 with the wait first, 329).
 template <bool INJECTED, bool MON, bool ROWS, typename I, bool GAUSS>
-__global__ void __launch_bounds__(128) hb_pass_kernel(Fields f, Geo g, int parity, HbArgs a) {
+__device__ __forceinline__ void hb_pass(const Fields &f, const Geo &g, int parity, const HbArgs &a) {
   pdl_launch();
   if (INJECTED) pdl_wait();
   int m, j, k;
@@ -486,6 +487,25 @@ __global__ void __launch_bounds__(128) hb_pass_kernel(Fields f, Geo g, int parit
   if (pass_site<ROWS>(g, m, j, k))
     hb_site<INJECTED, MON, false, I, GAUSS, true>(f, g, parity, a, m, j, k, mon);
   if (MON) mon_flush(mon, a.mon);
+}
+
+template <bool INJECTED, bool MON, bool ROWS, typename I, bool GAUSS>
+__global__ void __launch_bounds__(128) hb_pass_kernel(Fields f, Geo g, int parity, HbArgs a) {
+  hb_pass<INJECTED, MON, ROWS, I, GAUSS>(f, g, parity, a);
+}
+// The same compiled for few resident blocks: on a lattice that is over in a few
+// waves a pass is one chain of latencies, and the registers (76 against 40, with
+// Gaussian proposals 84 against 58) let a site's 28 loads be in flight together.
+// A sweep of 32^3 6.2 -> 4.8 us, 48^3 9.2 -> 5.7, 64^3 10.0 -> 7.6, 80^3 12.4 ->
+// 11.2, 96^3 16.6 -> 16.0, 110^3 23.7 -> 22.9; 128^3 33 either way, and beyond
+// that occupancy wins (256^3 329 against 334-342).  Gaussian: 32^3 7.0 -> 4.7,
+// 48^3 7.7 -> 4.9, but 64^3 8.6 -> 9.3.
+template <bool GAUSS>
+__global__ void __launch_bounds__(128, 1) hb_pass_small_kernel(Fields f, Geo g, int parity, HbArgs a) {
+  hb_pass<false, false, false, unsigned, GAUSS>(f, g, parity, a);
+}
+__host__ __forceinline__ bool hb_small(const Geo &g, bool gauss) {
+  return g.V2 <= 148LL * (gauss ? 512 : 3 * 2048);  // N up to 52, 122
 }
 
 // ----------------------------------------------------------------------------
@@ -2798,12 +2818,15 @@ cudaError_t launch_hb_pass(Fields f, const Geo &g, int parity, const HbArgs &a, 
   const bool rows = g.H % 128 == 0;
   const dim3 grid = pass_grid(g, rows);
   const bool i32 = idx32(g);
+  if (!inj && !mon && !rows && hb_small(g, gauss))  // 32-bit offsets hold
+    return launch_pdl(gauss ? hb_pass_small_kernel<true> : hb_pass_small_kernel<false>, grid, dim3(128), 0, st, f, g, parity,
+                      a);
 #define LGV_HBP(I, M, R, T, G) \
   return launch_pdl(hb_pass_kernel<I, M, R, T, G>, grid, dim3(128), 0, st, f, g, parity, a)
 #define LGV_HBP_T(I, M, G)                                     \
   if (i32) {                                                   \
-    if (rows) LGV_HBP(I, M, true, unsigned, G);                     \
-    else LGV_HBP(I, M, false, unsigned, G);                         \
+    if (rows) LGV_HBP(I, M, true, unsigned, G);                \
+    else LGV_HBP(I, M, false, unsigned, G);                    \
   } else if (rows) LGV_HBP(I, M, true, long long, G);          \
   else LGV_HBP(I, M, false, long long, G)
   if (inj) {
