@@ -291,7 +291,9 @@ int lgv_ensemble_step(lgv_ensemble *e, int evolver, int inner, int outer, double
 /* volume averages of the 11 OAverage observables, [nrep][11] */
 int lgv_ensemble_oaverage(lgv_ensemble *e, double *host_out);
 int lgv_ensemble_oaverage_device(lgv_ensemble *e, double *dev_out);
-/* explicit tuning: ideal tile (LGV_TILE_*), its z-chunk, packing (LGV_PACK_*) */
+/* explicit tuning: ideal tile (LGV_TILE_*), its z-chunk (planes per block at
+ * most), packing (LGV_PACK_*); until then tile and chunk follow from the
+ * replicas' sizes */
 int lgv_ensemble_tune(lgv_ensemble *e, int tile, int zchunk, int order);
 /* time every (tile, z-chunk in {8,16,32}, packing) candidate over `steps`
  * steps on a copy of the state (state and counter restored), keep the
