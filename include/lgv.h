@@ -292,12 +292,13 @@ int lgv_ensemble_step(lgv_ensemble *e, int evolver, int inner, int outer, double
 int lgv_ensemble_oaverage(lgv_ensemble *e, double *host_out);
 int lgv_ensemble_oaverage_device(lgv_ensemble *e, double *dev_out);
 /* explicit tuning: ideal tile (LGV_TILE_*), its z-chunk (planes per block at
- * most), packing (LGV_PACK_*); until then tile and chunk follow from the
- * replicas' sizes */
+ * most; 8 is cut to 4 where blocks of 8 leave the device idle), packing
+ * (LGV_PACK_*); until then tile and chunk follow from the replicas' sizes */
 int lgv_ensemble_tune(lgv_ensemble *e, int tile, int zchunk, int order);
-/* time every (tile, z-chunk in {8,16,32}, packing) candidate over `steps`
- * steps on a copy of the state (state and counter restored), keep the
- * fastest; choice[3] = (tile, zchunk, order), *ms_per_step its time */
+/* time the choice in use and every (tile, z-chunk in {8,16,32}, packing)
+ * candidate over `steps` steps on a copy of the state (state and counter
+ * restored), keep the fastest; choice[3] = (tile, zchunk, order),
+ * *ms_per_step its time */
 int lgv_ensemble_autotune(lgv_ensemble *e, int evolver, int inner, int outer, double dt, int steps, int *choice,
                           double *ms_per_step);
 /* CUDA-graph replay of lgv_ensemble_step (on by default): two steps are

@@ -221,17 +221,38 @@ int tensor_maps(lgv_ensemble *e) {
   return LGV_OK;
 }
 
+// Blocks of a chunk of n planes march n + 3, and two blocks per SM are resident,
+// so an ideal step takes about the longer of one block's march and the sum of
+// all marches over 296: that number for chunks of at most zc planes.
+double march_cost(const lgv_ensemble *e, int zc) {
+  int tx = 0, ty = 0;
+  lgv::ideal_tile_dims(e->tile, &tx, &ty);
+  long long sum = 0, longest = 0;
+  for (int r = 0; r < e->R; ++r) {
+    const int N = e->hd[r].g.N, nz = (N + zc - 1) / zc, march = (N + nz - 1) / nz + 3;
+    sum += (long long)(e->tma_ok[r] ? lgv::batch_tma_blocks(N, zc) : (N + tx - 1) / tx * ((N + ty - 1) / ty) * nz) * march;
+    longest = std::max<long long>(longest, march);
+  }
+  return std::max((double)longest, sum / 296.0);
+}
+
+// The chunk that a choice of `zchunk` planes at most means: 8 is cut to 4 where
+// that is the shorter march, so that the choices the autotuner tries (8, 16, 32)
+// hold the one of creation (two of 48^3 22 us at 8 and 19 at 4; 32 of 24^3 30 and
+// 34, where the march says 8 too).
+int chunk_planes(const lgv_ensemble *e) {
+  return e->zchunk == 8 && march_cost(e, 4) < march_cost(e, 8) ? 4 : e->zchunk;
+}
+
 // Tile and z-chunk of the ideal step until the caller chooses (lgv_ensemble_tune
 // or _autotune).  Tile: the one that covers the replicas without a tensor map
 // with fewer columns (an ideal step of 16 replicas of 48^3 110 us at 32 x 8, 94
-// at 16 x 16, which divides 48; of 56^3 133 and 150).  Chunk: a block of n planes
-// marches n + 3, and two blocks per SM are resident, so the step takes about the
-// longer of one block's march and the sum of all marches over 296: the longest of
-// 16, 8 and 4 that makes this least (at 16, 8 and 4: 32 of 24^3 41, 30 and 34 us;
+// at 16 x 16, which divides 48; of 56^3 133 and 150).  Chunk: the longest of 16, 8
+// and 4 with the shortest march (at 16, 8 and 4: 32 of 24^3 41, 30 and 34 us;
 // two of 48^3 37, 22 and 19; 16 of 48^3 94, 96 and 106; 48 of 20^3 35, 46 and 42).
 // Before, every ensemble had 32 x 8 and 16: 51, 37, 110 and 51 us.
 void choose_tuning(lgv_ensemble *e) {
-  const int tiles[2] = {LGV_TILE_32x8, LGV_TILE_16x16}, zcs[3] = {16, 8, 4};
+  const int tiles[2] = {LGV_TILE_32x8, LGV_TILE_16x16};
   long long cols[2] = {0, 0};
   for (int t = 0; t < 2; ++t)
     for (int r = 0; r < e->R; ++r) {
@@ -241,22 +262,7 @@ void choose_tuning(lgv_ensemble *e) {
       if (!e->tma_ok[r]) cols[t] += N * ((N + tx - 1) / tx * tx) * ((N + ty - 1) / ty * ty);
     }
   e->tile = tiles[cols[1] < cols[0]];
-  int tx = 0, ty = 0;
-  lgv::ideal_tile_dims(e->tile, &tx, &ty);
-  double best = 0;
-  for (int zc : zcs) {
-    long long sum = 0, longest = 0;
-    for (int r = 0; r < e->R; ++r) {
-      const int N = e->hd[r].g.N, nz = (N + zc - 1) / zc, march = (N + nz - 1) / nz + 3;
-      sum += (long long)(e->tma_ok[r] ? lgv::batch_tma_blocks(N, zc) : (N + tx - 1) / tx * ((N + ty - 1) / ty) * nz) * march;
-      longest = std::max<long long>(longest, march);
-    }
-    const double t = std::max((double)longest, sum / 296.0);
-    if (best == 0 || t < best) {
-      best = t;
-      e->zchunk = zc;
-    }
-  }
+  e->zchunk = std::min(march_cost(e, 8), march_cost(e, 4)) < march_cost(e, 16) ? 8 : 16;
 }
 
 // (Re)derive the per-replica launch geometry for the current tuning and
@@ -264,6 +270,7 @@ void choose_tuning(lgv_ensemble *e) {
 int configure(lgv_ensemble *e) {
   int tx = 32, ty = 8;
   lgv::ideal_tile_dims(e->tile, &tx, &ty);
+  const int zc = chunk_planes(e);
   std::vector<int> ib(e->R), pb(e->R), sb(e->R), tb(e->R), rb(e->R);
   for (int r = 0; r < e->R; ++r) {
     RepDesc &d = e->hd[r];
@@ -271,7 +278,7 @@ int configure(lgv_ensemble *e) {
     d.nchunk = (int)(((long long)N * d.g.H + 127) / 128);
     d.igx = (N + tx - 1) / tx;
     d.igy = (N + ty - 1) / ty;
-    d.igz = (N + std::min(e->zchunk, N) - 1) / std::min(e->zchunk, N);
+    d.igz = (N + std::min(zc, N) - 1) / std::min(zc, N);
     d.izc = (N + d.igz - 1) / d.igz;  // as many chunks, evenly long
     ib[r] = e->tma_ok[r] ? 0 : d.igx * d.igy * d.igz;
     tb[r] = e->tma_ok[r] ? lgv::batch_tma_blocks(N, d.izc) : 0;
@@ -914,10 +921,11 @@ int lgv_ensemble_use_persistent(lgv_ensemble *e, int enable) {
   return LGV_OK;
 }
 
-// Times every (tile, z-chunk, packing order) candidate on a copy of the
-// current state (the state and the counter are restored afterwards) and
-// keeps the fastest.  choice[3] receives (tile, zchunk, order); ms_per_step
-// the candidate's time per step.
+// Times the choice in use and every (tile, z-chunk, packing order) candidate on a
+// copy of the current state (the state and the counter are restored afterwards)
+// and keeps the fastest: a candidate replaces the choice in use only where it
+// measures faster.  choice[3] receives (tile, zchunk, order); ms_per_step its time
+// per step.
 int lgv_ensemble_autotune(lgv_ensemble *e, int evolver, int inner, int outer, double dt, int steps, int *choice,
                           double *ms_per_step) {
   if (!e) return efail(LGV_ERR_INVALID, "ensemble is NULL");
@@ -953,33 +961,35 @@ int lgv_ensemble_autotune(lgv_ensemble *e, int evolver, int inner, int outer, do
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
-  double best = 1e300;
+  double best = 0;
   int bt = e->tile, bz = e->zchunk, bo = e->order;
+  auto time_choice = [&](int tile, int zchunk, int order) -> int {
+    e->tile = tile;
+    e->zchunk = zchunk;
+    e->order = order;
+    ETRY(configure(e));
+    ETRY(lgv_ensemble_step(e, evolver, inner, outer, dt, 0.0, 2));  // warm / capture
+    cudaEventRecord(a, e->stream);
+    ETRY(lgv_ensemble_step(e, evolver, inner, outer, dt, 0.0, steps));
+    cudaEventRecord(b, e->stream);
+    cudaEventSynchronize(b);
+    float ms = 0;
+    cudaEventElapsedTime(&ms, a, b);
+    if (best == 0 || ms / steps < best) {
+      best = ms / steps;
+      bt = tile;
+      bz = zchunk;
+      bo = order;
+    }
+    restore();
+    return LGV_OK;
+  };
   const int tiles[2] = {LGV_TILE_32x8, LGV_TILE_16x16};
   const int zcs[3] = {8, 16, 32};
-  int rc = LGV_OK;
+  int rc = time_choice(bt, bz, bo);
   for (int ti = 0; ti < 2 && rc == LGV_OK; ++ti)
     for (int zi = 0; zi < 3 && rc == LGV_OK; ++zi)
-      for (int oi = 0; oi < 3 && rc == LGV_OK; ++oi) {
-        e->tile = tiles[ti];
-        e->zchunk = zcs[zi];
-        e->order = oi;
-        if ((rc = configure(e)) != LGV_OK) break;
-        if ((rc = lgv_ensemble_step(e, evolver, inner, outer, dt, 0.0, 2)) != LGV_OK) break;  // warm / capture
-        cudaEventRecord(a, e->stream);
-        if ((rc = lgv_ensemble_step(e, evolver, inner, outer, dt, 0.0, steps)) != LGV_OK) break;
-        cudaEventRecord(b, e->stream);
-        cudaEventSynchronize(b);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, a, b);
-        if (ms / steps < best) {
-          best = ms / steps;
-          bt = e->tile;
-          bz = e->zchunk;
-          bo = e->order;
-        }
-        restore();
-      }
+      for (int oi = 0; oi < 3 && rc == LGV_OK; ++oi) rc = time_choice(tiles[ti], zcs[zi], oi);
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   e->tile = bt;
