@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/lgv.h"
 #include "lgv_dft.cuh"
@@ -206,8 +207,11 @@ __global__ void __launch_bounds__(128) x2k_rotated_kernel(const double *__restri
 // out[tau * ns + s] (complex: pairs).
 //
 // Block: 32 series (lanes) x kCorrLagWarps lag groups (warps); a thread owns G
-// consecutive lags and keeps their sums in registers.  Each lag's sum runs over
-// t in increasing order.
+// consecutive lags and keeps their sums in registers.  Every sum has a fixed
+// order: with decim = 1 the products of G steps, then those sums over t, then the
+// shares of the blocks that divide the time, whose number follows from T, ntmax
+// and the number of series (and with it the last bits); with decim > 1 the
+// products in increasing t.
 template <bool CPLX>
 struct Val {
   double re, im;
@@ -300,6 +304,47 @@ __device__ __forceinline__ void copy_val(double *dst, const double *src) {
   }
 }
 
+// The products of G steps (values of a from xa on) with G lags each, added to
+// acc: step u and lag g take row u + g of the window of b, whose first G rows are
+// at w0 and the others at w1 (rows are 32 values apart).  FULL: all products are
+// wanted; otherwise those with u + g < left, and no other is formed.  The G steps'
+// products are added by themselves first; the two that a complex multiply-add
+// gives one sum are G chains apart.
+template <bool CPLX, int G, bool FULL>
+__device__ __forceinline__ void add_group(Val<CPLX> (&acc)[G], const double *xa, const double *w0, const double *w1,
+                                          int left) {
+  constexpr int W = CPLX ? 2 : 1;
+  Val<CPLX> wb[2 * G - 1], sum[G];
+#pragma unroll
+  for (int i = 0; i < 2 * G - 1; ++i) wb[i] = ld_val<CPLX, true>((i < G ? w0 : w1) + (i < G ? i : i - G) * 32 * W);
+#pragma unroll
+  for (int g = 0; g < G; ++g) sum[g].re = sum[g].im = 0.0;
+#pragma unroll
+  for (int u = 0; u < G; ++u) {
+    const Val<CPLX> x = ld_val<CPLX, true>(xa + u * 32 * W);
+    auto in = [&](int g) { return FULL || u + g < left; };
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+      if (in(g)) sum[g].re = u == 0 ? x.re * wb[g].re : fma(x.re, wb[u + g].re, sum[g].re);
+    if (CPLX) {
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (in(g)) sum[g].im = u == 0 ? x.re * wb[g].im : fma(x.re, wb[u + g].im, sum[g].im);
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (in(g)) sum[g].re = fma(-x.im, wb[u + g].im, sum[g].re);
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (in(g)) sum[g].im = fma(x.im, wb[u + g].re, sum[g].im);
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    acc[g].re += sum[g].re;
+    if (CPLX) acc[g].im += sum[g].im;
+  }
+}
+
 // Every sample (decim 1).  Time runs in chunks of kCorrChunk steps: the block
 // keeps the chunk's rows of a (two chunks, one arriving by cp.async while the
 // other is used) and a ring of the rows of b its lags reach, each row loaded
@@ -309,12 +354,18 @@ __device__ __forceinline__ void copy_val(double *dst, const double *src) {
 // per issue on the load, FP64 pipe a fifth busy.  2000 samples of 1419 complex
 // series, 250 lags: 600 -> 276 us (a complex multiply-add is four fma's, 155 us
 // of FP64 pipe; 320 us without the time shared by two blocks, when 360 blocks
-// left half the SMs with two and half with three).  Two warps per block copy more per product (424 us), six and
-// eight leave the last wave emptier (374, 437 us).
+// left half the SMs with two and half with three).  Two warps per block copy more
+// per product (424 us), six and eight leave the last wave emptier (374, 437 us).
+// The groups of the last chunks, where some products lie past the end, are
+// unrolled like the others with each product under its test: taken one by one
+// (ring row by ring row) they cost a block of real series some 40 us (100 samples
+// of 20 000, 20 lags 111 -> 32 us; 300 of 4257, 15 lags 70 -> 20; 1000 of 4257,
+// 200 lags 166 -> 123; 2000 of 1419, 250 lags 134 -> 104).
+// Complex blocks are held to 128 registers, which four per SM need.
 constexpr int kCorrChunk = 16;
 
 template <bool CPLX, bool VEC, int G>
-__global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *__restrict__ a,
+__global__ void __launch_bounds__(32 * kCorrLagWarps, CPLX ? 4 : 3) otot_kernel(const double *__restrict__ a,
                                                                  const double *__restrict__ b, long long T,
                                                                  long long Tz, long long ns, long long ld, int ntmax,
                                                                  int conn, double *__restrict__ out) {
@@ -356,19 +407,6 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *
   Val<CPLX> acc[G];
 #pragma unroll
   for (int g = 0; g < G; ++g) acc[g].re = acc[g].im = 0.0;
-  auto val = [&](const double *base, int row) {
-    Val<CPLX> v;
-    const double *p = base + (row * 32 + lane) * W;
-    if (CPLX) {
-      const double2 q = *reinterpret_cast<const double2 *>(p);
-      v.re = q.x;
-      v.im = q.y;
-    } else {
-      v.re = p[0];
-      v.im = 0.0;
-    }
-    return v;
-  };
   int ra = 0, rb = 0;  // ring rows of the chunk's first a and b
   for (long long t0 = tz; t0 < te; t0 += C) {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -376,51 +414,21 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_kernel(const double *
     load_rows(ga, sa + (C - ra) * 32 * W, Ta - t0 - C);
     load_rows(gb, sb + (rb >= C ? rb - C : rb + RB - C) * 32 * W, Ta - t0 - C - L);  // onto the rows before rb
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    if (t0 + C - 1 + tau0 - tb + G - 1 < Ta) {
+    // The G steps' window of b: rows r .. r + 2G - 2, where the ring can end only at r + G (RB, rb, h, wp G are
+    // multiples of G).  Step u and lag g of a group meet at window row u + g: a sample while h + u + g < left.
+    const long long left = Ta - t0 - (tau0 - tb);
+    auto groups = [&](auto full) {
 #pragma unroll 1
       for (int h = 0; h < C; h += G) {
-        // the G steps' window of b: rows r .. r + 2G - 2, where the ring can end only at r + G (RB, rb, h, wp G
-        // are multiples of G)
         int r = rb + h + wp * G;
         if (r >= RB) r -= RB;
         const double *w0 = sb + (r * 32 + lane) * W, *w1 = sb + ((r + G < RB ? r + G : 0) * 32 + lane) * W;
-        const double *xa = sa + ((ra + h) * 32 + lane) * W;
-        Val<CPLX> wb[2 * G - 1], sum[G];
-#pragma unroll
-        for (int i = 0; i < 2 * G - 1; ++i) wb[i] = ld_val<CPLX, true>((i < G ? w0 : w1) + (i < G ? i : i - G) * 32 * W);
-#pragma unroll
-        for (int u = 0; u < G; ++u) {
-          const Val<CPLX> x = ld_val<CPLX, true>(xa + u * 32 * W);
-          // the G steps' products are added by themselves first; the two
-          // that a complex multiply-add gives one sum are G chains apart
-#pragma unroll
-          for (int g = 0; g < G; ++g) sum[g].re = u == 0 ? x.re * wb[g].re : fma(x.re, wb[u + g].re, sum[g].re);
-          if (CPLX) {
-#pragma unroll
-            for (int g = 0; g < G; ++g) sum[g].im = u == 0 ? x.re * wb[g].im : fma(x.re, wb[u + g].im, sum[g].im);
-#pragma unroll
-            for (int g = 0; g < G; ++g) sum[g].re = fma(-x.im, wb[u + g].im, sum[g].re);
-#pragma unroll
-            for (int g = 0; g < G; ++g) sum[g].im = fma(x.im, wb[u + g].re, sum[g].im);
-          }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          acc[g].re += sum[g].re;
-          if (CPLX) acc[g].im += sum[g].im;
-        }
+        add_group<CPLX, G, decltype(full)::value>(acc, sa + ((ra + h) * 32 + lane) * W, w0, w1, (int)left - h);
       }
-    } else {  // some products lie past the end
-#pragma unroll 1
-      for (int u = 0; u < C; ++u) {
-        const Val<CPLX> x = val(sa, ra + u);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          int r = rb + u + wp * G + g;
-          if (r >= RB) r -= RB;
-          if (t0 + u + tau0 - tb + g < Ta) mac<CPLX>(acc[g], x, val(sb, r));
-        }
-      }
+    };
+    if (left > 0 && (CPLX || tau0 < ntmax)) {
+      if (left >= C + G - 1) groups(std::true_type{});
+      else groups(std::false_type{});
     }
     ra = C - ra;
     rb += C;
