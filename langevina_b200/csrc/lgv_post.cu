@@ -56,7 +56,9 @@ int launched(const char *where) {
 // 92 (rows of 90, 500, 24 and 166: the first is the fastest too); at 5 and 5, 8
 // rows and four blocks per SM 138 us, 16 rows and two blocks 90.
 constexpr int kX2kThreads = 256, kX2kB1 = 3, kX2kB2 = 2, kX2kStageMaxN = 4096;
-constexpr int kX2kLogRows = 4;  // 16 rows per block where they fit
+// 16 rows per block where they fit; of rows below kX2kRunN up to 256, so that the
+// blocks stay one round
+constexpr int kX2kLogRows = 4, kX2kMaxLogRows = 8;
 constexpr int kX2kBlocks = 3;   // blocks per SM
 
 constexpr size_t kX2kSmem = 226 * 1024 / kX2kBlocks - 1024;
@@ -67,6 +69,31 @@ struct X2kShape {
   int SA, SZ;   // strides of a row of walls / modes (doubles) and of Z (double2), odd
 };
 
+// A warp per row leaves lanes idle where rows are short, and so do 16 rows where a
+// row has few columns: below this the block copies its rows as one run, takes more
+// of them, and divides by N as they leave (10 000 rows of 6: 9.8 -> 6.9 us, 60 000:
+// 27 -> 10, where direct sums take 6.0 and 12; 60 000 of 20 and 46: 30 -> 21 and 38
+// -> 34, but of 62 45 -> 47).
+constexpr int kX2kRunN = 48;
+
+// This thread's elements of the nr rows of M doubles that are one run at g, and
+// that lie `stride` apart in shared memory; f(element of g, element of shared memory).
+template <typename F>
+__device__ __forceinline__ void run_elements(int nr, int M, int stride, F f) {
+  int r = threadIdx.x / M, x = threadIdx.x - r * M;
+  const int dr = kX2kThreads / M, dx = kX2kThreads - dr * M;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < nr * M; e += kX2kThreads) {
+    f(e, r * stride + x);
+    r += dr;
+    x += dx;
+    if (x >= M) {
+      x -= M;
+      ++r;
+    }
+  }
+}
+
 template <bool STAGE>
 __global__ void __launch_bounds__(kX2kThreads, kX2kBlocks) x2k_kernel(const double *__restrict__ w, long long rows, X2kShape s,
                                                           double *__restrict__ out) {
@@ -76,12 +103,19 @@ __global__ void __launch_bounds__(kX2kThreads, kX2kBlocks) x2k_kernel(const doub
   double2 *tw = sm2, *Z = sm2 + N;
   double *A = (double *)(Z + (size_t)R * s.SZ);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool runs = STAGE && N < kX2kRunN;  // rows as one run, divided by N as they leave
   dft::fill_twiddles(tw, N);
   for (long long r0 = (long long)blockIdx.x * R; r0 < rows; r0 += (long long)gridDim.x * R) {
   const int nr = (int)min((long long)R, rows - r0);
-  if (STAGE)
-    for (int rr = warp; rr < nr; rr += kX2kThreads / 32)
-      for (int x = lane; x < N; x += 32) A[rr * s.SA + x] = w[(r0 + rr) * N + x];
+  if (STAGE) {
+    const double *src = w + r0 * N;
+    if (runs) {
+      run_elements(nr, N, s.SA, [&](int e, int a) { A[a] = src[e]; });
+    } else {
+      for (int rr = warp; rr < nr; rr += kX2kThreads / 32)
+        for (int x = lane; x < N; x += 32) A[rr * s.SA + x] = src[(size_t)rr * N + x];
+    }
+  }
   __syncthreads();
   const int rr = threadIdx.x & (R - 1), u0 = threadIdx.x >> s.logR, nu = kX2kThreads >> s.logR;
   const bool live = rr < nr;
@@ -115,15 +149,20 @@ __global__ void __launch_bounds__(kX2kThreads, kX2kBlocks) x2k_kernel(const doub
 #pragma unroll
       for (int b = 0; b < kX2kB2; ++b) {
         if (c0 + b >= n2h) continue;
-        dft::store(p, k1, k2[b], W[b], o);
-        if (k2[b] > 0 && 2 * k2[b] < p.N2) dft::store(p, k1, p.N2 - k2[b], M[b], o);
+        dft::store(p, k1, k2[b], W[b], o, !runs);
+        if (k2[b] > 0 && 2 * k2[b] < p.N2) dft::store(p, k1, p.N2 - k2[b], M[b], o, !runs);
       }
     }
   }
   __syncthreads();
   if (STAGE) {
-    for (int r = warp; r < nr; r += kX2kThreads / 32)
-      for (int x = lane; x < 2 * NK; x += 32) out[(r0 + r) * NK * 2 + x] = A[r * s.SA + x];
+    double *dst = out + r0 * NK * 2;
+    if (runs) {
+      run_elements(nr, 2 * NK, s.SA, [&](int e, int a) { dst[e] = dft::scaled(p, A[a]); });
+    } else {
+      for (int r = warp; r < nr; r += kX2kThreads / 32)
+        for (int x = lane; x < 2 * NK; x += 32) dst[(size_t)r * NK * 2 + x] = A[r * s.SA + x];
+    }
     __syncthreads();
   }
   }
@@ -525,6 +564,8 @@ int lgv_x2k(const double *walls, int64_t rows, int N, double *out, void *stream)
   const size_t per_row = s.SZ * sizeof(double2) + (stage ? s.SA * sizeof(double) : 0);
   const size_t table = (size_t)N * sizeof(double2);
   s.logR = stage ? kX2kLogRows : 0;
+  // more rows per block where that leaves fewer rounds of blocks
+  while (N < kX2kRunN && s.logR < kX2kMaxLogRows && (rows >> s.logR) > 148LL * kX2kBlocks) ++s.logR;
   while (s.logR > 0 && table + (per_row << s.logR) > kX2kSmem) --s.logR;
   s.R = 1 << s.logR;
   const size_t smem = table + (per_row << s.logR);
