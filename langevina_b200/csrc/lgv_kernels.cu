@@ -963,9 +963,11 @@ __device__ __forceinline__ void charge_link_site(const Fields &f, const Geo &g, 
 
 // Grid as hb_pass_kernel (pass_site).
 // 16 blocks of 128 threads per SM (32 registers): the link updates are long
-// integer / FP64 chains, and full occupancy hides them best
+// integer / FP64 chains, and full occupancy hides them best.  With statistics
+// eight: in 32 registers the tallies spill 300 to 600 bytes (a charge step of 48^3
+// 102 us, 256^3 2917; in 64 registers 37 and 2350).
 template <bool INJECTED, bool MON, bool ROWS, typename I>
-__global__ void __launch_bounds__(128, 16) charge_pass_kernel(Fields f, Geo g, int dir, int eoA, ChargeArgs a) {
+__global__ void __launch_bounds__(128, MON ? 8 : 16) charge_pass_kernel(Fields f, Geo g, int dir, int eoA, ChargeArgs a) {
   pdl_launch();
   pdl_wait();
   int m, j, k;
