@@ -489,13 +489,18 @@ __device__ __forceinline__ void hb_pass(const Fields &f, const Geo &g, int parit
   if (MON) mon_flush(mon, a.mon);
 }
 
+// Eight blocks per SM: 60 to 64 registers let more of a site's loads be in flight
+// than the 40 that the compiler takes by itself with 32-bit offsets (Gaussian
+// proposals 44): a sweep of 256^3 311 -> 285 us, 512^3 2589 -> 2470; Gaussian 64^3
+// 9.2 -> 7.9, 128^3 55 -> 52, 196^3 232 -> 204, 256^3 543 -> 480, 512^3 4390 -> 3800
+// (219, 513 and 3990 before the 32-bit byte offsets). Ten, seven: within 5 %.
 template <bool INJECTED, bool MON, bool ROWS, typename I, bool GAUSS>
-__global__ void __launch_bounds__(128) hb_pass_kernel(Fields f, Geo g, int parity, HbArgs a) {
+__global__ void __launch_bounds__(128, 8) hb_pass_kernel(Fields f, Geo g, int parity, HbArgs a) {
   hb_pass<INJECTED, MON, ROWS, I, GAUSS>(f, g, parity, a);
 }
 // The same compiled for few resident blocks: on a lattice that is over in a few
-// waves a pass is one chain of latencies, and the registers (76 against 40, with
-// Gaussian proposals 84 against 58) let a site's 28 loads be in flight together.
+// waves a pass is one chain of latencies, and the registers (76, with Gaussian
+// proposals 84) let a site's 28 loads be in flight together.
 // A sweep of 32^3 6.2 -> 4.8 us, 48^3 9.2 -> 5.7, 64^3 10.0 -> 7.6, 80^3 12.4 ->
 // 11.2, 96^3 16.6 -> 16.0, 110^3 23.7 -> 22.9; 128^3 33 either way, and beyond
 // that occupancy wins (256^3 329 against 334-342).  Gaussian: 32^3 7.0 -> 4.7,
