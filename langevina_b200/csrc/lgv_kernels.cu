@@ -1165,7 +1165,8 @@ __global__ void __launch_bounds__(1024) charge_row_kernel(Geo g, ChargeDirArgs a
 // (j, m) elements of a plane, threads 0..127 in the even and 128..255 in the odd
 // half.  Grid (ceil(N H / 128), planes).
 constexpr int kSiteThreads = 256;
-// resident blocks per SM of the Euler-Maruyama step, its adjoint and the ideal step's adjoint (48, 80 and 86-128 registers)
+// resident blocks per SM of the Euler-Maruyama step with sums, its adjoint and the ideal step's adjoint (48, 80 and
+// 86-128 registers)
 constexpr int kEmBlocks = 5, kEmAdjBlocks = 3, kIdealAdjBlocks = 2;
 
 __device__ __forceinline__ bool all_site(const Geo &g, int chunk, int &parity, int &m, int &j) {
@@ -1215,9 +1216,9 @@ __device__ __forceinline__ void em_site(const Fields &in, const Fields &out, con
   }
 }
 
-// SUM: also the sums of the new phi, a row per block.
-template <bool INJECTED, bool SUM, typename I>
-__global__ void __launch_bounds__(kSiteThreads, kEmBlocks) em_kernel(Fields in, Fields out, Geo g, EmArgs a, double *partial) {
+// SUM: also the sums of the new phi, a row per block.  NB: resident blocks per SM.
+template <bool INJECTED, bool SUM, typename I, int NB = kEmBlocks>
+__global__ void __launch_bounds__(kSiteThreads, NB) em_kernel(Fields in, Fields out, Geo g, EmArgs a, double *partial) {
   pdl_launch();
   int parity, m, j;
   double acc[4] = {0, 0, 0, 0};
@@ -3079,11 +3080,17 @@ cudaError_t launch_em(Fields in, Fields out, int N, const EmArgs &a, cudaStream_
 }
 
 cudaError_t launch_em(Fields in, Fields out, const Geo &g, const EmArgs &a, cudaStream_t st) {
-  const bool i32 = idx32(g), el = idx_el(g);
-  const auto kern = a.xi ? (i32 ? em_kernel<true, false, unsigned> : el ? em_kernel<true, false, int>
-                                                                        : em_kernel<true, false, long long>)
-                         : (i32 ? em_kernel<false, false, unsigned> : el ? em_kernel<false, false, int>
-                                                                         : em_kernel<false, false, long long>);
+  // Five blocks per SM (48 registers) where that is one round of blocks (24^3 to
+  // 56^3 0.2 to 0.3 us faster than six), six beyond (128^3 51.1 -> 50.3 us, 300^3
+  // 675 -> 643, 400^3 1602 -> 1533, 720^3 10.3 -> 9.9 ms), and eight (32 registers)
+  // for the largest lattices' int offsets (814^3 16.3 -> 15.4 ms).
+  const bool one_round = 2 * g.V2 <= 148LL * kEmBlocks * kSiteThreads;
+#define LGV_EM(J)                                                                      \
+  (one_round ? em_kernel<J, false, unsigned>                                           \
+             : idx32(g) ? em_kernel<J, false, unsigned, 6>                             \
+                        : idx_el(g) ? em_kernel<J, false, int, 8> : em_kernel<J, false, long long, 6>)
+  const auto kern = a.xi ? LGV_EM(true) : LGV_EM(false);
+#undef LGV_EM
   return launch_pdl(kern, site_grid(g), dim3(kSiteThreads), 0, st, in, out, g, a, nullptr);
 }
 
