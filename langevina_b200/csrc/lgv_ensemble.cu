@@ -136,6 +136,19 @@ int ens_check_waits(lgv_ensemble *e) {
   return LGV_OK;
 }
 
+// Device memory for the ensemble's other needs: where there is no room the kept
+// staging makes some, so that it never refuses a call.  Not under capture.
+cudaError_t ens_malloc(lgv_ensemble *e, void **p, size_t bytes) {
+  cudaError_t c = cudaMalloc(p, bytes);
+  if (c == cudaErrorMemoryAllocation && e->staging) {
+    cudaGetLastError();
+    cudaFree(e->staging);  // waits for the copies that use it
+    e->staging = nullptr;
+    c = cudaMalloc(p, bytes);
+  }
+  return c;
+}
+
 void free_map(BlockMap &m) {
   if (m.rep) cudaFree(m.rep);
   if (m.first) cudaFree(m.first);
@@ -183,9 +196,9 @@ int build_map(lgv_ensemble *e, BlockMap &m, const std::vector<int> &blocks_per_r
     rep.insert(rep.end(), blocks_per_rep[r], r);
   }
   m.nblocks = (int)rep.size();
-  ECK(cudaMalloc((void **)&m.rep, std::max<size_t>(rep.size(), 1) * sizeof(int)));
-  ECK(cudaMalloc((void **)&m.first, e->R * sizeof(int)));
-  ECK(cudaMalloc((void **)&m.count, e->R * sizeof(int)));
+  ECK(ens_malloc(e, (void **)&m.rep, std::max<size_t>(rep.size(), 1) * sizeof(int)));
+  ECK(ens_malloc(e, (void **)&m.first, e->R * sizeof(int)));
+  ECK(ens_malloc(e, (void **)&m.count, e->R * sizeof(int)));
   ECK(cudaMemcpy(m.rep, rep.data(), rep.size() * sizeof(int), cudaMemcpyHostToDevice));
   ECK(cudaMemcpy(m.first, first.data(), e->R * sizeof(int), cudaMemcpyHostToDevice));
   ECK(cudaMemcpy(m.count, count.data(), e->R * sizeof(int), cudaMemcpyHostToDevice));
@@ -294,7 +307,7 @@ int configure(lgv_ensemble *e) {
   ETRY(build_map(e, e->run_map, rb));
   if (e->partial) cudaFree(e->partial);
   e->partial = nullptr;
-  ECK(cudaMalloc((void **)&e->partial, (size_t)e->plane_map.nblocks * 11 * sizeof(double)));
+  ECK(ens_malloc(e, (void **)&e->partial, (size_t)e->plane_map.nblocks * 11 * sizeof(double)));
   clear_graphs(e);
   return LGV_OK;
 }
@@ -475,9 +488,9 @@ Fields cur_fields(const lgv_ensemble *e, int r) {
   return f;
 }
 
-// Staging for the host boundary, kept for the ensemble's life: a cudaMalloc and
-// cudaFree per call cost more than the copy (52 replicas, 244 MB: 70 ms to read
-// back, now 7).
+// Staging for the host boundary, kept between calls (80 B per site of the largest
+// replica): a cudaMalloc and cudaFree per call cost more than the copy (52
+// replicas, 244 MB: 70 ms to read back, now 7).
 int ensure_staging(lgv_ensemble *e) {
   if (e->staging) return LGV_OK;
   size_t V = 0;
@@ -654,7 +667,7 @@ int lgv_ensemble_initialize(lgv_ensemble *e, int kind, double scale) {
     const size_t V = (size_t)e->p[r].N * e->p[r].N * e->p[r].N;
     need = std::max(need, ((V + 255) / 256) * 6 + 16);
   }
-  if (kind == LGV_INIT_CHARGES_GAUSSIAN) ECK(cudaMalloc((void **)&scratch, need * sizeof(double)));
+  if (kind == LGV_INIT_CHARGES_GAUSSIAN) ECK(ens_malloc(e, (void **)&scratch, need * sizeof(double)));
   int rc = LGV_OK;
   for (int r = 0; r < e->R && rc == LGV_OK; ++r) {
     const Fields f = cur_fields(e, r);
@@ -756,8 +769,8 @@ int lgv_ensemble_diff_forward(lgv_ensemble *e, double dt, double t, int nsteps, 
     D.bufs.assign(R, nullptr);
     D.lens.assign(R, 0);
     D.hd.assign(R, lgv::DiffDesc{});
-    ECK(cudaMalloc((void **)&D.dd, R * sizeof(lgv::DiffDesc)));
-    ECK(cudaMalloc((void **)&D.wg, (size_t)R * 6 * sizeof(double)));
+    ECK(ens_malloc(e, (void **)&D.dd, R * sizeof(lgv::DiffDesc)));
+    ECK(ens_malloc(e, (void **)&D.wg, (size_t)R * 6 * sizeof(double)));
   }
   const int slots = lgv::sum_slots(e->plane_map.nblocks);
   const size_t need_partial = (size_t)slots * e->plane_map.nblocks * 4;
@@ -765,7 +778,7 @@ int lgv_ensemble_diff_forward(lgv_ensemble *e, double dt, double t, int nsteps, 
     if (D.partial) cudaFree(D.partial);
     D.partial = nullptr;
     D.partial_len = 0;
-    ECK(cudaMalloc((void **)&D.partial, need_partial * sizeof(double)));
+    ECK(ens_malloc(e, (void **)&D.partial, need_partial * sizeof(double)));
     D.partial_len = need_partial;
   }
   for (int r = 0; r < R; ++r) {
@@ -776,7 +789,7 @@ int lgv_ensemble_diff_forward(lgv_ensemble *e, double dt, double t, int nsteps, 
       if (D.bufs[r]) cudaFree(D.bufs[r]);
       D.bufs[r] = nullptr;
       D.lens[r] = 0;
-      ECK(cudaMalloc((void **)&D.bufs[r], need * sizeof(double)));
+      ECK(ens_malloc(e, (void **)&D.bufs[r], need * sizeof(double)));
       D.lens[r] = need;
     }
     lgv::DiffDesc &d = D.hd[r];
@@ -938,7 +951,7 @@ int lgv_ensemble_autotune(lgv_ensemble *e, int evolver, int inner, int outer, do
   for (int r = 0; r < e->R; ++r) {
     const size_t V = (size_t)e->p[r].N * e->p[r].N * e->p[r].N;
     double *s = nullptr;
-    if (cudaMalloc((void **)&s, 10 * V * sizeof(double)) != cudaSuccess) {
+    if (ens_malloc(e, (void **)&s, 10 * V * sizeof(double)) != cudaSuccess) {
       for (double *q : saved) cudaFree(q);
       return efail(LGV_ERR_NOMEM, "autotune: no room for the state copy");
     }

@@ -69,7 +69,7 @@ def test_substeps_equal_small_slabs(lgv, N):
             s = S.SlabLattice(N, k0, 2, NoExchange(), **COEF)
             try:
                 s.L = g.L
-                g.L.check(s.lib.lgv_set_state(s.h, g.L.ptr(np.ascontiguousarray(box))), "set_state")
+                g.L.check(s.lib.lgv_set_state(s.h, g.L.ptr(box)), "set_state")
                 if ev == HB:
                     g.L.check(s.lib.lgv_set_hb_proposal(s.h, gauss), "proposal")
                 s.set_counter(ctr)
