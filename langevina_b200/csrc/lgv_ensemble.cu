@@ -643,9 +643,13 @@ int lgv_ensemble_set_state(lgv_ensemble *e, int r, const double *host_aos) {
   if (!host_aos) return efail(LGV_ERR_INVALID, "NULL state");
   const size_t V = (size_t)e->p[r].N * e->p[r].N * e->p[r].N;
   ETRY(ensure_staging(e));
-  ECK(cudaMemcpyAsync(e->staging, host_aos, 10 * V * sizeof(double), cudaMemcpyHostToDevice, e->stream));
-  ECK(lgv::launch_aos_to_rb(e->staging, cur_fields(e, r), e->p[r].N, e->stream));
-  ECK(cudaStreamSynchronize(e->stream));
+  // host_aos may be pinned: the stream is waited for whatever failed before
+  const cudaError_t c1 = cudaMemcpyAsync(e->staging, host_aos, 10 * V * sizeof(double), cudaMemcpyHostToDevice, e->stream);
+  const cudaError_t c2 = lgv::launch_aos_to_rb(e->staging, cur_fields(e, r), e->p[r].N, e->stream);
+  const cudaError_t c3 = cudaStreamSynchronize(e->stream);
+  ECK(c1);
+  ECK(c2);
+  ECK(c3);
   return LGV_OK;
 }
 
