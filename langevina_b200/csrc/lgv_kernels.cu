@@ -121,7 +121,7 @@ __device__ void mon_flush(MonLocal &m, MonAcc *acc) {
   warp_sum(m.un);
   warp_sum(m.dd);
   warp_sum(m.ud);
-  // linear thread index: CTAs may be two-dimensional (charge_x_kernel)
+  // linear thread index: CTAs may be two-dimensional (hb_zpass_kernel)
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
   const int nwarps = (blockDim.x * blockDim.y + 31) >> 5;
   const int w = tid >> 5, l = tid & 31;
@@ -2457,7 +2457,7 @@ __device__ __noinline__ void persist_charge_item(const PersistPtrs &q, int blk, 
 // round robin over the grid: ideal tiles (TMA replicas first, through the
 // same CTA bodies as batch_ideal_tma_kernel and batch_ideal_kernel), or pairs
 // of 128-lane slab items of the heat-bath and charge sub-steps (each half of
-// the CTA one item, as batch_hb_kernel / batch_charge_kernel).  Phases are
+// the CTA one item: batch_hb_item, batch_charge_item).  Phases are
 // separated by grid_barrier; after the last one block 0 advances the
 // ensemble's counter and clock, as launch_ens_advance does after the
 // one-launch-per-sub-step sequence.  Results equal that sequence's bit for
@@ -2616,13 +2616,13 @@ __global__ void __launch_bounds__(kThreads) rot_phi_kernel(Fields u, Fields P1, 
 // The ideal step of a small lattice in two launches: rot_phi_kernel writes phi'
 // to P1, and this one, a thread per site, advects the charges with the stencil
 // on phi' and rotates phi' by the second half step.  Reads the charges of `in`,
-// writes `out`, which may be `in`.
-template <typename I>
+// writes `out`, which may be `in`.  Byte offsets: the lattices it takes have planes
+// far below 4 GB (ideal_flat).
 __global__ void __launch_bounds__(kSiteThreads, 3) ideal_flat_kernel(Fields in, Fields P1, Fields out, Geo g, IdealArgs a) {
   pdl_launch();
   int parity, m, j;
   const bool ok = all_site(g, blockIdx.x, parity, m, j);
-  const Nbrs<I> o = nbrs_of<I>(g, parity, m, j, blockIdx.y);
+  const Nbrs<unsigned> o = nbrs_of<unsigned>(g, parity, m, j, blockIdx.y);
   pdl_wait();
   if (!ok) return;
   double c[4], S[4], q[6];
@@ -3118,8 +3118,7 @@ cudaError_t launch_ideal_flat(Fields in, Fields P1, Fields out, const Geo &g, co
   const cudaError_t e =
       launch_pdl(rot_phi_kernel, dim3(nblocks(V, kThreads)), dim3(kThreads), 0, st, in, P1, V, a.dto2chi);
   if (e != cudaSuccess) return e;
-  return launch_pdl(idx32(g) ? ideal_flat_kernel<unsigned> : ideal_flat_kernel<long long>, site_grid(g), dim3(kSiteThreads), 0,
-                    st, in, P1, out, g, a);
+  return launch_pdl(ideal_flat_kernel, site_grid(g), dim3(kSiteThreads), 0, st, in, P1, out, g, a);
 }
 
 cudaError_t launch_ideal(Fields in, Fields out, int N, const IdealArgs &a, cudaStream_t st) {
