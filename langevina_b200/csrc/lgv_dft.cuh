@@ -135,18 +135,21 @@ __device__ __forceinline__ void outer(const double2 *z, const Plan &p, const dou
 // v / N
 __device__ __forceinline__ double scaled(const Plan &p, double v) { return p.inv != 0.0 ? v * p.inv : v / (double)p.N; }
 
-// Stores W = N W(k1 + N1 k2), divided by N if `scale`, into o[2 kk], o[2 kk + 1]
+// Stores W = N W(k1 + N1 k2), divided by N if SCALE, into o[2 kk], o[2 kk + 1]
 // where it gives an output kk = 0..N/2 that no other (k1, k2) gives.
-__device__ __forceinline__ void store(const Plan &p, int k1, int k2, const double2 &W, double *o, bool scale = true) {
+template <bool SCALE = true>
+__device__ __forceinline__ void store(const Plan &p, int k1, int k2, const double2 &W, double *o) {
   const int k = k1 + p.N1 * k2;
   const bool conj = 2 * k > p.N;
   if (conj && (k1 == 0 || 2 * k1 == p.N1)) return;
   const int kk = conj ? p.N - k : k;
   const double y = conj ? -W.y : W.y;
-  if (!scale || p.inv != 0.0) {
-    const double f = scale ? p.inv : 1.0;
-    o[2 * kk] = W.x * f;
-    o[2 * kk + 1] = y * f;
+  if (!SCALE) {
+    o[2 * kk] = W.x;
+    o[2 * kk + 1] = y;
+  } else if (p.inv != 0.0) {
+    o[2 * kk] = W.x * p.inv;
+    o[2 * kk + 1] = y * p.inv;
   } else {
     o[2 * kk] = W.x / (double)p.N;
     o[2 * kk + 1] = y / (double)p.N;

@@ -94,7 +94,8 @@ __device__ __forceinline__ void run_elements(int nr, int M, int stride, F f) {
   }
 }
 
-template <bool STAGE>
+// RUNS: rows copied as one run, and divided by N as they leave.
+template <bool STAGE, bool RUNS>
 __global__ void __launch_bounds__(kX2kThreads, kX2kBlocks) x2k_kernel(const double *__restrict__ w, long long rows, X2kShape s,
                                                           double *__restrict__ out) {
   extern __shared__ __align__(16) double2 sm2[];
@@ -103,17 +104,16 @@ __global__ void __launch_bounds__(kX2kThreads, kX2kBlocks) x2k_kernel(const doub
   double2 *tw = sm2, *Z = sm2 + N;
   double *A = (double *)(Z + (size_t)R * s.SZ);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool runs = STAGE && N < kX2kRunN;  // rows as one run, divided by N as they leave
   dft::fill_twiddles(tw, N);
   for (long long r0 = (long long)blockIdx.x * R; r0 < rows; r0 += (long long)gridDim.x * R) {
   const int nr = (int)min((long long)R, rows - r0);
   if (STAGE) {
-    const double *src = w + r0 * N;
-    if (runs) {
+    if (RUNS) {
+      const double *src = w + r0 * N;
       run_elements(nr, N, s.SA, [&](int e, int a) { A[a] = src[e]; });
     } else {
       for (int rr = warp; rr < nr; rr += kX2kThreads / 32)
-        for (int x = lane; x < N; x += 32) A[rr * s.SA + x] = src[(size_t)rr * N + x];
+        for (int x = lane; x < N; x += 32) A[rr * s.SA + x] = w[(r0 + rr) * N + x];
     }
   }
   __syncthreads();
@@ -149,19 +149,19 @@ __global__ void __launch_bounds__(kX2kThreads, kX2kBlocks) x2k_kernel(const doub
 #pragma unroll
       for (int b = 0; b < kX2kB2; ++b) {
         if (c0 + b >= n2h) continue;
-        dft::store(p, k1, k2[b], W[b], o, !runs);
-        if (k2[b] > 0 && 2 * k2[b] < p.N2) dft::store(p, k1, p.N2 - k2[b], M[b], o, !runs);
+        dft::store<!RUNS>(p, k1, k2[b], W[b], o);
+        if (k2[b] > 0 && 2 * k2[b] < p.N2) dft::store<!RUNS>(p, k1, p.N2 - k2[b], M[b], o);
       }
     }
   }
   __syncthreads();
   if (STAGE) {
-    double *dst = out + r0 * NK * 2;
-    if (runs) {
+    if (RUNS) {
+      double *dst = out + r0 * NK * 2;
       run_elements(nr, 2 * NK, s.SA, [&](int e, int a) { dst[e] = dft::scaled(p, A[a]); });
     } else {
       for (int r = warp; r < nr; r += kX2kThreads / 32)
-        for (int x = lane; x < 2 * NK; x += 32) dst[(size_t)r * NK * 2 + x] = A[r * s.SA + x];
+        for (int x = lane; x < 2 * NK; x += 32) out[(r0 + r) * NK * 2 + x] = A[r * s.SA + x];
     }
     __syncthreads();
   }
@@ -570,7 +570,7 @@ int lgv_x2k(const double *walls, int64_t rows, int N, double *out, void *stream)
   s.R = 1 << s.logR;
   const size_t smem = table + (per_row << s.logR);
   const long long blocks = std::min<long long>((rows + s.R - 1) / s.R, 148LL * kX2kBlocks);
-  const auto kern = stage ? x2k_kernel<true> : x2k_kernel<false>;
+  const auto kern = !stage ? x2k_kernel<false, false> : N < kX2kRunN ? x2k_kernel<true, true> : x2k_kernel<true, false>;
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return fail(LGV_ERR_CUDA, "lgv_x2k: shared memory for the rows");
