@@ -286,19 +286,46 @@ __device__ __forceinline__ void mac(Val<CPLX> &acc, const Val<CPLX> &x, const Va
 
 constexpr int kCorrLagWarps = 4;
 
-// mean(a_s) mean(b_s) over all T samples, each sum in increasing t.
+// The sums of n samples of both series, each in increasing t: U samples of both are
+// asked for before the first is added.
 template <bool CPLX, bool VEC>
-__device__ __forceinline__ Val<CPLX> mean_product(const double *pa, const double *pb, long long T, long long ld) {
-  Val<CPLX> sa, sb, cc;
-  sa.re = sa.im = sb.re = sb.im = cc.re = cc.im = 0.0;
-#pragma unroll 8
-  for (long long t = 0; t < T; ++t) {
-    const Val<CPLX> x = ld_val<CPLX, VEC>(pa + t * ld), y = ld_val<CPLX, VEC>(pb + t * ld);
-    sa.re += x.re;
-    sa.im += x.im;
-    sb.re += y.re;
-    sb.im += y.im;
+__device__ __forceinline__ void sample_sums(const double *pa, const double *pb, long long n, long long ld,
+                                            Val<CPLX> &sa, Val<CPLX> &sb) {
+  constexpr int U = CPLX ? 8 : 16;
+  sa.re = sa.im = sb.re = sb.im = 0.0;
+  auto add = [](Val<CPLX> &s, const Val<CPLX> &x) {
+    s.re += x.re;
+    s.im += x.im;
+  };
+  long long t = 0;
+#pragma unroll 1
+  for (; t + U <= n; t += U) {
+    Val<CPLX> x[U], y[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      x[u] = ld_val<CPLX, VEC>(pa + u * ld);
+      y[u] = ld_val<CPLX, VEC>(pb + u * ld);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      add(sa, x[u]);
+      add(sb, y[u]);
+    }
+    pa += U * ld;
+    pb += U * ld;
   }
+#pragma unroll 1
+  for (; t < n; ++t, pa += ld, pb += ld) {
+    add(sa, ld_val<CPLX, VEC>(pa));
+    add(sb, ld_val<CPLX, VEC>(pb));
+  }
+}
+
+// mean(a_s) mean(b_s) from the sums over all T samples
+template <bool CPLX>
+__device__ __forceinline__ Val<CPLX> mean_product(Val<CPLX> sa, Val<CPLX> sb, long long T) {
+  Val<CPLX> cc;
+  cc.re = cc.im = 0.0;
   sa.re /= (double)T;
   sa.im /= (double)T;
   sb.re /= (double)T;
@@ -465,7 +492,7 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps, CPLX ? 4 : 3) otot_kernel(
         add_group<CPLX, G, decltype(full)::value>(acc, sa + ((ra + h) * 32 + lane) * W, w0, w1, (int)left - h);
       }
     };
-    if (left > 0 && (CPLX || tau0 < ntmax)) {
+    if (left > 0 && tau0 < ntmax) {
       if (left >= C + G - 1) groups(std::true_type{});
       else groups(std::false_type{});
     }
@@ -495,10 +522,31 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps, CPLX ? 4 : 3) otot_kernel(
     cluster_sync();  // the other blocks' shared memory stays until it is read
     if (blockIdx.z > 0) return;
   }
-  if (!live || tau0 >= ntmax) return;
   Val<CPLX> cc;
   cc.re = cc.im = 0.0;
-  if (conn) cc = mean_product<CPLX, VEC>(pa, pb, T, ld);
+  if (conn) {  // each warp sums its share of the time, all add the shares in order
+    const long long share = (T + NW - 1) / NW, t0 = min(T, wp * share);
+    Val<CPLX> sums[2];
+    sample_sums<CPLX, VEC>(pa + t0 * ld, pb + t0 * ld, min(T, t0 + share) - t0, ld, sums[0], sums[1]);
+    __syncthreads();  // the last reads of the ring are over
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      sm[((wp * 2 + i) * 2) * 32 + lane] = sums[i].re;
+      if (CPLX) sm[((wp * 2 + i) * 2 + 1) * 32 + lane] = sums[i].im;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      sums[i].re = sums[i].im = 0.0;
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        sums[i].re += sm[((w * 2 + i) * 2) * 32 + lane];
+        if (CPLX) sums[i].im += sm[((w * 2 + i) * 2 + 1) * 32 + lane];
+      }
+    }
+    cc = mean_product<CPLX>(sums[0], sums[1], T);
+  }
+  if (!live || tau0 >= ntmax) return;
   store_lags<CPLX, G>(acc, cc, tau0, T, ntmax, 1, out + s * W, ns * W);
 }
 
@@ -541,7 +589,11 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps) otot_decim_kernel(const do
   }
   Val<CPLX> cc;
   cc.re = cc.im = 0.0;
-  if (conn) cc = mean_product<CPLX, VEC>(pa, pb, T, ld);
+  if (conn) {
+    Val<CPLX> sa, sb;
+    sample_sums<CPLX, VEC>(pa, pb, T, ld, sa, sb);
+    cc = mean_product<CPLX>(sa, sb, T);
+  }
   store_lags<CPLX, G>(acc, cc, tau0, T, ntmax, decim, out + s * W, ns * W);
 }
 
