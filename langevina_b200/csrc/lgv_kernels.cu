@@ -510,8 +510,8 @@ __global__ void __launch_bounds__(128, 8) hb_pass_kernel(Fields f, Geo g, int pa
 // proposals 84) let a site's 28 loads be in flight together.
 // A sweep of 32^3 6.2 -> 4.8 us, 48^3 9.2 -> 5.7, 64^3 10.0 -> 7.6, 80^3 12.4 ->
 // 11.2, 96^3 16.6 -> 16.0, 110^3 23.7 -> 22.9; 128^3 33 either way, and beyond
-// that occupancy wins (256^3 329 against 334-342).  Gaussian: 32^3 7.0 -> 4.7,
-// 48^3 7.7 -> 4.9, but 64^3 8.6 -> 9.3.
+// that eight blocks are faster (256^3 285 against 334-342).  Gaussian: 32^3 7.0 ->
+// 4.7, 48^3 7.7 -> 4.9, but 64^3 7.9 -> 9.3.
 template <bool GAUSS>
 __global__ void __launch_bounds__(128, 1) hb_pass_small_kernel(Fields f, Geo g, int parity, HbArgs a) {
   hb_pass<false, false, false, unsigned, GAUSS>(f, g, parity, a);
